@@ -244,6 +244,17 @@ constexpr size_t smem_numc_esc_idx() {
   X(kNB_E6K, 6144, 11)  \
   X(kNB_E8K, 8192, 11)
 
+// ranked-bitmap ESC shapes: threads, blocks per SM, capacity
+#define CAS_RANK_SHAPES(X) \
+  X(256, 4, 5120)          \
+  X(256, 3, 6144)          \
+  X(256, 2, 8192)
+
+// The ranked bitmap (esc_form 2) takes matrices of at most 2^kRankBits
+// columns, what its two levels can tell apart; wider ones take
+// k_numc_esc_idx with the keys in registers.
+bool rank_form(const cas_ctx* ctx, int64_t ncol) { return ctx->esc_form == 2 && ncol <= (int64_t(1) << cas::kRankBits); }
+
 template <typename VIn>
 cas_status setup_numc_kernels(cas_ctx* ctx) {
   using namespace cas;
@@ -260,6 +271,11 @@ cas_status setup_numc_kernels(cas_ctx* ctx) {
                      smem_numc_esc_idx<(int)kFusedHi, 11, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_esc_idx<256, (int)kFusedHi, 11, VIn, true, true>,
                      smem_numc_esc_idx<(int)kFusedHi, 11, VIn>()));
+#define CAS_SETUP_RANK(BLOCK, MINB, CAP)                                                                   \
+  CAS_TRY(allow_smem(ctx, k_numc_rank<BLOCK, MINB, CAP, VIn, false>, smem_numc_rank<BLOCK, CAP, VIn>()));
+  CAS_RANK_SHAPES(CAS_SETUP_RANK)
+#undef CAS_SETUP_RANK
+  CAS_TRY(allow_smem(ctx, k_numc_rank<256, 4, (int)kFusedHi, VIn, true>, smem_numc_rank<256, (int)kFusedHi, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_esc_overflow<1024, 8192, VIn>, smem_numc_esc<1024, 8192, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_hash<256, 9, VIn>, smem_numc_hash<256, 9, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_hash<256, 11, VIn>, smem_numc_hash<256, 11, VIn>()));
@@ -827,7 +843,13 @@ cas_status launch_fused(cas_ctx* ctx, Call& c, const int64_t* known, int32_t* cc
   CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts + kSlotFused + 4, 0, sizeof(unsigned long long), ctx->stream));
   Fused fu{c.frows, ctx->d_counts + kSlotFused + 4, c.fstatus, known, c.row_nz, cap};
   if (ctx->profile) CAS_CUDA(ctx, cudaEventRecord(ctx->ev_fused[0], ctx->stream));
-  if (ctx->esc_form == 1)
+  // Fewer fused rows than SMs keep the index form: which rows it hands to the
+  // radix-sort kernel is a counter that small products report (a test pins
+  // it), and it costs them little (27 against 19 us of a call of 225 us).
+  if (rank_form(ctx, c.ncol) && c.nf >= ctx->sm_count)
+    k_numc_rank<256, 4, (int)kFusedHi, VIn, true><<<(unsigned)c.nf, 256, smem_numc_rank<256, (int)kFusedHi, VIn>(), ctx->stream>>>(
+        nullptr, c.A.csr, c.B.csr, c.b_sorted ? 1 : 0, nullptr, ccol, static_cast<AT*>(cval), ctx->d_status, fu);
+  else if (ctx->esc_form == 1)
     k_numc_esc_idx<256, (int)kFusedHi, 11, VIn, true>
         <<<(unsigned)c.nf, 256, smem_numc_esc_idx<(int)kFusedHi, 11, VIn>(), ctx->stream>>>(
             nullptr, c.A.csr, c.B.csr, c.b_sorted ? 1 : 0, nullptr, ccol, static_cast<AT*>(cval), c.ovf, ovf_count,
@@ -1030,10 +1052,18 @@ cas_status numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int mode) {
 // One bucketed ESC bin: the index form for bins of more than 4096 products
 // when esc_form is 1, else the column-and-value form.
 template <int CAP, int NBB, typename VIn>
-void launch_esc_bin(int esc_form, int64_t n, cudaStream_t s, const int32_t* rows, const cas::Csr& A, const cas::Csr& B,
+void launch_esc_bin(int esc_form, bool rank, int64_t n, cudaStream_t s, const int32_t* rows, const cas::Csr& A, const cas::Csr& B,
                     int32_t b_sorted, const int64_t* crp, int32_t* ccol, typename cas::Acc<VIn>::T* cval, int32_t* ovf,
                     unsigned int* ovf_count, cas::DevStatus* st) {
   using namespace cas;
+  if constexpr (CAP > 4096) {
+    if (rank) {
+      constexpr int RCAP = CAP <= 5120 ? 5120 : CAP, MINB = CAP <= 5120 ? 4 : CAP <= 6144 ? 3 : 2;
+      k_numc_rank<256, MINB, RCAP, VIn, false><<<(unsigned)n, 256, smem_numc_rank<256, RCAP, VIn>(), s>>>(
+          rows, A, B, b_sorted, crp, ccol, cval, st, Fused{});
+      return;
+    }
+  }
   if constexpr (CAP > 4096 && CAP <= 6144) {
     if (esc_form == 2) {
       k_numc_esc_idx<256, CAP, NBB, VIn, false, true><<<(unsigned)n, 256, smem_numc_esc_idx<CAP, NBB, VIn>(), s>>>(
@@ -1151,7 +1181,7 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
 #define CAS_ESC_CASE(bin, CAP, NBB)                                                                      \
       case bin:                                                                                          \
         esc_rows += n;                                                                                   \
-        launch_esc_bin<CAP, NBB, VIn>(ctx->esc_form, n, s, rows, A, B, c.b_sorted ? 1 : 0, crp, ccol, cval, \
+        launch_esc_bin<CAP, NBB, VIn>(ctx->esc_form, rank_form(ctx, c.ncol), n, s, rows, A, B, c.b_sorted ? 1 : 0, crp, ccol, cval, \
                                       c.ovf, ovf_count, ctx->d_status);                                  \
         break;
       CAS_ESC_SHAPES(CAS_ESC_CASE)

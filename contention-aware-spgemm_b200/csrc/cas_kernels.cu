@@ -1031,13 +1031,16 @@ constexpr unsigned long long kLbInc = 2ull << 62;   // the word holds the inclus
 constexpr unsigned long long kLbVal = (1ull << 62) - 1;
 constexpr int kLbSpins = 1 << 22;                   // polls (about 64 ns apart) before giving up
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
+// Relaxed: a status word is all that one row tells another, so no other
+// memory needs ordering (an acquire would drop the SM's L1 lines at every
+// poll, a release wait for the row's earlier stores).
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // Warp 0 of the block holding ticket t: publishes `count`, returns the sum of
@@ -1045,16 +1048,16 @@ __device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned l
 __device__ long long lookback_prefix(unsigned long long* status, int64_t t, long long count) {
   const int lane = threadIdx.x & 31;
   if (t == 0) {
-    if (lane == 0) st_release_u64(&status[0], kLbInc | (unsigned long long)count);
+    if (lane == 0) st_relaxed_u64(&status[0], kLbInc | (unsigned long long)count);
     return 0;
   }
-  if (lane == 0) st_release_u64(&status[t], kLbAgg | (unsigned long long)count);
+  if (lane == 0) st_relaxed_u64(&status[t], kLbAgg | (unsigned long long)count);
   long long excl = 0;
   int64_t j = t - 1;
   int spins = 0;
   for (;;) {
     const int64_t idx = j - lane;
-    const unsigned long long v = idx >= 0 ? ld_acquire_u64(&status[idx]) : kLbInc;
+    const unsigned long long v = idx >= 0 ? ld_relaxed_u64(&status[idx]) : kLbInc;
     if (__any_sync(kFull, (v >> 62) == 0)) {
       if (++spins > kLbSpins) return -1;
       __nanosleep(64);
@@ -1067,7 +1070,7 @@ __device__ long long lookback_prefix(unsigned long long* status, int64_t t, long
     if (inc) break;
     j -= 32;
   }
-  if (lane == 0) st_release_u64(&status[t], kLbInc | (unsigned long long)(excl + count));
+  if (lane == 0) st_relaxed_u64(&status[t], kLbInc | (unsigned long long)(excl + count));
   return excl;
 }
 
@@ -1075,7 +1078,7 @@ __device__ long long lookback_prefix(unsigned long long* status, int64_t t, long
 // them: one thread publishes the row's count (ticket 0: its inclusive
 // prefix) ...
 __device__ __forceinline__ void lookback_publish(unsigned long long* status, int64_t t, long long count) {
-  st_release_u64(&status[t], (t == 0 ? kLbInc : kLbAgg) | (unsigned long long)count);
+  st_relaxed_u64(&status[t], (t == 0 ? kLbInc : kLbAgg) | (unsigned long long)count);
 }
 
 // ... and later warp 0 sums the counts of all earlier tickets, publishes the
@@ -1088,7 +1091,7 @@ __device__ long long lookback_resolve(unsigned long long* status, int64_t t, lon
   int spins = 0;
   for (;;) {
     const int64_t idx = j - lane;
-    const unsigned long long v = idx >= 0 ? ld_acquire_u64(&status[idx]) : kLbInc;
+    const unsigned long long v = idx >= 0 ? ld_relaxed_u64(&status[idx]) : kLbInc;
     if (__any_sync(kFull, (v >> 62) == 0)) {
       if (++spins > kLbSpins) return -1;
       __nanosleep(64);
@@ -1101,7 +1104,7 @@ __device__ long long lookback_resolve(unsigned long long* status, int64_t t, lon
     if (inc) break;
     j -= 32;
   }
-  if (lane == 0) st_release_u64(&status[t], kLbInc | (unsigned long long)(excl + count));
+  if (lane == 0) st_relaxed_u64(&status[t], kLbInc | (unsigned long long)(excl + count));
   return excl;
 }
 
@@ -1933,6 +1936,519 @@ k_numc_esc_idx(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted,
   }
   if (!FUSED && threadIdx.x == 0 && distinct != nz)
     dev_report(st, distinct > nz ? kDevRowOverflow : kDevRowUnderflow, 16, r);
+}
+
+// ---- ranked-bitmap form of the ESC kernel -----------------------------------
+// Rows of at most CAP products whose column range spans at most 2^kRankBits
+// columns (kRankCells cells of up to 16 columns each).  No sort: the place of
+// a column in the row is its rank among the row's columns, read from a
+// two-level bitmap in shared memory.
+//   1. every thread loads the columns of its products (product tid + u*BLOCK)
+//      into registers and marks each column's cell in a bitmap of kRankCells
+//      bits;
+//   2. a scan of the bitmap's population counts ranks the occupied cells;
+//      each gets a 32-bit slot, in which the products mark their exact
+//      column (16 bits).  The product that sets a bit first owns the column,
+//      the others repeat it.  A row whose range is at most kRankCells has one
+//      column per cell and needs no slots;
+//   3. a scan of the slots' population counts gives the distinct columns
+//      before each slot (its upper 16 bits), so a product's place is that
+//      plus the lower columns of its slot;
+//   4. values are loaded in product order (B's own): owners store
+//      a_ik * b_kj at their places, the repeats add theirs by shared-memory
+//      atomics (listed and summed per warp first when they are few: the
+//      diagonal of A*A^T brings one per A entry);
+//   5. the values, then the columns (still in registers), are copied to C in
+//      order.
+// The slots are scanned eight to a thread; rank_slot swaps every second pair
+// of 16-byte groups, so that those accesses meet no bank twice.
+// Bound: shared-memory accesses (about 59 wavefronts per 32 products, half of
+// them bank conflicts of the random cell, slot and value accesses; the LSU
+// data pipe is 69% busy) and, at 32 warps per SM, their latency.  A sort of
+// each row (k_numc_esc_idx) issues half as many instructions again.  Uniform
+// rows of about 4115 products (505,000 of them, 5.2e5 columns): 31.3 ms with
+// k_numc_esc_idx, 22.7 ms here; skewed rows over 1.3e5 columns (12,918 of
+// 3,500 products): 1.63 and 0.37 ms.
+constexpr int kRankCellBits = 17;
+constexpr int kRankCells = 1 << kRankCellBits;
+constexpr int kRankWords = kRankCells / 32;
+constexpr int kRankBits = kRankCellBits + 4;  // columns a row may span: 2^21
+constexpr int kRankChunk = 128;               // A entries staged at a time (byte indices)
+
+__device__ __forceinline__ uint32_t rank_slot(uint32_t q) { return q ^ ((q >> 3) & 4u); }
+
+template <typename VIn>
+struct alignas(16) StageR {
+  // per entry: the address its B row would have at product 0 of the row, so
+  // that product p is element p from there
+  const int32_t* cp[kRankChunk];
+  const VIn* vp[kRankChunk];
+  VIn av[kRankChunk];
+  int32_t pre[kRankChunk + 4];  // first product of each entry (row-wide)
+  unsigned long long tmp[2][16];
+  uint32_t kmin, kmax;
+  int repeats;
+};
+
+// Exclusive prefix over the block with one barrier: `tmp` holds BLOCK/32
+// words that no other call uses until the block has passed another barrier.
+template <int BLOCK, typename T>
+__device__ __forceinline__ T block_exclusive_sum1(T v, T* tmp, T& total) {
+  constexpr int NW = BLOCK / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T inc = warp_inclusive_sum(v);
+  if (lane == 31) tmp[warp] = inc;
+  __syncthreads();
+  T w = lane < NW ? tmp[lane] : T(0);
+#pragma unroll
+  for (int d = 1; d < NW; d <<= 1) {
+    const T u = __shfl_up_sync(kFull, w, d);
+    if (lane >= d) w += u;
+  }
+  total = __shfl_sync(kFull, w, NW - 1);
+  const T before = __shfl_sync(kFull, w, warp > 0 ? warp - 1 : 0);
+  return (warp > 0 ? before : T(0)) + inc - v;
+}
+
+// Shared-memory accesses under a predicate, without a branch.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void sts_if(bool c, uint32_t* p, uint32_t v) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %0, 0;\n@q st.shared.u32 [%1], %2;\n}" ::"r"((int)c), "r"(smem_addr(p)),
+               "r"(v)
+               : "memory");
+}
+__device__ __forceinline__ void sts_if(bool c, double* p, double v) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %0, 0;\n@q st.shared.f64 [%1], %2;\n}" ::"r"((int)c), "r"(smem_addr(p)),
+               "d"(v)
+               : "memory");
+}
+__device__ __forceinline__ void sts_if(bool c, long long* p, long long v) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %0, 0;\n@q st.shared.u64 [%1], %2;\n}" ::"r"((int)c), "r"(smem_addr(p)),
+               "l"(v)
+               : "memory");
+}
+// *p |= v where c holds; returns the old word there, `other` elsewhere.
+__device__ __forceinline__ uint32_t atomic_or_if(bool c, uint32_t* p, uint32_t v, uint32_t other) {
+  uint32_t old = other;
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %1, 0;\n@q atom.shared.or.b32 %0, [%2], %3;\n}"
+               : "+r"(old)
+               : "r"((int)c), "r"(smem_addr(p)), "r"(v)
+               : "memory");
+  return old;
+}
+
+// Sum of x over the lanes of `peers` (the lanes with this lane's key), at
+// their lowest lane; the whole warp takes part.
+template <typename T>
+__device__ __forceinline__ T peers_sum(unsigned peers, T x) {
+  const int lane = threadIdx.x & 31;
+  int rel = __popc(peers & lanemask_lt());
+  peers &= 0xFFFFFFFEu << lane;  // the lanes above
+  while (__any_sync(kFull, peers != 0)) {
+    const int next = __ffs(peers);
+    const T y = __shfl_sync(kFull, x, next > 0 ? next - 1 : lane);
+    if (next > 0) x += y;
+    peers &= __ballot_sync(kFull, (rel & 1) == 0);
+    rel >>= 1;
+  }
+  return x;
+}
+
+// Bytes of shared memory that hold the bitmap, its word prefixes and the
+// slots, later the values, then the columns.
+template <int CAP>
+__host__ __device__ constexpr size_t rank_arena() {
+  return size_t(kRankWords) * 6 + size_t(CAP) * 4 > size_t(CAP) * 8 ? size_t(kRankWords) * 6 + size_t(CAP) * 4
+                                                                     : size_t(CAP) * 8;
+}
+template <int BLOCK, int CAP, typename VIn>
+__host__ __device__ constexpr size_t smem_numc_rank() {
+  return rank_arena<CAP>() + CAP + sizeof(StageR<VIn>) + BLOCK * 4;
+}
+
+// Stages the A entries [a0, a0 + na) of a row whose earlier entries have
+// pbase products: cp, vp, av, pre and the byte table (entry of each
+// product).  Returns the products up to the end of the chunk, or CAP + 1
+// when they exceed CAP (nothing is written to the byte table then).
+template <int BLOCK, int CAP, typename VIn>
+__device__ __forceinline__ int stage_rank(const Csr& A, const Csr& B, int64_t a0, int na, int pbase, StageR<VIn>& sg,
+                                          uint8_t* __restrict__ segof, bool range) {
+  static_assert(BLOCK >= kRankChunk, "one staged entry per thread");
+  constexpr int NW = BLOCK / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int len = 0;
+  int64_t bs = 0;
+  uint32_t lo_key = 0xFFFFFFFFu, hi_key = 0u;
+  if (threadIdx.x < na) {
+    const int32_t k = A.col[a0 + threadIdx.x];
+    bs = B.rp[k];
+    const int64_t l = B.rp[k + 1] - bs;
+    len = l > CAP ? CAP + 1 : (int)l;
+    sg.av[threadIdx.x] = static_cast<const VIn*>(A.val)[a0 + threadIdx.x];
+    if (range && len > 0) {
+      lo_key = (uint32_t)__ldg(B.col + bs);
+      hi_key = (uint32_t)__ldg(B.col + bs + l - 1);
+    }
+  }
+  if (range && warp * 32 < na) {
+    lo_key = __reduce_min_sync(kFull, lo_key);
+    hi_key = __reduce_max_sync(kFull, hi_key);
+    if (lane == 0 && hi_key >= lo_key) {
+      atomicMin(&sg.kmin, lo_key);
+      atomicMax(&sg.kmax, hi_key);
+    }
+  }
+  int total;
+  const int ex = pbase + block_exclusive_sum1<BLOCK, int>(len, reinterpret_cast<int*>(sg.tmp[0]), total);
+  const int end = pbase + total > CAP ? CAP + 1 : pbase + total;
+  if (end > CAP) return end;
+  if (threadIdx.x < na) {
+    sg.cp[threadIdx.x] = B.col + (bs - ex);
+    sg.vp[threadIdx.x] = static_cast<const VIn*>(B.val) + (bs - ex);
+    sg.pre[threadIdx.x] = ex;
+  }
+  if (threadIdx.x == 0) sg.pre[na] = end;
+  __syncthreads();
+  for (int e = warp; e < na; e += NW) {
+    const int p1 = sg.pre[e + 1];
+    for (int p = sg.pre[e] + lane; p < p1; p += 32) segof[p] = (uint8_t)e;
+  }
+  __syncthreads();
+  return end;
+}
+
+template <int BLOCK, int MINB, int CAP, typename VIn, bool FUSED>
+__global__ void __launch_bounds__(BLOCK, MINB)
+k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, const int64_t* __restrict__ crp,
+            int32_t* __restrict__ ccol, typename Acc<VIn>::T* __restrict__ cval, DevStatus* st, Fused fu) {
+  using AT = typename Acc<VIn>::T;
+  constexpr int NW = BLOCK / 32;
+  constexpr int NPT = (CAP + BLOCK - 1) / BLOCK;  // products per thread
+  constexpr int G = 4;                            // products whose loads are in flight together
+  constexpr int WCH = kRankWords / (4 * BLOCK);   // bitmap chunks of 4 words per thread
+  constexpr int SCH = (CAP + 8 * BLOCK - 1) / (8 * BLOCK);  // slot chunks of 8 per thread
+  static_assert(CAP < 16384 && NPT % G == 0 && NPT <= 32, "places in 16 bits, whole groups, one flag per product");
+  static_assert(WCH >= 1 && WCH <= 4 && SCH <= 4, "four 16-bit counts in one word of a scan");
+  static_assert(CAP % 16 == 0 && NW <= 16, "vector access to the slots; the scans' words");
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint32_t* bits = reinterpret_cast<uint32_t*>(smem);
+  uint16_t* wpre = reinterpret_cast<uint16_t*>(bits + kRankWords);
+  uint32_t* slot = reinterpret_cast<uint32_t*>(wpre + kRankWords);
+  AT* sval = reinterpret_cast<AT*>(smem);              // over all three
+  uint32_t* scol = reinterpret_cast<uint32_t*>(smem);  // after the values
+  uint8_t* segof = smem + rank_arena<CAP>();
+  StageR<VIn>& sg = *reinterpret_cast<StageR<VIn>*>(segof + CAP);
+  // the repeats, when they are at most one per thread: product, place
+  uint32_t* rep = reinterpret_cast<uint32_t*>(segof + CAP + sizeof(StageR<VIn>));
+  __shared__ long long s_tick, s_off;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t r, tick = 0;
+  if (threadIdx.x == 0) {
+    if (FUSED) s_tick = (long long)atomicAdd(fu.ticket, 1ull);
+    sg.kmin = b_sorted ? 0xFFFFFFFFu : 0u;
+    sg.kmax = b_sorted ? 0u : (uint32_t)(B.ncol > 0 ? B.ncol - 1 : 0);
+    sg.repeats = 0;
+  }
+  for (int i = threadIdx.x; i < kRankWords / 4; i += BLOCK) reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  if (FUSED) {
+    tick = s_tick;
+    r = fu.rows[tick];
+  } else {
+    r = rows[blockIdx.x];
+  }
+  const int64_t as = A.rp[r], ae = A.rp[r + 1];
+  auto give_up = [&]() {  // uniform: a row this kernel's bounds do not hold
+    if (threadIdx.x == 0) dev_report(st, kDevCapacity, 17, r);
+    if (FUSED && warp == 0) {
+      lookback_prefix(fu.status, tick, 0);
+      if (lane == 0) fu.row_nz[r] = 0;
+    }
+  };
+  // 1. columns into registers, chunk by chunk of A entries (nearly always
+  // one).  Here and below a product past the row's last reads as the last
+  // one (no branch), and `valid` leaves it out where that matters.
+  uint32_t key[NPT];
+  int n = 0;
+  for (int64_t a0 = as; a0 < ae; a0 += kRankChunk) {
+    const int p0 = n;
+    const int na = (int)(ae - a0 < kRankChunk ? ae - a0 : kRankChunk);
+    n = stage_rank<BLOCK, CAP, VIn>(A, B, a0, na, p0, sg, segof, b_sorted != 0);
+    if (n > CAP) {
+      give_up();
+      return;
+    }
+    if (n > p0) {
+#pragma unroll
+      for (int g = 0; g < NPT; g += G) {
+        if (g * BLOCK >= n) break;
+        if ((g + G) * BLOCK <= p0) continue;
+#pragma unroll
+        for (int u = g; u < g + G; ++u) {
+          const int p = threadIdx.x + u * BLOCK;
+          const int pc = min(max(p, p0), n - 1);
+          const uint32_t k = (uint32_t)__ldg(sg.cp[segof[pc]] + pc);
+          if (p >= p0) key[u] = k;
+        }
+      }
+    }
+    if (ae - a0 > kRankChunk) __syncthreads();  // the next chunk overwrites cp
+  }
+  const uint32_t lo = sg.kmin;
+  const uint32_t range = sg.kmax > sg.kmin ? sg.kmax - sg.kmin : 0u;
+  const int rbits = 32 - __clz(range);
+  const int shift = rbits > kRankCellBits ? rbits - kRankCellBits : 0;
+  if (shift > kRankBits - kRankCellBits) {  // the host takes this kernel for narrower matrices only
+    give_up();
+    return;
+  }
+  const int nwords = (int)((range >> shift) >> 5) + 1;
+  const int cnt = n > (int)threadIdx.x ? (n - (int)threadIdx.x + BLOCK - 1) / BLOCK : 0;
+  const uint32_t valid = cnt >= 32 ? 0xFFFFFFFFu : (1u << cnt) - 1u;
+  uint32_t own = 0;  // bit u: the thread's product u set its cell's bit
+#pragma unroll
+  for (int g = 0; g < NPT; g += G) {
+    if (g * BLOCK >= n) break;
+#pragma unroll
+    for (int u = g; u < g + G; ++u) {
+      key[u] -= lo;
+      const uint32_t c = key[u] >> shift;
+      const uint32_t bit = 1u << (c & 31);
+      const uint32_t old = atomic_or_if((valid >> u) & 1u, &bits[c >> 5], bit, bit);
+      if (!(old & bit)) own |= 1u << u;
+    }
+  }
+  __syncthreads();
+  // 2. ranks of the occupied cells: four words per thread and chunk, the
+  // chunks' counts in the 16-bit fields of one scanned word
+  int distinct;
+  {
+    uint2 pc[WCH];  // set bits before each of the four words
+    unsigned long long packed = 0;
+#pragma unroll
+    for (int k = 0; k < WCH; ++k) {
+      pc[k] = make_uint2(0, 0);
+      if (k * BLOCK * 4 < nwords) {
+        const uint4 w = reinterpret_cast<const uint4*>(bits)[k * BLOCK + threadIdx.x];
+        const uint32_t c0 = __popc(w.x), c1 = c0 + __popc(w.y), c2 = c1 + __popc(w.z);
+        pc[k] = make_uint2(c0 << 16, c1 | (c2 << 16));
+        packed |= (unsigned long long)(c2 + __popc(w.w)) << (16 * k);
+      }
+    }
+    unsigned long long total;
+    const unsigned long long ex = block_exclusive_sum1<BLOCK, unsigned long long>(packed, sg.tmp[1], total);
+    uint32_t base = 0;
+#pragma unroll
+    for (int k = 0; k < WCH; ++k) {
+      if (k * BLOCK * 4 < nwords) {
+        const uint32_t b = base + (uint32_t)((ex >> (16 * k)) & 0xFFFFu);
+        reinterpret_cast<uint2*>(wpre)[k * BLOCK + threadIdx.x] =
+            make_uint2(pc[k].x + b * 0x10001u, pc[k].y + b * 0x10001u);
+        base += (uint32_t)((total >> (16 * k)) & 0xFFFFu);
+      }
+    }
+    distinct = (int)base;
+  }
+  const uint32_t submask = (1u << shift) - 1u;
+  if (shift > 0) {
+    for (int i = threadIdx.x; i < ((distinct + 7) >> 3) * 2; i += BLOCK)
+      reinterpret_cast<uint4*>(slot)[i] = make_uint4(0, 0, 0, 0);
+    own = 0;
+  }
+  __syncthreads();
+  uint32_t pos[NPT / 2] = {};  // rank of each product's cell, later its column's place: two per word
+  auto get_pos = [&](int u) -> uint32_t { return (u & 1) ? pos[u >> 1] >> 16 : pos[u >> 1] & 0xFFFFu; };
+#pragma unroll
+  for (int g = 0; g < NPT; g += G) {
+    if (g * BLOCK >= n) break;
+    uint32_t q[G];
+#pragma unroll
+    for (int v = 0; v < G; ++v) {
+      const uint32_t c = key[g + v] >> shift, w = c >> 5;
+      q[v] = wpre[w] + __popc(bits[w] & ((1u << (c & 31)) - 1u));
+    }
+    if (shift > 0) {
+#pragma unroll
+      for (int v = 0; v < G; ++v) {
+        q[v] = rank_slot(q[v]);
+        const uint32_t bit = 1u << (key[g + v] & submask);
+        const uint32_t old = atomic_or_if((valid >> (g + v)) & 1u, &slot[q[v]], bit, bit);
+        if (!(old & bit)) own |= 1u << (g + v);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < G; v += 2) pos[(g + v) >> 1] = q[v] | (q[v + 1] << 16);
+  }
+  __syncthreads();
+  // 3. places: the distinct columns before each slot
+  if (shift > 0) {
+    const int nocc = distinct;
+    unsigned long long packed = 0;
+#pragma unroll
+    for (int k = 0; k < SCH; ++k) {
+      const int i = k * BLOCK + threadIdx.x;
+      if (i * 8 < nocc) {
+        const int j = (2 * i) ^ ((i >> 2) & 1);  // the group of slots 8 i to 8 i + 3
+        const uint4 a = reinterpret_cast<const uint4*>(slot)[j], b = reinterpret_cast<const uint4*>(slot)[j ^ 1];
+        packed |= (unsigned long long)(__popc(a.x | (a.y << 16)) + __popc(a.z | (a.w << 16)) +
+                                       __popc(b.x | (b.y << 16)) + __popc(b.z | (b.w << 16)))
+                  << (16 * k);
+      }
+    }
+    unsigned long long total;
+    const unsigned long long ex = block_exclusive_sum1<BLOCK, unsigned long long>(packed, sg.tmp[0], total);
+    uint32_t base = 0;
+#pragma unroll
+    for (int k = 0; k < SCH; ++k) {
+      const int i = k * BLOCK + threadIdx.x;
+      if (i * 8 < nocc) {
+        uint32_t b = base + (uint32_t)((ex >> (16 * k)) & 0xFFFFu);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int j = (2 * i + h) ^ ((i >> 2) & 1);
+          uint4 m = reinterpret_cast<const uint4*>(slot)[j];
+          const uint32_t b1 = b + __popc(m.x), b2 = b1 + __popc(m.y), b3 = b2 + __popc(m.z), b4 = b3 + __popc(m.w);
+          m.x |= b << 16;
+          m.y |= b1 << 16;
+          m.z |= b2 << 16;
+          m.w |= b3 << 16;
+          reinterpret_cast<uint4*>(slot)[j] = m;
+          b = b4;
+        }
+      }
+      base += (uint32_t)((total >> (16 * k)) & 0xFFFFu);
+    }
+    distinct = (int)base;
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < NPT; g += G) {
+      if (g * BLOCK >= n) break;
+#pragma unroll
+      for (int u = g; u < g + G; u += 2) {
+        const uint32_t s0 = slot[pos[u >> 1] & 0xFFFFu], s1 = slot[pos[u >> 1] >> 16];
+        const uint32_t q0 = (s0 >> 16) + __popc(s0 & ((1u << (key[u] & submask)) - 1u));
+        const uint32_t q1 = (s1 >> 16) + __popc(s1 & ((1u << (key[u + 1] & submask)) - 1u));
+        pos[u >> 1] = q0 | (q1 << 16);
+      }
+    }
+  }
+  // fused rows: the count goes out now; the look-back waits until the values
+  // are in place, so the wait for earlier rows overlaps them
+  if (FUSED && threadIdx.x == 0) lookback_publish(fu.status, tick, distinct);
+  const bool listed = n - distinct <= BLOCK;
+  const uint32_t dup = valid & ~own;
+  if (listed && dup) {
+#pragma unroll
+    for (int g = 0; g < NPT; g += G) {
+      if (((dup >> g) & ((1u << G) - 1u)) == 0) continue;
+#pragma unroll
+      for (int u = g; u < g + G; ++u)
+        if ((dup >> u) & 1u) rep[atomicAdd(&sg.repeats, 1)] = (uint32_t)(threadIdx.x + u * BLOCK) | (get_pos(u) << 16);
+    }
+  }
+  __syncthreads();
+  // 4. values
+  auto values = [&](int p0, int p1, uint32_t which, auto&& put) {
+#pragma unroll
+    for (int g = 0; g < NPT; g += G) {
+      if (g * BLOCK >= p1) break;
+      if (((which >> g) & ((1u << G) - 1u)) == 0) continue;
+      VIn av[G], bv[G];
+#pragma unroll
+      for (int v = 0; v < G; ++v) {
+        const int pc = min(max((int)threadIdx.x + (g + v) * BLOCK, p0), p1 - 1);
+        const int e = segof[pc];
+        bv[v] = __ldg(sg.vp[e] + pc);
+        av[v] = sg.av[e];
+      }
+#pragma unroll
+      for (int v = 0; v < G; ++v) put((which >> (g + v)) & 1u, &sval[get_pos(g + v)], Acc<VIn>::mul(av[v], bv[v]));
+    }
+  };
+  // the products of [p0, p1) among the thread's
+  auto within = [&](int p0, int p1) -> uint32_t {
+    const int t = threadIdx.x;
+    const int c1 = p1 > t ? (p1 - t + BLOCK - 1) / BLOCK : 0, c0 = p0 > t ? (p0 - t + BLOCK - 1) / BLOCK : 0;
+    return (c1 >= 32 ? 0xFFFFFFFFu : (1u << c1) - 1u) & ~((1u << c0) - 1u);
+  };
+  auto store = [](bool c, AT* p, AT v) { sts_if(c, p, v); };
+  auto add = [](bool c, AT* p, AT v) {
+    if (c) atomic_add_sh(p, v);
+  };
+  auto add_listed = [&](int p0, int p1) {
+    if (warp * 32 >= n - distinct) return;
+    const uint32_t d = threadIdx.x < n - distinct ? rep[threadIdx.x] : 0xFFFFFFFFu;
+    const int p = (int)(d & 0xFFFFu);
+    const bool in = p >= p0 && p < p1;
+    AT x = AT(0);
+    if (in) {
+      const int e = segof[p];
+      x = Acc<VIn>::mul(sg.av[e], __ldg(sg.vp[e] + p));
+    }
+    const unsigned peers = __match_any_sync(kFull, in ? d >> 16 : 0x10000u);
+    x = peers_sum(peers, x);
+    if (in && lane == __ffs(peers) - 1) atomic_add_sh(&sval[d >> 16], x);
+  };
+  if (ae - as <= kRankChunk) {
+    values(0, n, own, store);
+    if (distinct < n) {  // uniform
+      __syncthreads();
+      if (listed) add_listed(0, n);
+      else values(0, n, dup, add);
+    }
+  } else {
+    // each chunk of A entries staged again, once for the owners and once for
+    // the repeats
+    for (int pass = 0; pass < 2; ++pass) {
+      int p1 = 0;
+      for (int64_t a0 = as; a0 < ae; a0 += kRankChunk) {
+        const int p0 = p1;
+        const int na = (int)(ae - a0 < kRankChunk ? ae - a0 : kRankChunk);
+        p1 = stage_rank<BLOCK, CAP, VIn>(A, B, a0, na, p0, sg, segof, false);
+        if (pass == 0) values(p0, p1, own & within(p0, p1), store);
+        else if (listed) add_listed(p0, p1);
+        else values(p0, p1, dup & within(p0, p1), add);
+        __syncthreads();
+      }
+    }
+  }
+  int64_t c0;
+  if (FUSED) {
+    if (warp == 0) {
+      const long long ex = lookback_resolve(fu.status, tick, distinct);
+      if (lane == 0) {
+        s_off = ex < 0 ? -1 : (long long)fu.known[r] + ex;
+        fu.row_nz[r] = ex < 0 ? 0 : distinct;
+        if (ex < 0) dev_report(st, kDevTimeout, 17, r);
+      }
+    }
+    __syncthreads();
+    c0 = s_off;
+    if (c0 < 0) return;
+    if (c0 + distinct > fu.cap) {
+      if (threadIdx.x == 0) dev_report(st, kDevRowOverflow, 17, r);
+      return;
+    }
+  } else {
+    c0 = crp[r];
+    const int64_t nz = crp[r + 1] - c0;
+    if (distinct != nz) {  // uniform
+      if (threadIdx.x == 0) dev_report(st, distinct > nz ? kDevRowOverflow : kDevRowUnderflow, 17, r);
+      return;
+    }
+    __syncthreads();
+  }
+  // 5. the row in order; the columns follow over the same shared memory
+  for (int i = threadIdx.x; i < distinct; i += BLOCK) cval[c0 + i] = sval[i];
+  __syncthreads();
+#pragma unroll
+  for (int g = 0; g < NPT; g += G) {
+    if (g * BLOCK >= n) break;
+#pragma unroll
+    for (int u = g; u < g + G; ++u) sts_if((own >> u) & 1u, &scol[get_pos(u)], key[u] + lo);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < distinct; i += BLOCK) ccol[c0 + i] = (int32_t)scol[i];
 }
 
 // Hash accumulator for rows with at most 2^TBITS / 2 distinct columns: linear

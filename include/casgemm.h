@@ -153,12 +153,14 @@ typedef struct {
 	                                larger rows take the dense kernels */
 	int32_t esc_form;            /* bucketed ESC kernel of the fused rows and of ESC rows over 4096
 	                                products: 1 keeps column, product index and place per product in
-	                                shared memory, 4 rows per SM; 2 [the default] is form 1 with each thread's
-	                                columns held in registers between its histogram and scatter
-	                                passes (B's columns read once) and, for rows whose B rows average
-	                                32 products or more, a warp per B row in the value pass (rows of
-	                                up to 6144 products; larger ones take form 1); 0 keeps column and
-	                                value, 3 rows per SM */
+	                                shared memory, 4 rows per SM; 2 [the default] ranks the columns in a
+	                                two-level bitmap instead of sorting them, where B has at most 2^21
+	                                columns (and, for the fused rows, there is at least one per SM),
+	                                else it is form 1 with each thread's columns held in registers
+	                                between its histogram and scatter passes (B's columns read once)
+	                                and, for rows whose B rows average 32 products or more, a warp per
+	                                B row in the value pass (rows of up to 6144 products; larger ones
+	                                take form 1); 0 keeps column and value, 3 rows per SM */
 	int32_t heavy_split;         /* 1: dense rows of 2^17 products or more are split across thread blocks
 	                                by A-entry ranges, heaviest row first, adding into C by atomics that
 	                                stay in L2 [1]; 0: one block per dense row */
