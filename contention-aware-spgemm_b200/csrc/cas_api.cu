@@ -246,6 +246,8 @@ constexpr size_t smem_numc_esc_idx() {
 
 // ranked-bitmap ESC shapes: threads, blocks per SM, capacity
 #define CAS_RANK_SHAPES(X) \
+  X(128, 12, 1024)         \
+  X(256, 6, 2048)          \
   X(256, 4, 5120)          \
   X(256, 3, 6144)          \
   X(256, 2, 8192)
@@ -272,10 +274,11 @@ cas_status setup_numc_kernels(cas_ctx* ctx) {
   CAS_TRY(allow_smem(ctx, k_numc_esc_idx<256, (int)kFusedHi, 11, VIn, true, true>,
                      smem_numc_esc_idx<(int)kFusedHi, 11, VIn>()));
 #define CAS_SETUP_RANK(BLOCK, MINB, CAP)                                                                   \
-  CAS_TRY(allow_smem(ctx, k_numc_rank<BLOCK, MINB, CAP, VIn, false>, smem_numc_rank<BLOCK, CAP, VIn>()));
+  CAS_TRY(allow_smem(ctx, k_numc_rank<BLOCK, MINB, CAP, VIn, false>, smem_numc_rank<BLOCK, CAP, VIn>(kRankCellBits)));
   CAS_RANK_SHAPES(CAS_SETUP_RANK)
 #undef CAS_SETUP_RANK
-  CAS_TRY(allow_smem(ctx, k_numc_rank<256, 4, (int)kFusedHi, VIn, true>, smem_numc_rank<256, (int)kFusedHi, VIn>()));
+  CAS_TRY(allow_smem(ctx, k_numc_rank<256, 4, (int)kFusedHi, VIn, true>,
+                     smem_numc_rank<256, (int)kFusedHi, VIn>(kRankCellBits)));
   CAS_TRY(allow_smem(ctx, k_numc_esc_overflow<1024, 8192, VIn>, smem_numc_esc<1024, 8192, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_hash<256, 9, VIn>, smem_numc_hash<256, 9, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_hash<256, 11, VIn>, smem_numc_hash<256, 11, VIn>()));
@@ -685,6 +688,7 @@ struct Call {
   int64_t* fpos = nullptr;
   unsigned long long* fstatus = nullptr;
   bool ovf_preset = false;
+  bool may_defer = false;  // some kernel launched may hand rows to the radix-sort ESC kernel
   // bitmaps of heavy rows kept by the symbolic kernel for the numeric one
   uint32_t* dbits = nullptr;
   int32_t* dslot = nullptr;
@@ -846,9 +850,14 @@ cas_status launch_fused(cas_ctx* ctx, Call& c, const int64_t* known, int32_t* cc
   // Fewer fused rows than SMs keep the index form: which rows it hands to the
   // radix-sort kernel is a counter that small products report (a test pins
   // it), and it costs them little (27 against 19 us of a call of 225 us).
-  if (rank_form(ctx, c.ncol) && c.nf >= ctx->sm_count)
-    k_numc_rank<256, 4, (int)kFusedHi, VIn, true><<<(unsigned)c.nf, 256, smem_numc_rank<256, (int)kFusedHi, VIn>(), ctx->stream>>>(
-        nullptr, c.A.csr, c.B.csr, c.b_sorted ? 1 : 0, nullptr, ccol, static_cast<AT*>(cval), ctx->d_status, fu);
+  const int cell_bits = rank_cell_bits<(int)kFusedHi>(c.ncol);
+  const bool rank = rank_form(ctx, c.ncol) && c.nf >= ctx->sm_count;
+  if (!rank) c.may_defer = true;
+  if (rank)
+    k_numc_rank<256, 4, (int)kFusedHi, VIn, true>
+        <<<(unsigned)c.nf, 256, smem_numc_rank<256, (int)kFusedHi, VIn>(cell_bits), ctx->stream>>>(
+            nullptr, c.A.csr, c.B.csr, c.b_sorted ? 1 : 0, cell_bits, nullptr, ccol, static_cast<AT*>(cval),
+            ctx->d_status, fu);
   else if (ctx->esc_form == 1)
     k_numc_esc_idx<256, (int)kFusedHi, 11, VIn, true>
         <<<(unsigned)c.nf, 256, smem_numc_esc_idx<(int)kFusedHi, 11, VIn>(), ctx->stream>>>(
@@ -1049,20 +1058,25 @@ cas_status numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int mode) {
 }
 
 // ------------------------------------------------------------------ NUMC
-// One bucketed ESC bin: the index form for bins of more than 4096 products
-// when esc_form is 1, else the column-and-value form.
+// One ESC bin.  esc_form 2 ranks the columns in a bitmap where the matrix is
+// narrow enough (rank_form), for all bins: rows of 33..1024 products 2.07 ->
+// 0.72 ms (131,070 uniform rows of 272 over 1.3e5 columns) and 4.30 -> 1.71 ms
+// (292,119 join rows of 400 over 6e5), of 1025..2048 4.91 -> 1.66 ms (120,789
+// of 1424).  Otherwise the index form for bins of more than 4096 products when
+// esc_form is at least 1, else the column-and-value form.
 template <int CAP, int NBB, typename VIn>
 void launch_esc_bin(int esc_form, bool rank, int64_t n, cudaStream_t s, const int32_t* rows, const cas::Csr& A, const cas::Csr& B,
                     int32_t b_sorted, const int64_t* crp, int32_t* ccol, typename cas::Acc<VIn>::T* cval, int32_t* ovf,
                     unsigned int* ovf_count, cas::DevStatus* st) {
   using namespace cas;
-  if constexpr (CAP > 4096) {
-    if (rank) {
-      constexpr int RCAP = CAP <= 5120 ? 5120 : CAP, MINB = CAP <= 5120 ? 4 : CAP <= 6144 ? 3 : 2;
-      k_numc_rank<256, MINB, RCAP, VIn, false><<<(unsigned)n, 256, smem_numc_rank<256, RCAP, VIn>(), s>>>(
-          rows, A, B, b_sorted, crp, ccol, cval, st, Fused{});
-      return;
-    }
+  if (rank) {
+    constexpr int RCAP = CAP <= 1024 ? 1024 : CAP <= 2048 ? 2048 : CAP <= 5120 ? 5120 : CAP;
+    constexpr int BLOCK = CAP <= 1024 ? 128 : 256;
+    constexpr int MINB = CAP <= 1024 ? 12 : CAP <= 2048 ? 6 : CAP <= 5120 ? 4 : CAP <= 6144 ? 3 : 2;
+    const int cell_bits = rank_cell_bits<RCAP>(B.ncol);
+    k_numc_rank<BLOCK, MINB, RCAP, VIn, false><<<(unsigned)n, BLOCK, smem_numc_rank<BLOCK, RCAP, VIn>(cell_bits), s>>>(
+        rows, A, B, b_sorted, cell_bits, crp, ccol, cval, st, Fused{});
+    return;
   }
   if constexpr (CAP > 4096 && CAP <= 6144) {
     if (esc_form == 2) {
@@ -1163,6 +1177,7 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
   unsigned int* ovf_count = reinterpret_cast<unsigned int*>(ctx->d_counts + kSlotOvf);
   if (!c.ovf_preset) CAS_CUDA(ctx, cudaMemsetAsync(ovf_count, 0, sizeof(unsigned int), ctx->stream));
   CAS_TRY(fork(ctx));
+  const bool rank = rank_form(ctx, c.ncol);
   int64_t esc_rows = c.nf;  // fused rows may have handed rows to the radix-sort kernel too
   int si = 0;
   for (int oi = 0; oi < 12; ++oi) {
@@ -1181,7 +1196,8 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
 #define CAS_ESC_CASE(bin, CAP, NBB)                                                                      \
       case bin:                                                                                          \
         esc_rows += n;                                                                                   \
-        launch_esc_bin<CAP, NBB, VIn>(ctx->esc_form, rank_form(ctx, c.ncol), n, s, rows, A, B, c.b_sorted ? 1 : 0, crp, ccol, cval, \
+        if (!rank) c.may_defer = true;                                                                   \
+        launch_esc_bin<CAP, NBB, VIn>(ctx->esc_form, rank, n, s, rows, A, B, c.b_sorted ? 1 : 0, crp, ccol, cval, \
                                       c.ovf, ovf_count, ctx->d_status);                                  \
         break;
       CAS_ESC_SHAPES(CAS_ESC_CASE)
@@ -1220,7 +1236,7 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
     if (ctx->profile) CAS_CUDA(ctx, cudaEventRecord(ctx->ev_numc[1][b], s));
   }
   CAS_TRY(join(ctx));
-  if (esc_rows > 0) {
+  if (c.may_defer) {
     // rows whose columns bucket unevenly: radix-sort ESC, one persistent CTA per SM
     if (ctx->profile) CAS_CUDA(ctx, cudaEventRecord(ctx->ev_ovf[0], ctx->stream));
     k_numc_esc_overflow<1024, 8192, VIn><<<(unsigned)std::min<int64_t>(esc_rows, ctx->sm_count), 1024,

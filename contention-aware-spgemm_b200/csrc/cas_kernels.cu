@@ -1939,17 +1939,16 @@ k_numc_esc_idx(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted,
 }
 
 // ---- ranked-bitmap form of the ESC kernel -----------------------------------
-// Rows of at most CAP products whose column range spans at most 2^kRankBits
-// columns (kRankCells cells of up to 16 columns each).  No sort: the place of
-// a column in the row is its rank among the row's columns, read from a
-// two-level bitmap in shared memory.
+// Rows of at most CAP products of matrices of at most 2^kRankBits columns.  No
+// sort: the place of a column in the row is its rank among the row's columns,
+// read from a two-level bitmap in shared memory.
 //   1. every thread loads the columns of its products (product tid + u*BLOCK)
-//      into registers and marks each column's cell in a bitmap of kRankCells
-//      bits;
+//      into registers and marks each column's cell, 1 to 16 columns, in a
+//      bitmap of 2^cell_bits cells (rank_cell_bits);
 //   2. a scan of the bitmap's population counts ranks the occupied cells;
 //      each gets a 32-bit slot, in which the products mark their exact
 //      column (16 bits).  The product that sets a bit first owns the column,
-//      the others repeat it.  A row whose range is at most kRankCells has one
+//      the others repeat it.  A row whose range is at most 2^cell_bits has one
 //      column per cell and needs no slots;
 //   3. a scan of the slots' population counts gives the distinct columns
 //      before each slot (its upper 16 bits), so a product's place is that
@@ -1969,9 +1968,7 @@ k_numc_esc_idx(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted,
 // rows of about 4115 products (505,000 of them, 5.2e5 columns): 31.3 ms with
 // k_numc_esc_idx, 22.7 ms here; skewed rows over 1.3e5 columns (12,918 of
 // 3,500 products): 1.63 and 0.37 ms.
-constexpr int kRankCellBits = 17;
-constexpr int kRankCells = 1 << kRankCellBits;
-constexpr int kRankWords = kRankCells / 32;
+constexpr int kRankCellBits = 17;             // most cells: 2^17
 constexpr int kRankBits = kRankCellBits + 4;  // columns a row may span: 2^21
 constexpr int kRankChunk = 128;               // A entries staged at a time (byte indices)
 
@@ -2054,16 +2051,30 @@ __device__ __forceinline__ T peers_sum(unsigned peers, T x) {
   return x;
 }
 
+// log2 of the bitmap's cells for rows of up to `cap` products over ncol
+// columns.  Clearing and scanning the bitmap is work for every row, the
+// second level work for every product: one column per cell while that is at
+// most a bitmap word for each of the cap products, else 16.
+template <int CAP>
+__host__ __device__ constexpr int rank_cell_bits(int64_t ncol) {
+  int rb = 0;
+  while ((int64_t(1) << rb) < ncol) ++rb;
+  int one = 8;
+  while (one < kRankCellBits && (2 << one) <= 32 * CAP) ++one;
+  const int bits = rb <= one ? rb : rb - 4;
+  return bits < 8 ? 8 : bits;
+}
 // Bytes of shared memory that hold the bitmap, its word prefixes and the
 // slots, later the values, then the columns.
 template <int CAP>
-__host__ __device__ constexpr size_t rank_arena() {
-  return size_t(kRankWords) * 6 + size_t(CAP) * 4 > size_t(CAP) * 8 ? size_t(kRankWords) * 6 + size_t(CAP) * 4
-                                                                     : size_t(CAP) * 8;
+__host__ __device__ constexpr size_t rank_arena(int cell_bits) {
+  return (size_t(1) << (cell_bits - 5)) * 6 + size_t(CAP) * 4 > size_t(CAP) * 8
+             ? (size_t(1) << (cell_bits - 5)) * 6 + size_t(CAP) * 4
+             : size_t(CAP) * 8;
 }
 template <int BLOCK, int CAP, typename VIn>
-__host__ __device__ constexpr size_t smem_numc_rank() {
-  return rank_arena<CAP>() + CAP + sizeof(StageR<VIn>) + BLOCK * 4;
+__host__ __device__ constexpr size_t smem_numc_rank(int cell_bits) {
+  return ((rank_arena<CAP>(cell_bits) + 15) & ~size_t(15)) + CAP + sizeof(StageR<VIn>) + BLOCK * 4;
 }
 
 // Stages the A entries [a0, a0 + na) of a row whose earlier entries have
@@ -2119,24 +2130,25 @@ __device__ __forceinline__ int stage_rank(const Csr& A, const Csr& B, int64_t a0
 
 template <int BLOCK, int MINB, int CAP, typename VIn, bool FUSED>
 __global__ void __launch_bounds__(BLOCK, MINB)
-k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, const int64_t* __restrict__ crp,
-            int32_t* __restrict__ ccol, typename Acc<VIn>::T* __restrict__ cval, DevStatus* st, Fused fu) {
+k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, int cell_bits,
+            const int64_t* __restrict__ crp, int32_t* __restrict__ ccol, typename Acc<VIn>::T* __restrict__ cval, DevStatus* st, Fused fu) {
   using AT = typename Acc<VIn>::T;
   constexpr int NW = BLOCK / 32;
   constexpr int NPT = (CAP + BLOCK - 1) / BLOCK;  // products per thread
-  constexpr int G = 4;                            // products whose loads are in flight together
-  constexpr int WCH = kRankWords / (4 * BLOCK);   // bitmap chunks of 4 words per thread
+  constexpr int G = NPT >= 16 ? 4 : 2;            // products whose loads are in flight together
+  constexpr int WCH = 4;                          // bitmap chunks of 4 words per thread in one scan
   constexpr int SCH = (CAP + 8 * BLOCK - 1) / (8 * BLOCK);  // slot chunks of 8 per thread
   static_assert(CAP < 16384 && NPT % G == 0 && NPT <= 32, "places in 16 bits, whole groups, one flag per product");
-  static_assert(WCH >= 1 && WCH <= 4 && SCH <= 4, "four 16-bit counts in one word of a scan");
+  static_assert(WCH <= 4 && SCH <= 4, "four 16-bit counts in one word of a scan");
   static_assert(CAP % 16 == 0 && NW <= 16, "vector access to the slots; the scans' words");
   extern __shared__ __align__(16) uint8_t smem[];
   uint32_t* bits = reinterpret_cast<uint32_t*>(smem);
-  uint16_t* wpre = reinterpret_cast<uint16_t*>(bits + kRankWords);
-  uint32_t* slot = reinterpret_cast<uint32_t*>(wpre + kRankWords);
+  const int words = 1 << (cell_bits - 5);
+  uint16_t* wpre = reinterpret_cast<uint16_t*>(bits + words);
+  uint32_t* slot = reinterpret_cast<uint32_t*>(wpre + words);
   AT* sval = reinterpret_cast<AT*>(smem);              // over all three
   uint32_t* scol = reinterpret_cast<uint32_t*>(smem);  // after the values
-  uint8_t* segof = smem + rank_arena<CAP>();
+  uint8_t* segof = smem + ((rank_arena<CAP>(cell_bits) + 15) & ~size_t(15));
   StageR<VIn>& sg = *reinterpret_cast<StageR<VIn>*>(segof + CAP);
   // the repeats, when they are at most one per thread: product, place
   uint32_t* rep = reinterpret_cast<uint32_t*>(segof + CAP + sizeof(StageR<VIn>));
@@ -2149,7 +2161,7 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, co
     sg.kmax = b_sorted ? 0u : (uint32_t)(B.ncol > 0 ? B.ncol - 1 : 0);
     sg.repeats = 0;
   }
-  for (int i = threadIdx.x; i < kRankWords / 4; i += BLOCK) reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < words / 4; i += BLOCK) reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
   if (FUSED) {
     tick = s_tick;
@@ -2197,8 +2209,8 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, co
   const uint32_t lo = sg.kmin;
   const uint32_t range = sg.kmax > sg.kmin ? sg.kmax - sg.kmin : 0u;
   const int rbits = 32 - __clz(range);
-  const int shift = rbits > kRankCellBits ? rbits - kRankCellBits : 0;
-  if (shift > kRankBits - kRankCellBits) {  // the host takes this kernel for narrower matrices only
+  const int shift = rbits > cell_bits ? rbits - cell_bits : 0;
+  if (shift > 4) {  // the host takes this kernel for narrower matrices only
     give_up();
     return;
   }
@@ -2220,32 +2232,34 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, co
   }
   __syncthreads();
   // 2. ranks of the occupied cells: four words per thread and chunk, the
-  // chunks' counts in the 16-bit fields of one scanned word
-  int distinct;
-  {
+  // counts of WCH chunks in the 16-bit fields of one scanned word
+  int distinct = 0;
+  for (int w0 = 0, round = 0; w0 < nwords; w0 += WCH * 4 * BLOCK, ++round) {
     uint2 pc[WCH];  // set bits before each of the four words
     unsigned long long packed = 0;
 #pragma unroll
     for (int k = 0; k < WCH; ++k) {
       pc[k] = make_uint2(0, 0);
-      if (k * BLOCK * 4 < nwords) {
-        const uint4 w = reinterpret_cast<const uint4*>(bits)[k * BLOCK + threadIdx.x];
+      const int i = (w0 >> 2) + k * BLOCK + threadIdx.x;
+      if (i * 4 < nwords) {
+        const uint4 w = reinterpret_cast<const uint4*>(bits)[i];
         const uint32_t c0 = __popc(w.x), c1 = c0 + __popc(w.y), c2 = c1 + __popc(w.z);
         pc[k] = make_uint2(c0 << 16, c1 | (c2 << 16));
         packed |= (unsigned long long)(c2 + __popc(w.w)) << (16 * k);
       }
     }
     unsigned long long total;
-    const unsigned long long ex = block_exclusive_sum1<BLOCK, unsigned long long>(packed, sg.tmp[1], total);
-    uint32_t base = 0;
+    const unsigned long long ex =
+        block_exclusive_sum1<BLOCK, unsigned long long>(packed, sg.tmp[(round & 1) ^ 1], total);
+    uint32_t base = distinct;
 #pragma unroll
     for (int k = 0; k < WCH; ++k) {
-      if (k * BLOCK * 4 < nwords) {
+      const int i = (w0 >> 2) + k * BLOCK + threadIdx.x;
+      if (i * 4 < nwords) {
         const uint32_t b = base + (uint32_t)((ex >> (16 * k)) & 0xFFFFu);
-        reinterpret_cast<uint2*>(wpre)[k * BLOCK + threadIdx.x] =
-            make_uint2(pc[k].x + b * 0x10001u, pc[k].y + b * 0x10001u);
-        base += (uint32_t)((total >> (16 * k)) & 0xFFFFu);
+        reinterpret_cast<uint2*>(wpre)[i] = make_uint2(pc[k].x + b * 0x10001u, pc[k].y + b * 0x10001u);
       }
+      base += (uint32_t)((total >> (16 * k)) & 0xFFFFu);
     }
     distinct = (int)base;
   }

@@ -75,6 +75,16 @@ def test_product_bounds(ctx, products, ncol):
     check(ctx, A, B)
 
 
+@pytest.mark.parametrize("products", [33, 127, 128, 129, 511, 1023, 1024, 1025, 1535, 2047, 2048])
+@pytest.mark.parametrize("ncol", [300, 1 << 15, (1 << 15) + 1, 1 << 16, (1 << 16) + 1, 600001, 1 << 21])
+def test_small_bins(ctx, products, ncol):
+    """Rows of the 1024 and 2048 bins, at the widths where each starts its second level (2^15 and 2^16 columns)."""
+    entries = 3 if products < 100 else 11
+    per = products // entries
+    A, B = make(entries, per, ncol, last=products - per * (entries - 1), seed=products)
+    check(ctx, A, B)
+
+
 @pytest.mark.parametrize("span", [300, 5000])
 @pytest.mark.parametrize("dtype", [np.float64, np.int32])
 def test_crowded_columns(ctx, span, dtype):
