@@ -82,6 +82,7 @@ struct cas_ctx {
   int esc_max = 8192;                      // ESC rows: at most this many products
   int hash_max = 4096;                     // hash rows: at most this many distinct columns
   int out_blocks = 0;                      // C in host memory: row blocks (0: by C's size)
+  cudaMemPool_t scratch = nullptr;         // the device's scratch pool (scratch_pool_get)
   double mem_share = 1.0;                  // share of the free device memory this context sizes
                                            // its optional scratch by (a batch worker's: 1 / workers)
   double acc_thres = 2.0;
@@ -322,11 +323,67 @@ cas_status free_owned(cas_ctx* ctx, DevMat& m) {
   return CAS_OK;
 }
 
+// Scratch and results come from two stream-ordered pools.  A call frees its
+// scratch in its own order, so with one pool the holes that the last C left
+// were cut up by the next call's scratch, and the pool mapped its memory anew
+// for the next C: a program that keeps three Graph500 scale 17 products paid 6
+// to 25 ms beside each call's 19 for its first fifteen calls; with two pools
+// it pays for the first C of each product only.  Results (C, B = A^T) stay in the device's default pool, where
+// equal sizes find their holes again; scratch has a pool of its own per
+// device, which the contexts of a process share and the last one destroys.  It
+// keeps at most kScratchKeep of the device's memory when idle, and both pools
+// give their idle memory back before an allocation fails.
+constexpr double kScratchKeep = 1.0 / 8;
+constexpr int kMaxDevices = 64;
+struct ScratchPool {
+  cudaMemPool_t pool = nullptr;
+  int users = 0;
+};
+std::mutex g_scratch_mu;
+ScratchPool g_scratch[kMaxDevices];
+
+cas_status scratch_pool_get(cas_ctx* ctx) {
+  if (ctx->device < 0 || ctx->device >= kMaxDevices)
+    return set_err(ctx, CAS_ERR_BAD_INPUT, "device %d is not supported", ctx->device);
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  ScratchPool& sp = g_scratch[ctx->device];
+  if (!sp.pool) {
+    size_t free_b = 0, total_b = 0;
+    CAS_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    CAS_CUDA(ctx, cudaMemPoolCreate(&sp.pool, &props));
+    uint64_t keep = (uint64_t)(kScratchKeep * (double)total_b);
+    const cudaError_t e = cudaMemPoolSetAttribute(sp.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(sp.pool);
+      sp.pool = nullptr;
+      return set_err(ctx, CAS_ERR_CUDA, "scratch pool: %s", cudaGetErrorString(e));
+    }
+  }
+  ++sp.users;
+  ctx->scratch = sp.pool;
+  return CAS_OK;
+}
+
+void scratch_pool_put(cas_ctx* ctx) {
+  if (!ctx->scratch) return;
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  ScratchPool& sp = g_scratch[ctx->device];
+  if (--sp.users == 0) {
+    cudaMemPoolDestroy(sp.pool);  // allocations still in flight keep it until they are freed
+    sp.pool = nullptr;
+  }
+  ctx->scratch = nullptr;
+}
+
 // Device memory a stream-ordered allocation can still get: the device's free
-// memory plus what the pool holds reserved but unused (freed allocations it
-// keeps, since its release threshold is unbounded).  cudaMemGetInfo alone
-// would count the pool's idle reserve as taken, so sizes chosen from it would
-// shrink after every large product.
+// memory plus what the pools hold reserved but unused (freed allocations they
+// keep).  cudaMemGetInfo alone would count the pools' idle reserve as taken, so
+// sizes chosen from it would shrink after every large product.
 double free_device_bytes(cas_ctx* ctx) {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
@@ -334,25 +391,53 @@ double free_device_bytes(cas_ctx* ctx) {
     return 0.0;
   }
   double idle = 0.0;
-  cudaMemPool_t pool;
-  uint64_t reserved = 0, used = 0;  // 64-bit attribute values
-  if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
-    idle = (double)(reserved - used);
+  cudaMemPool_t pools[2] = {nullptr, ctx->scratch};
+  if (cudaDeviceGetDefaultMemPool(&pools[0], ctx->device) != cudaSuccess) pools[0] = nullptr;
+  for (cudaMemPool_t pool : pools) {
+    uint64_t reserved = 0, used = 0;  // 64-bit attribute values
+    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+      idle += (double)(reserved - used);
+  }
   cudaGetLastError();
   return (double)free_b + idle;
 }
 
-cas_status dev_alloc(cas_ctx* ctx, void** p, size_t bytes) {
+// An allocation from `pool` on stream s.  Out of memory, both pools give
+// back what they hold idle, once the stream's pending frees are done, and the
+// allocation is tried again.
+cudaError_t pool_alloc(cas_ctx* ctx, cudaMemPool_t pool, void** p, size_t bytes, cudaStream_t s) {
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
-  if (e != cudaSuccess) {
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    return set_err(ctx, e == cudaErrorMemoryAllocation ? CAS_ERR_OOM : CAS_ERR_CUDA,
-                   "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+    cudaMemPool_t def = nullptr;
+    cudaStreamSynchronize(s);
+    if (cudaDeviceGetDefaultMemPool(&def, ctx->device) == cudaSuccess) cudaMemPoolTrimTo(def, 0);
+    cudaMemPoolTrimTo(ctx->scratch, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
   }
-  return CAS_OK;
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
+cas_status alloc_err(cas_ctx* ctx, cudaError_t e, size_t bytes) {
+  if (e == cudaSuccess) return CAS_OK;
+  return set_err(ctx, e == cudaErrorMemoryAllocation ? CAS_ERR_OOM : CAS_ERR_CUDA,
+                 "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+}
+
+// scratch of a call, on the context's stream or stream s
+cas_status dev_alloc(cas_ctx* ctx, void** p, size_t bytes, cudaStream_t s) {
+  return alloc_err(ctx, pool_alloc(ctx, ctx->scratch, p, bytes, s), bytes);
+}
+cas_status dev_alloc(cas_ctx* ctx, void** p, size_t bytes) { return dev_alloc(ctx, p, bytes, ctx->stream); }
+
+// an array of a result, which outlives the call
+cas_status out_alloc(cas_ctx* ctx, void** p, size_t bytes) {
+  cudaMemPool_t pool = nullptr;
+  CAS_CUDA(ctx, cudaDeviceGetDefaultMemPool(&pool, ctx->device));
+  return alloc_err(ctx, pool_alloc(ctx, pool, p, bytes, ctx->stream), bytes);
 }
 
 // Host memory for C: 2 MiB-aligned and marked for transparent huge pages,
@@ -713,18 +798,23 @@ cas_status join(cas_ctx* ctx) {
   return CAS_OK;
 }
 
+// The per-row arrays of a call, one allocation (row_flp is its start).
 cas_status scratch_alloc(cas_ctx* ctx, Call& c) {
-  CAS_TRY(dev_alloc(ctx, (void**)&c.row_flp, sizeof(int64_t) * (c.m + 1)));
-  CAS_TRY(dev_alloc(ctx, (void**)&c.row_nz, sizeof(int64_t) * (c.m + 1)));
-  CAS_TRY(dev_alloc(ctx, (void**)&c.rows, sizeof(int32_t) * (c.m + 1)));
-  CAS_TRY(dev_alloc(ctx, (void**)&c.ovf, sizeof(int32_t) * (c.m + 1)));
+  const size_t rows8 = (sizeof(int64_t) * (size_t)(c.m + 1) + 255) & ~size_t(255);
+  const size_t rows4 = (sizeof(int32_t) * (size_t)(c.m + 1) + 255) & ~size_t(255);
   c.nparts = (c.m + 1 + cas::kScanTile - 1) / cas::kScanTile;
-  CAS_TRY(dev_alloc(ctx, (void**)&c.partial, sizeof(int64_t) * (c.nparts + 1)));
+  char* p = nullptr;
+  CAS_TRY(dev_alloc(ctx, (void**)&p, 2 * rows8 + 2 * rows4 + sizeof(int64_t) * (size_t)(c.nparts + 1)));
+  c.row_flp = reinterpret_cast<int64_t*>(p);
+  c.row_nz = reinterpret_cast<int64_t*>(p + rows8);
+  c.rows = reinterpret_cast<int32_t*>(p + 2 * rows8);
+  c.ovf = reinterpret_cast<int32_t*>(p + 2 * rows8 + rows4);
+  c.partial = reinterpret_cast<int64_t*>(p + 2 * rows8 + 2 * rows4);
   return CAS_OK;
 }
 
 cas_status scratch_free(cas_ctx* ctx, Call& c) {
-  void* ps[] = {c.row_flp, c.row_nz, c.rows, c.ovf, c.partial, c.frows, c.fpos, c.fstatus, c.dbits, c.dslot};
+  void* ps[] = {c.row_flp, c.frows, c.fpos, c.fstatus, c.dbits, c.dslot};
   for (void* p : ps)
     if (p) CAS_CUDA(ctx, cudaFreeAsync(p, ctx->stream));
   c.row_flp = c.row_nz = nullptr;
@@ -889,12 +979,7 @@ cas_status symb_split_heavy(cas_ctx* ctx, Call& c, int32_t*& rows, int64_t& n, i
   const int64_t max_slices = (c.ncol + kRankCols - 1) / kRankCols;
   const int64_t cap = (int64_t)((double)kSplitScratch * ctx->mem_share) / (max_slices * (kRankCols / 8));
   auto alloc = [&](void** p, size_t bytes) -> cas_status {
-    cudaError_t e = cudaMallocAsync(p, bytes ? bytes : 16, s);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return set_err(ctx, e == cudaErrorMemoryAllocation ? CAS_ERR_OOM : CAS_ERR_CUDA,
-                     "device allocation of %zu bytes for the split rows failed", bytes);
-    }
+    CAS_TRY(dev_alloc(ctx, p, bytes, s));
     c.heavy_tmp.push_back(*p);
     return CAS_OK;
   };
@@ -1111,12 +1196,7 @@ cas_status launch_heavy_split(cas_ctx* ctx, Call& c, const int32_t* rows, int64_
   hp.max_slices = (int)((c.ncol + kRankCols - 1) / kRankCols);
   std::vector<void*> tmp;
   auto alloc = [&](void** p, size_t bytes) -> cas_status {
-    cudaError_t e = cudaMallocAsync(p, bytes ? bytes : 16, s);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return set_err(ctx, e == cudaErrorMemoryAllocation ? CAS_ERR_OOM : CAS_ERR_CUDA,
-                     "device allocation of %zu bytes for the split rows failed", bytes);
-    }
+    CAS_TRY(dev_alloc(ctx, p, bytes, s));
     tmp.push_back(*p);
     return CAS_OK;
   };
@@ -1313,7 +1393,7 @@ cas_status compute_dev(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, De
   CAS_TRY(phase_init(ctx, c, validate));
   CAS_CUDA(ctx, cudaEventRecord(ctx->ev_phase[1], ctx->stream));
   // SYMB
-  CAS_TRY(dev_alloc(ctx, (void**)&o.crp, sizeof(int64_t) * (c.m + 1)));
+  CAS_TRY(out_alloc(ctx, (void**)&o.crp, sizeof(int64_t) * (c.m + 1)));
   CAS_TRY(launch_symb_bins(ctx, c, c.row_nz));
   CAS_TRY(launch_scan(ctx, o.crp, c.row_nz, c.m + 1, c.partial,
                       reinterpret_cast<int64_t*>(ctx->d_counts + kSlotNnz)));
@@ -1326,8 +1406,8 @@ cas_status compute_dev(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, De
   const int64_t cap = o.nnz_known + (c.nf > 0 ? c.f_bound : 0);
   CAS_CUDA(ctx, cudaEventRecord(ctx->ev_phase[2], ctx->stream));
   // MGMT
-  CAS_TRY(dev_alloc(ctx, (void**)&o.ccol, sizeof(int32_t) * cap));
-  CAS_TRY(dev_alloc(ctx, &o.cval, vbytes * cap));
+  CAS_TRY(out_alloc(ctx, (void**)&o.ccol, sizeof(int32_t) * cap));
+  CAS_TRY(out_alloc(ctx, &o.cval, vbytes * cap));
   CAS_TRY(at_cap(cap));
   CAS_TRY(numc_bins(ctx, c, o.crp, mode_of(accum)));
   CAS_CUDA(ctx, cudaEventRecord(ctx->ev_phase[3], ctx->stream));
@@ -1780,6 +1860,7 @@ cas_status cas_create(int device, cas_ctx** out) {
     CAS_CUDA(ctx, cudaDeviceGetDefaultMemPool(&pool, device));
     uint64_t thresh = UINT64_MAX;
     CAS_CUDA(ctx, cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thresh));
+    CAS_TRY(scratch_pool_get(ctx));
     CAS_TRY(setup_kernels(ctx));
     return CAS_OK;
   }();
@@ -1839,6 +1920,7 @@ void cas_destroy(cas_ctx* ctx) {
     for (auto& b : ctx->host_free) free(b.first);
   }
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+  scratch_pool_put(ctx);
   delete ctx;
 }
 

@@ -206,19 +206,21 @@ cas_status transpose_device(cas_ctx* ctx, const DevMat& A, int vt, cas_csr* B, b
   auto release = [&]() {
     for (void* p : tmp) cudaFreeAsync(p, ctx->stream);
   };
+  // all from the results' pool: B comes first, so the scratch cuts up none of
+  // its holes
   cas_status rc = [&]() -> cas_status {
-    CAS_TRY(dev_alloc(ctx, (void**)&brp, sizeof(int64_t) * (size_t)(n + 1)));
-    CAS_TRY(dev_alloc(ctx, (void**)&bcol, sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1)));
-    CAS_TRY(dev_alloc(ctx, &bval, vbytes * (size_t)(nnz > 0 ? nnz : 1)));
-    CAS_TRY(dev_alloc(ctx, (void**)&cnt, sizeof(int64_t) * (size_t)(n + 1)));
+    CAS_TRY(out_alloc(ctx, (void**)&brp, sizeof(int64_t) * (size_t)(n + 1)));
+    CAS_TRY(out_alloc(ctx, (void**)&bcol, sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1)));
+    CAS_TRY(out_alloc(ctx, &bval, vbytes * (size_t)(nnz > 0 ? nnz : 1)));
+    CAS_TRY(out_alloc(ctx, (void**)&cnt, sizeof(int64_t) * (size_t)(n + 1)));
     tmp.push_back(cnt);
-    CAS_TRY(dev_alloc(ctx, (void**)&partial, sizeof(int64_t) * (size_t)((n + 1 + cas::kScanTile - 1) / cas::kScanTile + 1)));
+    CAS_TRY(out_alloc(ctx, (void**)&partial, sizeof(int64_t) * (size_t)((n + 1 + cas::kScanTile - 1) / cas::kScanTile + 1)));
     tmp.push_back(partial);
-    CAS_TRY(dev_alloc(ctx, (void**)&key, sizeof(unsigned long long) * (size_t)(nnz > 0 ? nnz : 1)));
+    CAS_TRY(out_alloc(ctx, (void**)&key, sizeof(unsigned long long) * (size_t)(nnz > 0 ? nnz : 1)));
     tmp.push_back(key);
-    CAS_TRY(dev_alloc(ctx, (void**)&aux, sizeof(unsigned long long) * (size_t)(nnz > 0 ? nnz : 1)));
+    CAS_TRY(out_alloc(ctx, (void**)&aux, sizeof(unsigned long long) * (size_t)(nnz > 0 ? nnz : 1)));
     tmp.push_back(aux);
-    CAS_TRY(dev_alloc(ctx, (void**)&big, sizeof(int32_t) * (size_t)(n > 0 ? n : 1)));
+    CAS_TRY(out_alloc(ctx, (void**)&big, sizeof(int32_t) * (size_t)(n > 0 ? n : 1)));
     tmp.push_back(big);
     CAS_CUDA(ctx, cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (size_t)(n + 1), ctx->stream));
     CAS_CUDA(ctx, cudaMemsetAsync(nbig, 0, sizeof(unsigned int), ctx->stream));
