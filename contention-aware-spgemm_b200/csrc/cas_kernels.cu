@@ -240,21 +240,30 @@ k_scan_apply(const int64_t* __restrict__ in, int64_t n_in, const int64_t* __rest
 }
 
 // ============================================================ row expansion
-// Enumerates the products of one row of A*B inside a thread block: A entries
-// are staged min(BLOCK, kAChunk) at a time (B row start, length, A value), their lengths
-// scanned, and each thread then takes products p = tid, tid+BLOCK, ... and
-// finds its A entry by binary search, so work is balanced whatever the B row
-// lengths.  Loads of U products are issued before any is consumed.  With
-// `ranged`, every B row is cut to the columns [c0, c1) by binary search (B
-// rows sorted); otherwise f receives every product.
+// Enumerates the products of one row of A*B inside a thread block.  A entries
+// are staged min(BLOCK, kAChunk) at a time, those with an empty B row left
+// out: where the B row starts, its first product, the A value.  The chunk's
+// products are split evenly over the warps, which walk their part 32
+// consecutive products at a time: the lanes look at the next 32 entries'
+// first products, an OR over the warp marks those that start among these 32
+// products, and a product's entry is the running entry plus the marks up to
+// its lane.  So no product searches for its entry, the B rows' lengths do not
+// matter, and a warp's loads are consecutive.  Loads of four groups of 32 are
+// issued before any is consumed.  With `ranged`, every B row is cut to the
+// columns [c0, c1) by binary search (B rows sorted); otherwise f receives
+// every product.  (Finding each product's entry from an interpolated guess,
+// checked and repaired by binary search, took 125 to 170 instructions per 32
+// products in the dense kernels and bound them, issue slots 80% busy; the
+// symbolic dense kernels of Graph500 scale 17 took 4.4 ms that way and take
+// 2.1, those of a join matrix of 600000 rows 7.5 and 4.1.)
 constexpr int kAChunk = 256;
 constexpr int kUnroll = 8;
 
 template <typename VIn>
 struct alignas(16) Stage {
-  int64_t bs[kAChunk];
-  int64_t pre[kAChunk + 1];
+  int64_t off[kAChunk];       // first element of the B row less its first product: product p is element off + p
   VIn av[kAChunk];
+  uint32_t pre[kAChunk + 1];  // first product of each entry, then the chunk's products
   long long tmp[33];
 };
 
@@ -264,78 +273,95 @@ __device__ __forceinline__ int64_t expand_entries(const Csr& A, const Csr& B, in
   const VIn* __restrict__ aval = static_cast<const VIn*>(A.val);
   const VIn* __restrict__ bval = static_cast<const VIn*>(B.val);
   constexpr int ACH = BLOCK < kAChunk ? BLOCK : kAChunk;  // one staged A entry per thread
+  constexpr int NW = BLOCK / 32;
+  constexpr int U = 4;                  // groups of 32 products in flight per warp
+  constexpr long long kOne = 1ll << 40;  // an entry in the scanned word, above the products
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned upto = (lanemask_lt() << 1) | 1u;
   int64_t pbase = 0;
   for (int64_t a0 = as; a0 < ae; a0 += ACH) {
     const int na = (int)((ae - a0) < (int64_t)ACH ? (ae - a0) : (int64_t)ACH);
     long long len = 0;
+    int64_t lo = 0;
     if (threadIdx.x < na) {
       const int32_t k = A.col[a0 + threadIdx.x];
-      int64_t lo = B.rp[k], hi = B.rp[k + 1];
+      lo = B.rp[k];
+      int64_t hi = B.rp[k + 1];
       if (ranged) {
         lo = lower_bound_g(B.col, lo, hi, c0);
         hi = lower_bound_g(B.col, lo, hi, c1);
       }
-      sg.bs[threadIdx.x] = lo;
       len = hi - lo;
-      if (NEED_VAL) sg.av[threadIdx.x] = aval[a0 + threadIdx.x];
     }
-    long long total;
-    const long long ex = block_exclusive_sum<BLOCK, long long>(len, sg.tmp, total);
-    if (threadIdx.x < ACH) sg.pre[threadIdx.x] = ex;
-    if (threadIdx.x == 0) sg.pre[na] = total;
-    __syncthreads();
-    // A entry of product p: the interpolated guess p * na / total, checked
-    // with its neighbours (exact for rows of near-equal B row lengths), else
-    // a binary search for the last entry whose prefix is <= p.
-    const float per = total > 0 ? (float)na / (float)total : 0.f;
-    for (int64_t p0 = threadIdx.x; p0 < total; p0 += (int64_t)BLOCK * kUnroll) {
-      int32_t key[kUnroll];
-      VIn bv[kUnroll];
-      int sgi[kUnroll];
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int64_t p = p0 + (int64_t)u * BLOCK;
-        sgi[u] = -1;
-        if (p < total) {
-          int s = min(na - 1, (int)((float)p * per));
-          if (sg.pre[s] > p) {
-            if (s > 0 && sg.pre[s - 1] <= p) {
-              --s;
-            } else {
-              int lo = 0, hi = s;
-              while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (sg.pre[mid] <= p) lo = mid; else hi = mid;
-              }
-              s = lo;
-            }
-          } else if (sg.pre[s + 1] <= p) {
-            if (sg.pre[s + 2] > p) {
-              ++s;
-            } else {
-              int lo = s + 2, hi = na;
-              while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (sg.pre[mid] <= p) lo = mid; else hi = mid;
-              }
-              s = lo;
-            }
-          }
-          const int lo = s;
-          const int64_t j = sg.bs[lo] + (p - sg.pre[lo]);
-          key[u] = __ldg(B.col + j);
-          if (NEED_VAL) bv[u] = __ldg(bval + j);
-          sgi[u] = lo;
+    long long sum;
+    const long long ex = block_exclusive_sum<BLOCK, long long>(len > 0 ? len + kOne : 0, sg.tmp, sum);
+    const int ne = (int)(sum >> 40);
+    const int64_t total = sum & (kOne - 1);
+    if (total < (int64_t(1) << 30)) {
+      if (len > 0) {
+        const int e = (int)(ex >> 40);
+        const int64_t first = ex & (kOne - 1);
+        sg.off[e] = lo - first;
+        sg.pre[e] = (uint32_t)first;
+        if (NEED_VAL) sg.av[e] = aval[a0 + threadIdx.x];
+      }
+      if (threadIdx.x == 0) sg.pre[ne] = (uint32_t)total;
+      __syncthreads();
+      const uint32_t tot = (uint32_t)total, groups = (tot + 31) >> 5;
+      const uint32_t g1 = (uint32_t)((uint64_t)groups * (warp + 1) / NW);
+      uint32_t g = (uint32_t)((uint64_t)groups * warp / NW);
+      int e0 = 0;  // the first entry that starts at or after the group
+      {
+        int h = ne;
+        while (e0 < h) {
+          const int mid = (e0 + h) >> 1;
+          if (sg.pre[mid] < (g << 5)) e0 = mid + 1; else h = mid;
         }
       }
+      for (; g < g1; g += U) {
+        int32_t key[U];
+        VIn bv[U];
+        int en[U];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        if (sgi[u] >= 0) {
-          if (!ranged || (key[u] >= c0 && key[u] < c1)) {
-            if (NEED_VAL) f(key[u], sg.av[sgi[u]], bv[u], pbase + p0 + (int64_t)u * BLOCK);
-            else f(key[u], VIn(0), VIn(0), pbase + p0 + (int64_t)u * BLOCK);
+        for (int u = 0; u < U; ++u) {
+          en[u] = -1;
+          if (g + u < g1) {
+            const uint32_t t = (g + u) << 5;
+            const uint32_t d = sg.pre[min(e0 + lane, ne)] - t;
+            const unsigned starts = __reduce_or_sync(kFull, d < 32u ? 1u << d : 0u);
+            const int e = e0 + __popc(starts & upto) - 1;
+            e0 += __popc(starts);
+            if (t + lane < tot) {
+              const int64_t j = sg.off[e] + (t + lane);
+              key[u] = __ldg(B.col + j);
+              if (NEED_VAL) bv[u] = __ldg(bval + j);
+              en[u] = e;
+            }
           }
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (en[u] >= 0 && (!ranged || (key[u] >= c0 && key[u] < c1))) {
+            const int64_t p = pbase + (int64_t)(((g + u) << 5) + lane);
+            if (NEED_VAL) f(key[u], sg.av[en[u]], bv[u], p);
+            else f(key[u], VIn(0), VIn(0), p);
+          }
+        }
+      }
+    } else {
+      // too many products for 32-bit positions: the entries one after another
+      int64_t before = 0;
+      for (int i = 0; i < na; ++i) {
+        const int32_t k = A.col[a0 + i];
+        int64_t l = B.rp[k], h = B.rp[k + 1];
+        if (ranged) {
+          l = lower_bound_g(B.col, l, h, c0);
+          h = lower_bound_g(B.col, l, h, c1);
+        }
+        const VIn av = NEED_VAL ? aval[a0 + i] : VIn(0);
+        for (int64_t j = l + threadIdx.x; j < h; j += BLOCK)
+          f(__ldg(B.col + j), av, NEED_VAL ? __ldg(bval + j) : VIn(0), pbase + before + (j - l));
+        before += h - l;
       }
     }
     pbase += total;
@@ -469,8 +495,8 @@ k_symb_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
     bool bad = false;
     expand_row<BLOCK, false, double>(A, B, r, sg, multi, (int32_t)c0, (int32_t)c1,
                                      [&](int32_t key, double, double, int64_t) {
-      const int64_t idx = (int64_t)key - c0;
-      if (idx < 0 || idx >= kDenseChunkBits) { bad = true; return; }
+      const uint32_t idx = (uint32_t)key - (uint32_t)c0;
+      if (idx >= kDenseChunkBits) { bad = true; return; }
       atomicOr(&bm[idx >> 5], 1u << (idx & 31));
     });
     if (bad && !multi) dev_report(st, kDevBadIndex, 3, r);
@@ -2591,8 +2617,8 @@ k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
       __syncthreads();
       expand_row<BLOCK, false, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1,
                                     [&](int32_t key, VIn, VIn, int64_t) {
-        const int64_t idx = (int64_t)key - s0;
-        if (idx >= 0 && idx < kRankCols) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
+        const uint32_t idx = (uint32_t)key - (uint32_t)s0;
+        if (idx < kRankCols) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
       });
       __syncthreads();
     }
@@ -2633,11 +2659,11 @@ k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
     __syncthreads();  // the zeroed values are visible to the block's atomic adds
     expand_row<BLOCK, true, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1,
                                  [&](int32_t key, VIn av, VIn bv, int64_t) {
-      const int64_t idx = (int64_t)key - s0;
-      if (idx < 0 || idx >= kRankCols) return;
-      const int w = (int)(idx >> 5);
-      const int64_t pos = (int64_t)gbase[w >> 3] + wrank[w] + __popc(bm[w] & ((1u << (idx & 31)) - 1u));
-      if (pos < room) Acc<VIn>::atomic_add(&cval[base + pos], Acc<VIn>::mul(av, bv));
+      const uint32_t idx = (uint32_t)key - (uint32_t)s0;
+      if (idx >= kRankCols) return;
+      const uint32_t w = idx >> 5;
+      const uint32_t pos = gbase[w >> 3] + wrank[w] + __popc(bm[w] & ((1u << (idx & 31)) - 1u));
+      if ((int64_t)pos < room) Acc<VIn>::atomic_add(&cval[base + pos], Acc<VIn>::mul(av, bv));
     });
     written += run;
     __syncthreads();
@@ -2788,8 +2814,8 @@ k_dense_setup(HeavyPlan hp, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, cons
       for (int w = threadIdx.x; w < nw; w += BLOCK) bm[w] = 0u;
       __syncthreads();
       expand_row<BLOCK, false, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1, [&](int32_t key, VIn, VIn, int64_t) {
-        const int64_t idx = (int64_t)key - s0;
-        if (idx >= 0 && idx < kRankCols) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
+        const uint32_t idx = (uint32_t)key - (uint32_t)s0;
+        if (idx < kRankCols) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
       });
       __syncthreads();
     }
@@ -2875,12 +2901,12 @@ k_dense_acc(HeavyPlan hp, Csr A, Csr B, const int64_t* __restrict__ crp, typenam
       const int64_t base = c0r + sb;
       expand_entries<BLOCK, true, VIn>(A, B, a0, a1, sg, ns > 1, (int32_t)s0, (int32_t)s1,
                                        [&](int32_t key, VIn av, VIn bv, int64_t) {
-        const int64_t idx = (int64_t)key - s0;
-        if (idx < 0 || idx >= s1 - s0) return;
-        const int w = (int)(idx >> 5);
+        const uint32_t idx = (uint32_t)key - (uint32_t)s0;
+        if (idx >= (uint32_t)(s1 - s0)) return;
+        const uint32_t w = idx >> 5;
         const uint32_t m = bm[w];
         if (!((m >> (idx & 31)) & 1u)) return;  // cannot happen for a consistent bitmap
-        const int64_t pos = (int64_t)gbase[w >> 3] + wrank[w] + __popc(m & ((1u << (idx & 31)) - 1u));
+        const uint32_t pos = gbase[w >> 3] + wrank[w] + __popc(m & ((1u << (idx & 31)) - 1u));
         Acc<VIn>::atomic_add(&cval[base + pos], Acc<VIn>::mul(av, bv));
       });
       __syncthreads();
@@ -2999,8 +3025,8 @@ k_heavy_bits(HeavyPlan hp, Csr A, Csr B, DevStatus* st) {
       __syncthreads();
       expand_entries<BLOCK, false, double>(A, B, a0, a1, sg, ns > 1, (int32_t)s0, (int32_t)s1,
                                            [&](int32_t key, double, double, int64_t) {
-        const int64_t idx = (int64_t)key - s0;
-        if (idx >= 0 && idx < s1 - s0) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
+        const uint32_t idx = (uint32_t)key - (uint32_t)s0;
+        if (idx < (uint32_t)(s1 - s0)) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
       });
       __syncthreads();
       uint32_t* g = hp.bits + ((size_t)i * hp.max_slices + sl) * NWORD;

@@ -1,0 +1,41 @@
+"""GPU: the block-wide walk over a row's products (hash and dense rows, both phases).
+
+B row lengths at the edges of the walk's groups of 32 products (empty rows, one entry, 31 to 33, 64, thousands), one
+to several staged chunks of 256 A entries, rows ending on a group and off it.  Whole-number values: bit for bit.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from matrices import from_coo
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = {"ones": [1], "with_empty": [0, 1, 0, 0, 33], "group_edges": [31, 32, 33, 64], "mixed": [0, 5, 2000, 1, 96],
+           "long": [3000, 0, 31]}
+
+
+def product(lengths, entries, ncol, dtype, seed):
+    rng = np.random.default_rng(seed)
+    mid, rows = 700, 6
+    lens = np.resize(lengths, mid)
+    A = from_coo(rows, mid, np.repeat(np.arange(rows), entries),
+                 np.concatenate([rng.choice(mid, entries, replace=False) for _ in range(rows)]),
+                 rng.integers(1, 8, rows * entries), dtype)
+    cols = np.concatenate([np.sort(rng.choice(ncol, n, replace=False)) for n in lens])
+    B = from_coo(mid, ncol, np.repeat(np.arange(mid), lens), cols, rng.integers(1, 8, len(cols)), dtype)
+    return A, B
+
+
+@pytest.mark.parametrize("lengths", sorted(LENGTHS))
+@pytest.mark.parametrize("entries", [1, 31, 255, 256, 257, 600])
+@pytest.mark.parametrize("algo,ncol,dtype", [("hash", 4000, np.float64), ("hash", 4000, np.int32),
+                                             ("hsersc", 700001, np.float64)])
+def test_walk(ctx, lengths, entries, algo, ncol, dtype):
+    A, B = product(LENGTHS[lengths], entries, ncol, dtype, entries)
+    out = ctx.spgemm(A, B, algo)
+    rp, cols, vals, flop = oracle.oracle_spgemm(A, B, algo)
+    assert out.stats["flop"] == flop
+    np.testing.assert_array_equal(out.csr.row_ptrs, rp)
+    np.testing.assert_array_equal(out.csr.cols.astype(np.int64), cols)
+    np.testing.assert_array_equal(out.csr.vals.astype(np.float64), vals)
