@@ -255,7 +255,7 @@ k_scan_apply(const int64_t* __restrict__ in, int64_t n_in, const int64_t* __rest
 // checked and repaired by binary search, took 125 to 170 instructions per 32
 // products in the dense kernels and bound them, issue slots 80% busy; the
 // symbolic dense kernels of Graph500 scale 17 took 4.4 ms that way and take
-// 2.1, those of a join matrix of 600000 rows 7.5 and 4.1.)
+// 1.8, those of a join matrix of 600000 rows 7.5 and 3.5.)
 constexpr int kAChunk = 256;
 constexpr int kUnroll = 8;
 
@@ -276,8 +276,10 @@ __device__ __forceinline__ int64_t expand_entries(const Csr& A, const Csr& B, in
   constexpr int NW = BLOCK / 32;
   constexpr int U = 4;                  // groups of 32 products in flight per warp
   constexpr long long kOne = 1ll << 40;  // an entry in the scanned word, above the products
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned upto = (lanemask_lt() << 1) | 1u;
+  const int warp = threadIdx.x >> 5;
+  uint32_t lane;  // volatile: kept in a register, not read again for every group
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  const unsigned upto = 0xFFFFFFFFu >> (31 - lane);
   int64_t pbase = 0;
   for (int64_t a0 = as; a0 < ae; a0 += ACH) {
     const int na = (int)((ae - a0) < (int64_t)ACH ? (ae - a0) : (int64_t)ACH);
@@ -318,34 +320,39 @@ __device__ __forceinline__ int64_t expand_entries(const Csr& A, const Csr& B, in
           if (sg.pre[mid] < (g << 5)) e0 = mid + 1; else h = mid;
         }
       }
-      for (; g < g1; g += U) {
+      // entry of this lane's product of the group at t; e0 moves on
+      auto entry = [&](uint32_t t) -> uint32_t {
+        const uint32_t d = sg.pre[min(e0 + (int)lane, ne)] - t;
+        const unsigned starts = __reduce_or_sync(kFull, d < 32u ? 1u << d : 0u);
+        const int e = e0 + __popc(starts & upto) - 1;
+        e0 += __popc(starts);
+        return (uint32_t)e;
+      };
+      auto product = [&](uint32_t p, uint32_t e, int32_t key, VIn bv) {
+        if (NEED_VAL) f(key, sg.av[e], bv, pbase + p);
+        else f(key, VIn(0), VIn(0), pbase + p);
+      };
+      const uint32_t full = g1 < (tot >> 5) ? g1 : tot >> 5;  // groups of 32 products
+      for (; g + U <= full; g += U) {
         int32_t key[U];
         VIn bv[U];
-        int en[U];
+        uint32_t en[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          en[u] = -1;
-          if (g + u < g1) {
-            const uint32_t t = (g + u) << 5;
-            const uint32_t d = sg.pre[min(e0 + lane, ne)] - t;
-            const unsigned starts = __reduce_or_sync(kFull, d < 32u ? 1u << d : 0u);
-            const int e = e0 + __popc(starts & upto) - 1;
-            e0 += __popc(starts);
-            if (t + lane < tot) {
-              const int64_t j = sg.off[e] + (t + lane);
-              key[u] = __ldg(B.col + j);
-              if (NEED_VAL) bv[u] = __ldg(bval + j);
-              en[u] = e;
-            }
-          }
+          const uint32_t t = (g + u) << 5;
+          en[u] = entry(t);
+          const int64_t j = sg.off[en[u]] + (t + lane);
+          key[u] = __ldg(B.col + j);
+          if (NEED_VAL) bv[u] = __ldg(bval + j);
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (en[u] >= 0 && (!ranged || (key[u] >= c0 && key[u] < c1))) {
-            const int64_t p = pbase + (int64_t)(((g + u) << 5) + lane);
-            if (NEED_VAL) f(key[u], sg.av[en[u]], bv[u], p);
-            else f(key[u], VIn(0), VIn(0), p);
-          }
+        for (int u = 0; u < U; ++u) product(((g + u) << 5) + lane, en[u], key[u], NEED_VAL ? bv[u] : VIn(0));
+      }
+      for (; g < g1; ++g) {
+        const uint32_t p = (g << 5) + lane, e = entry(g << 5);
+        if (p < tot) {
+          const int64_t j = sg.off[e] + p;
+          product(p, e, __ldg(B.col + j), NEED_VAL ? __ldg(bval + j) : VIn(0));
         }
       }
     } else {
