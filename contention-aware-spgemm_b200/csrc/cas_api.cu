@@ -204,10 +204,10 @@ constexpr size_t smem_numc_hash() {
   return (size_t(1) << TBITS) * (4 + sizeof(typename cas::Acc<VIn>::T)) + (size_t(1) << (TBITS - 1)) * 8 +
          sizeof(cas::SortScratch<BLOCK>) + sizeof(cas::Stage<VIn>);
 }
-template <int BLOCK, typename VIn>
-constexpr size_t smem_numc_dense() {
-  return size_t(cas::kRankCols / 32) * 4 + size_t(cas::kRankCols / 256) * 4 + size_t(cas::kRankCols / 32) * 2 +
-         sizeof(cas::Stage<VIn>);
+// Bitmap words of the widest slice of a matrix of ncol columns.
+int dense_words(int64_t ncol) {
+  const int64_t cols = std::min<int64_t>(std::max<int64_t>(ncol, 1), cas::kRankCols);
+  return (int)((cols + 255) / 256) * 8;
 }
 
 template <int CAP, int NBB, typename VIn>
@@ -284,9 +284,10 @@ cas_status setup_numc_kernels(cas_ctx* ctx) {
   CAS_TRY(allow_smem(ctx, k_numc_hash<256, 9, VIn>, smem_numc_hash<256, 9, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_hash<256, 11, VIn>, smem_numc_hash<256, 11, VIn>()));
   CAS_TRY(allow_smem(ctx, k_numc_hash<512, 13, VIn>, smem_numc_hash<512, 13, VIn>()));
-  CAS_TRY(allow_smem(ctx, k_numc_dense<512, VIn>, smem_numc_dense<512, VIn>()));
-  CAS_TRY(allow_smem(ctx, k_dense_setup<512, VIn>, smem_numc_dense<512, VIn>()));
-  CAS_TRY(allow_smem(ctx, k_dense_acc<512, VIn>, smem_numc_dense<512, VIn>()));
+  const size_t dense = DenseSmem<VIn>::bytes(kRankCols / 32);
+  CAS_TRY(allow_smem(ctx, k_numc_dense<512, VIn>, dense));
+  CAS_TRY(allow_smem(ctx, k_dense_setup<512, VIn>, dense));
+  CAS_TRY(allow_smem(ctx, k_dense_acc<512, VIn>, dense));
   return CAS_OK;
 }
 
@@ -1212,18 +1213,18 @@ cas_status launch_heavy_split(cas_ctx* ctx, Call& c, const int32_t* rows, int64_
     CAS_TRY(alloc((void**)&hp.apre, sizeof(int64_t) * (size_t)(c.A.nnz > 0 ? c.A.nnz : 1)));
     CAS_TRY(alloc((void**)&hp.ticket, sizeof(unsigned long long)));
     CAS_CUDA(ctx, cudaMemsetAsync(hp.ticket, 0, sizeof(unsigned long long), s));
-    k_dense_setup<512, VIn><<<(unsigned)n, 512, smem_numc_dense<512, VIn>(), s>>>(
-        hp, c.A.csr, c.B.csr, c.ncol, c.b_sorted ? 1 : 0, crp, ccol, cval, c.dbits, c.dslot, c.saved_slices, c.hbits,
+    const int words = dense_words(c.ncol);
+    const size_t smem = DenseSmem<VIn>::bytes(words);
+    k_dense_setup<512, VIn><<<(unsigned)n, 512, smem, s>>>(
+        hp, c.A.csr, c.B.csr, c.ncol, c.b_sorted ? 1 : 0, words, crp, ccol, cval, c.dbits, c.dslot, c.saved_slices, c.hbits,
         c.hslot, ctx->d_status);
     CAS_TRY(check_launch(ctx, "k_dense_setup"));
     k_scan_one_block<<<1, 1024, 0, s>>>(hp.nparts, n, hp.parts);
     CAS_TRY(check_launch(ctx, "k_scan_one_block"));
     int per_sm = 0;
-    CAS_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_acc<512, VIn>, 512,
-                                                                smem_numc_dense<512, VIn>()));
+    CAS_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_acc<512, VIn>, 512, smem));
     const int grid = std::max(1, per_sm) * ctx->sm_count;
-    k_dense_acc<512, VIn><<<grid, 512, smem_numc_dense<512, VIn>(), s>>>(hp, c.A.csr, c.B.csr, crp, cval,
-                                                                       ctx->d_status);
+    k_dense_acc<512, VIn><<<grid, 512, smem, s>>>(hp, c.A.csr, c.B.csr, words, crp, cval, ctx->d_status);
     CAS_TRY(check_launch(ctx, "k_dense_acc"));
     return CAS_OK;
   }();
@@ -1305,10 +1306,12 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
         if (!ctx->heavy_split) n_split = 0;
         ctx->stats.split_rows = n_split;
         if (n_split > 0) CAS_TRY(launch_heavy_split<VIn>(ctx, c, rows, n_split, crp, ccol, cval, s));
-        if (n > n_split)
-          k_numc_dense<512, VIn><<<(unsigned)(n - n_split), 512, smem_numc_dense<512, VIn>(), s>>>(
-              rows + n_split, A, B, c.ncol, c.b_sorted ? 1 : 0, crp, ccol, cval, c.dbits, c.dslot, c.saved_slices,
-              ctx->d_status);
+        if (n > n_split) {
+          const int words = dense_words(c.ncol);
+          k_numc_dense<512, VIn><<<(unsigned)(n - n_split), 512, DenseSmem<VIn>::bytes(words), s>>>(
+              rows + n_split, A, B, c.ncol, c.b_sorted ? 1 : 0, words, crp, ccol, cval, c.dbits, c.dslot,
+              c.saved_slices, ctx->d_status);
+        }
         break;
       }
     }

@@ -250,12 +250,12 @@ k_scan_apply(const int64_t* __restrict__ in, int64_t n_in, const int64_t* __rest
 // its lane.  So no product searches for its entry, the B rows' lengths do not
 // matter, and a warp's loads are consecutive.  Loads of four groups of 32 are
 // issued before any is consumed.  With `ranged`, every B row is cut to the
-// columns [c0, c1) by binary search (B rows sorted); otherwise f receives
-// every product.  (Finding each product's entry from an interpolated guess,
-// checked and repaired by binary search, took 125 to 170 instructions per 32
-// products in the dense kernels and bound them, issue slots 80% busy; the
-// symbolic dense kernels of Graph500 scale 17 took 4.4 ms that way and take
-// 1.8, those of a join matrix of 600000 rows 7.5 and 3.5.)
+// columns [c0, c1) by binary search (B rows sorted); otherwise f receives every
+// product.  (Finding each product's entry from an interpolated guess, checked
+// and repaired by binary search, took 125 to 170 instructions per 32 products
+// in the dense kernels and bound them, issue slots 80% busy; the symbolic
+// dense kernels of Graph500 scale 17 took 4.4 ms that way and take 1.8, those
+// of a join matrix of 600000 rows 7.5 and 3.5.)
 constexpr int kAChunk = 256;
 constexpr int kUnroll = 8;
 
@@ -2582,29 +2582,131 @@ k_numc_hash(const int32_t* __restrict__ rows, Csr A, Csr B, const int64_t* __res
   if (threadIdx.x == 0 && n != nz) dev_report(st, n > nz ? kDevRowOverflow : kDevRowUnderflow, 12, r);
 }
 
+// Word ranks of a slice bitmap in shared memory: for each word the set bits
+// of the words before it in its group of 8 (wrank) and the set bits before
+// the group (gbase); returns the slice's set bits.
+template <int BLOCK>
+__device__ __forceinline__ long long slice_ranks(const uint32_t* __restrict__ bm, int nw, uint32_t* __restrict__ gbase,
+                                                 uint8_t* __restrict__ wrank, long long* tmp) {
+  const int ng = (nw + 7) >> 3;
+  long long run = 0;
+  for (int g0 = 0; g0 < ng; g0 += BLOCK) {
+    const int g = g0 + threadIdx.x;
+    int cnt = 0;
+    if (g < ng) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int w = g * 8 + k;
+        wrank[w] = (uint8_t)cnt;
+        cnt += w < nw ? __popc(bm[w]) : 0;
+      }
+    }
+    long long tot;
+    const long long ex = block_exclusive_sum<BLOCK, long long>((long long)cnt, tmp, tot);
+    if (g < ng) gbase[g] = (uint32_t)(run + ex);
+    run += tot;
+  }
+  __syncthreads();
+  return run;
+}
+
+// The last word w in [w0, nw] with at most `limit` set bits before it.
+__device__ __forceinline__ int word_at_rank(const uint32_t* __restrict__ gbase, const uint8_t* __restrict__ wrank, int w0,
+                                            int nw, uint32_t cnt, uint32_t limit) {
+  if (cnt <= limit) return nw;
+  int l = w0, h = nw;  // l: at most limit before it; h: more
+  while (h - l > 1) {
+    const int mid = (l + h) >> 1;
+    if (gbase[mid >> 3] + wrank[mid] <= limit) l = mid; else h = mid;
+  }
+  return l;
+}
+
+constexpr int kDenseTile = 4096;  // columns
+// The slice's cnt columns to out, in order, through a tile of kDenseTile
+// columns in shared memory: the words' bits land scattered there, and leave in
+// whole lines.
+template <int BLOCK>
+__device__ __forceinline__ void emit_columns(const uint32_t* __restrict__ bm, int nw, const uint32_t* __restrict__ gbase,
+                                             const uint8_t* __restrict__ wrank, uint32_t cnt, int32_t col0,
+                                             int32_t* __restrict__ tile, int32_t* __restrict__ out) {
+  uint32_t b0 = 0;
+  for (int w0 = 0; b0 < cnt;) {
+    const int w1 = word_at_rank(gbase, wrank, w0, nw, cnt, b0 + (uint32_t)kDenseTile);
+    const uint32_t b1 = w1 < nw ? gbase[w1 >> 3] + wrank[w1] : cnt;
+    for (int w = w0 + threadIdx.x; w < w1; w += BLOCK) {
+      uint32_t word = bm[w];
+      uint32_t pos = gbase[w >> 3] + wrank[w] - b0;
+      while (word) {
+        tile[pos++] = col0 + w * 32 + (__ffs(word) - 1);
+        word &= word - 1;
+      }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < b1 - b0; i += BLOCK) out[b0 + i] = tile[i];
+    __syncthreads();
+    w0 = w1;
+    b0 = b1;
+  }
+}
+
+// Shared memory of the dense numeric kernels: the bitmap and ranks of the
+// matrix's widest slice (words: a multiple of 8; 5.5 bytes a word), and a
+// buffer that is the stage of a walk or a tile of columns on their way out.
+// The widest, 512 Ki columns, leaves room for two blocks per SM.
+template <typename VIn>
+struct DenseSmem {
+  uint32_t* bm;
+  uint32_t* gbase;  // words / 8 group bases
+  uint8_t* wrank;   // ranks within the group, at most 7 * 32
+  Stage<VIn>* sg;
+  int32_t* tile;    // over the stage
+  __host__ __device__ static size_t ranks(int words) {
+    return (size_t(words) * 5 + size_t(words) / 2 + 15) & ~size_t(15);
+  }
+  __host__ __device__ static size_t bytes(int words) {
+    return ranks(words) +
+           (sizeof(Stage<VIn>) > size_t(kDenseTile) * 4 ? sizeof(Stage<VIn>) : size_t(kDenseTile) * 4);
+  }
+  __device__ DenseSmem(uint8_t* smem, int words) {
+    bm = reinterpret_cast<uint32_t*>(smem);
+    gbase = bm + words;
+    wrank = reinterpret_cast<uint8_t*>(gbase + words / 8);
+    sg = reinterpret_cast<Stage<VIn>*>(smem + ranks(words));
+    tile = reinterpret_cast<int32_t*>(sg);
+  }
+};
+
 // Heavy rows in one pass per slice of kRankCols columns of the row's column
 // range: a keys-only expansion marks the row's columns in a shared-memory
 // bitmap (or the symbolic kernel's kept bitmap is loaded), the rank of every
-// column comes from a 32-bit base per group of 8 words plus a 16-bit rank of
-// each word within its group, the column indices are written to C from the
-// bitmap and the values zeroed, and a second expansion adds every product
-// straight into its place in C with a global atomic add (resolved in L2: a
-// row's values are at most 8 bytes x nnz(row) there).  A range wider than one
-// slice is cut into slices, B rows cut to each by binary search (B rows
-// sorted).
+// column comes from a 32-bit base per group of 8 words plus an 8-bit rank of
+// each word within its group, the column indices go to C from the bitmap, the
+// values are zeroed, and a second expansion adds every product straight into
+// its place in C with a global atomic add (resolved in L2: a row's values are
+// at most 8 bytes x nnz(row) there).  A range wider than one slice is cut into
+// slices, B rows cut to each by binary search (B rows sorted).
+// Bound: the atomic adds, 125e9 to 180e9 a second with their share of L2
+// misses, so two blocks per SM: with four, the rows open at once overflow L2
+// (dense rows of Graph500 scale 17, 1.13e9 products: 7.6 ms against 7.0).
+// Sums in shared memory, a run of columns at a time, are no faster where one
+// run holds the row (compare-and-swap loops) and slower where it takes several
+// walks (8.4 ms).  Columns and zeros leave in whole lines: each thread writing
+// the bits of its words where they belong made 3.5 times the store
+// instructions (8.8 ms).
 template <int BLOCK, typename VIn>
-__global__ void __launch_bounds__(BLOCK)
-k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted,
+__global__ void __launch_bounds__(BLOCK, 2)
+k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, int words,
              const int64_t* __restrict__ crp, int32_t* __restrict__ ccol, typename Acc<VIn>::T* __restrict__ cval,
              const uint32_t* __restrict__ saved, const int32_t* __restrict__ saved_slot, int saved_slices,
              DevStatus* st) {
   using AT = typename Acc<VIn>::T;
-  constexpr int NWORD = kRankCols / 32;
   extern __shared__ __align__(16) uint8_t smem[];
-  uint32_t* bm = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* gbase = bm + NWORD;                                       // NWORD / 8 group bases
-  uint16_t* wrank = reinterpret_cast<uint16_t*>(gbase + NWORD / 8);   // NWORD ranks within the group
-  Stage<VIn>& sg = *reinterpret_cast<Stage<VIn>*>(reinterpret_cast<uint8_t*>(wrank + NWORD));
+  const DenseSmem<VIn> sm(smem, words);
+  uint32_t* bm = sm.bm;
+  uint32_t* gbase = sm.gbase;
+  uint8_t* wrank = sm.wrank;
+  Stage<VIn>& sg = *sm.sg;
   const int64_t r = rows[blockIdx.x];
   const int64_t c0r = crp[r], nz = crp[r + 1] - c0r;
   int64_t lo, hi;
@@ -2625,57 +2727,31 @@ k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
       expand_row<BLOCK, false, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1,
                                     [&](int32_t key, VIn, VIn, int64_t) {
         const uint32_t idx = (uint32_t)key - (uint32_t)s0;
-        if (idx < kRankCols) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
+        if (idx < (uint32_t)(s1 - s0)) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
       });
       __syncthreads();
     }
-    const int ng = (nw + 7) >> 3;
-    long long run = 0;
-    for (int g0 = 0; g0 < ng; g0 += BLOCK) {
-      const int g = g0 + threadIdx.x;
-      int cnt = 0;
-      if (g < ng) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int w = g * 8 + k;
-          wrank[w] = (uint16_t)cnt;
-          cnt += w < nw ? __popc(bm[w]) : 0;
-        }
-      }
-      long long tot;
-      const long long ex = block_exclusive_sum<BLOCK, long long>((long long)cnt, sg.tmp, tot);
-      if (g < ng) gbase[g] = (uint32_t)(run + ex);
-      run += tot;
+    const uint32_t cnt = (uint32_t)slice_ranks<BLOCK>(bm, nw, gbase, wrank, sg.tmp);
+    if (written + cnt > nz) {  // uniform: the counts disagree
+      if (threadIdx.x == 0) dev_report(st, kDevRowOverflow, 13, r);
+      return;
     }
-    __syncthreads();
     const int64_t base = c0r + written;
-    const int64_t room = nz - written;  // guards the writes if the counts disagree
-    for (int w = threadIdx.x; w < nw; w += BLOCK) {
-      uint32_t word = bm[w];
-      int64_t pos = (int64_t)gbase[w >> 3] + wrank[w];
-      while (word) {
-        const int b = __ffs(word) - 1;
-        word &= word - 1;
-        if (pos < room) {
-          ccol[base + pos] = (int32_t)(s0 + w * 32 + b);
-          cval[base + pos] = AT(0);
-        }
-        ++pos;
-      }
-    }
+    for (uint32_t i = threadIdx.x; i < cnt; i += BLOCK) cval[base + i] = AT(0);
+    emit_columns<BLOCK>(bm, nw, gbase, wrank, cnt, (int32_t)s0, sm.tile, ccol + base);
     __syncthreads();  // the zeroed values are visible to the block's atomic adds
     expand_row<BLOCK, true, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1,
                                  [&](int32_t key, VIn av, VIn bv, int64_t) {
       const uint32_t idx = (uint32_t)key - (uint32_t)s0;
-      if (idx >= kRankCols) return;
+      if (idx >= (uint32_t)(s1 - s0)) return;
       const uint32_t w = idx >> 5;
       const uint32_t pos = gbase[w >> 3] + wrank[w] + __popc(bm[w] & ((1u << (idx & 31)) - 1u));
-      if ((int64_t)pos < room) Acc<VIn>::atomic_add(&cval[base + pos], Acc<VIn>::mul(av, bv));
+      Acc<VIn>::atomic_add(&cval[base + pos], Acc<VIn>::mul(av, bv));
     });
-    written += run;
+    written += cnt;
     __syncthreads();
   }
-  if (threadIdx.x == 0 && written != nz) dev_report(st, written > nz ? kDevRowOverflow : kDevRowUnderflow, 13, r);
+  if (threadIdx.x == 0 && written != nz) dev_report(st, kDevRowUnderflow, 13, r);
 }
 
 // ---- the heaviest rows over several blocks ----------------------------------
@@ -2716,34 +2792,6 @@ struct HeavyPlan {
   unsigned long long* ticket;
 };
 
-// Word ranks of a slice bitmap in shared memory: for each word the set bits
-// of the words before it in its group of 8 (wrank) and the set bits before
-// the group (gbase); returns the slice's set bits.
-template <int BLOCK>
-__device__ __forceinline__ long long slice_ranks(const uint32_t* __restrict__ bm, int nw, uint32_t* __restrict__ gbase,
-                                                 uint16_t* __restrict__ wrank, long long* tmp) {
-  const int ng = (nw + 7) >> 3;
-  long long run = 0;
-  for (int g0 = 0; g0 < ng; g0 += BLOCK) {
-    const int g = g0 + threadIdx.x;
-    int cnt = 0;
-    if (g < ng) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int w = g * 8 + k;
-        wrank[w] = (uint16_t)cnt;
-        cnt += w < nw ? __popc(bm[w]) : 0;
-      }
-    }
-    long long tot;
-    const long long ex = block_exclusive_sum<BLOCK, long long>((long long)cnt, tmp, tot);
-    if (g < ng) gbase[g] = (uint32_t)(run + ex);
-    run += tot;
-  }
-  __syncthreads();
-  return run;
-}
-
 // Exclusive scan of n counts into out[0..n], out[n] the total, by one block
 // (the split rows are at most a few thousand).
 __global__ void k_scan_one_block(const int64_t* __restrict__ in, int64_t n, int64_t* __restrict__ out) {
@@ -2761,18 +2809,19 @@ __global__ void k_scan_one_block(const int64_t* __restrict__ in, int64_t n, int6
 }
 
 template <int BLOCK, typename VIn>
-__global__ void __launch_bounds__(BLOCK)
-k_dense_setup(HeavyPlan hp, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, const int64_t* __restrict__ crp,
+__global__ void __launch_bounds__(BLOCK, 2)
+k_dense_setup(HeavyPlan hp, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, int words, const int64_t* __restrict__ crp,
               int32_t* __restrict__ ccol, typename Acc<VIn>::T* __restrict__ cval, const uint32_t* __restrict__ saved,
               const int32_t* __restrict__ saved_slot, int saved_slices, const uint32_t* __restrict__ sym_bits,
               const int32_t* __restrict__ sym_slot, DevStatus* st) {
   using AT = typename Acc<VIn>::T;
-  constexpr int NWORD = kRankCols / 32;
+  constexpr int NWORD = kRankCols / 32;  // of a slice kept in memory
   extern __shared__ __align__(16) uint8_t smem[];
-  uint32_t* bm = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* gbase = bm + NWORD;
-  uint16_t* wrank = reinterpret_cast<uint16_t*>(gbase + NWORD / 8);
-  Stage<VIn>& sg = *reinterpret_cast<Stage<VIn>*>(reinterpret_cast<uint8_t*>(wrank + NWORD));
+  const DenseSmem<VIn> sm(smem, words);
+  uint32_t* bm = sm.bm;
+  uint32_t* gbase = sm.gbase;
+  uint8_t* wrank = sm.wrank;
+  Stage<VIn>& sg = *sm.sg;
   const int64_t i = blockIdx.x;
   const int64_t r = hp.rows[i];
   const int64_t c0r = crp[r], nz = crp[r + 1] - c0r;
@@ -2822,45 +2871,41 @@ k_dense_setup(HeavyPlan hp, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, cons
       __syncthreads();
       expand_row<BLOCK, false, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1, [&](int32_t key, VIn, VIn, int64_t) {
         const uint32_t idx = (uint32_t)key - (uint32_t)s0;
-        if (idx < kRankCols) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
+        if (idx < (uint32_t)(s1 - s0)) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
       });
       __syncthreads();
     }
     uint32_t* dst = hp.bits + ((size_t)i * hp.max_slices + sl) * NWORD;
     for (int w = threadIdx.x; w < nw; w += BLOCK) dst[w] = bm[w];
     if (threadIdx.x == 0) hp.slice_base[(size_t)i * hp.max_slices + sl] = written;
-    const long long cnt = slice_ranks<BLOCK>(bm, nw, gbase, wrank, sg.tmp);
-    const int64_t base = c0r + written;
-    const int64_t room = nz - written;
-    for (int w = threadIdx.x; w < nw; w += BLOCK) {
-      uint32_t word = bm[w];
-      int64_t pos = (int64_t)gbase[w >> 3] + wrank[w];
-      while (word) {
-        const int b = __ffs(word) - 1;
-        word &= word - 1;
-        if (pos < room) {
-          ccol[base + pos] = (int32_t)(s0 + w * 32 + b);
-          cval[base + pos] = AT(0);
-        }
-        ++pos;
+    const uint32_t cnt = (uint32_t)slice_ranks<BLOCK>(bm, nw, gbase, wrank, sg.tmp);
+    if (written + cnt > nz) {  // uniform: the counts disagree; no part of the row runs
+      if (threadIdx.x == 0) {
+        hp.nparts[i] = 0;
+        dev_report(st, kDevRowOverflow, 14, r);
       }
+      return;
     }
+    const int64_t base = c0r + written;
+    for (uint32_t k = threadIdx.x; k < cnt; k += BLOCK) cval[base + k] = AT(0);
+    emit_columns<BLOCK>(bm, nw, gbase, wrank, cnt, (int32_t)s0, sm.tile, ccol + base);
     written += cnt;
     __syncthreads();
   }
-  if (threadIdx.x == 0 && written != nz) dev_report(st, written > nz ? kDevRowOverflow : kDevRowUnderflow, 14, r);
+  if (threadIdx.x == 0 && written != nz) dev_report(st, kDevRowUnderflow, 14, r);
 }
 
 template <int BLOCK, typename VIn>
-__global__ void __launch_bounds__(BLOCK)
-k_dense_acc(HeavyPlan hp, Csr A, Csr B, const int64_t* __restrict__ crp, typename Acc<VIn>::T* __restrict__ cval,
+__global__ void __launch_bounds__(BLOCK, 2)
+k_dense_acc(HeavyPlan hp, Csr A, Csr B, int words, const int64_t* __restrict__ crp, typename Acc<VIn>::T* __restrict__ cval,
             DevStatus* st) {
   constexpr int NWORD = kRankCols / 32;
   extern __shared__ __align__(16) uint8_t smem[];
-  uint32_t* bm = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* gbase = bm + NWORD;
-  uint16_t* wrank = reinterpret_cast<uint16_t*>(gbase + NWORD / 8);
-  Stage<VIn>& sg = *reinterpret_cast<Stage<VIn>*>(reinterpret_cast<uint8_t*>(wrank + NWORD));
+  const DenseSmem<VIn> sm(smem, words);
+  uint32_t* bm = sm.bm;
+  uint32_t* gbase = sm.gbase;
+  uint8_t* wrank = sm.wrank;
+  Stage<VIn>& sg = *sm.sg;
   __shared__ long long s_t, s_i;
   const int64_t total = hp.parts[hp.n];
   for (;;) {

@@ -39,3 +39,23 @@ def test_walk(ctx, lengths, entries, algo, ncol, dtype):
     np.testing.assert_array_equal(out.csr.row_ptrs, rp)
     np.testing.assert_array_equal(out.csr.cols.astype(np.int64), cols)
     np.testing.assert_array_equal(out.csr.vals.astype(np.float64), vals)
+
+
+@pytest.mark.parametrize("ncol", [16385, 131072, 524288, 524289, 1100000])
+@pytest.mark.parametrize("nnz", [4097, 8192, 20000])
+def test_dense_row_columns_leave_in_tiles(ctx, ncol, nnz):
+    """Dense rows whose columns fill one tile of 4096 on their way out, end on one, or take several, over one, two
+    and three column slices; one row crowds its columns into full bitmap words."""
+    rng = np.random.default_rng(nnz)
+    per, n_b = 500, max(20, 3 * nnz // 500)
+    picks = [np.sort(rng.choice(ncol, min(nnz, ncol), replace=False)), np.arange(min(nnz, ncol)) + (ncol - min(nnz, ncol))]
+    cols = [np.sort(rng.choice(picks[k % 2], min(per, len(picks[k % 2])), replace=False)) for k in range(2 * n_b)]
+    B = from_coo(2 * n_b, ncol, np.repeat(np.arange(2 * n_b), [len(c) for c in cols]), np.concatenate(cols),
+                 rng.integers(1, 8, sum(map(len, cols))))
+    A = from_coo(2, 2 * n_b, np.repeat([0, 1], n_b), np.concatenate([np.arange(0, 2 * n_b, 2), np.arange(1, 2 * n_b, 2)]),
+                 rng.integers(1, 8, 2 * n_b))
+    out = ctx.spgemm(A, B, "hash")
+    rp, cols, vals, _ = oracle.oracle_spgemm(A, B, "hash")
+    np.testing.assert_array_equal(out.csr.row_ptrs, rp)
+    np.testing.assert_array_equal(out.csr.cols.astype(np.int64), cols)
+    np.testing.assert_array_equal(out.csr.vals.astype(np.float64), vals)
