@@ -428,11 +428,18 @@ cas_status alloc_err(cas_ctx* ctx, cudaError_t e, size_t bytes) {
                  "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
 }
 
-// scratch of a call, on the context's stream or stream s
-cas_status dev_alloc(cas_ctx* ctx, void** p, size_t bytes, cudaStream_t s) {
-  return alloc_err(ctx, pool_alloc(ctx, ctx->scratch, p, bytes, s), bytes);
+// Scratch of a call: allocated and freed on the context's stream, which keeps
+// the pool's holes the same from call to call.  A kernel on another stream
+// waits for `scratch_ready` first.
+cas_status dev_alloc(cas_ctx* ctx, void** p, size_t bytes) {
+  return alloc_err(ctx, pool_alloc(ctx, ctx->scratch, p, bytes, ctx->stream), bytes);
 }
-cas_status dev_alloc(cas_ctx* ctx, void** p, size_t bytes) { return dev_alloc(ctx, p, bytes, ctx->stream); }
+cas_status scratch_ready(cas_ctx* ctx, cudaStream_t s) {
+  if (s == ctx->stream) return CAS_OK;
+  CAS_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
+  CAS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_fork, 0));
+  return CAS_OK;
+}
 
 // an array of a result, which outlives the call
 cas_status out_alloc(cas_ctx* ctx, void** p, size_t bytes) {
@@ -799,6 +806,13 @@ cas_status join(cas_ctx* ctx) {
   return CAS_OK;
 }
 
+// After an error: kernels of the call that may still run on the auxiliary
+// streams end before its memory is freed.
+void quiesce(cas_ctx* ctx) {
+  for (int i = 0; i < kAux; ++i) cudaStreamSynchronize(ctx->aux[i]);
+  cudaGetLastError();
+}
+
 // The per-row arrays of a call, one allocation (row_flp is its start).
 cas_status scratch_alloc(cas_ctx* ctx, Call& c) {
   const size_t rows8 = (sizeof(int64_t) * (size_t)(c.m + 1) + 255) & ~size_t(255);
@@ -980,7 +994,7 @@ cas_status symb_split_heavy(cas_ctx* ctx, Call& c, int32_t*& rows, int64_t& n, i
   const int64_t max_slices = (c.ncol + kRankCols - 1) / kRankCols;
   const int64_t cap = (int64_t)((double)kSplitScratch * ctx->mem_share) / (max_slices * (kRankCols / 8));
   auto alloc = [&](void** p, size_t bytes) -> cas_status {
-    CAS_TRY(dev_alloc(ctx, p, bytes, s));
+    CAS_TRY(dev_alloc(ctx, p, bytes));
     c.heavy_tmp.push_back(*p);
     return CAS_OK;
   };
@@ -990,6 +1004,7 @@ cas_status symb_split_heavy(cas_ctx* ctx, Call& c, int32_t*& rows, int64_t& n, i
   CAS_TRY(alloc((void**)&heavy, sizeof(int32_t) * (size_t)n));
   CAS_TRY(alloc((void**)&light, sizeof(int32_t) * (size_t)n));
   CAS_TRY(alloc((void**)&counts, 2 * sizeof(unsigned long long)));
+  CAS_TRY(scratch_ready(ctx, s));
   CAS_CUDA(ctx, cudaMemsetAsync(c.hslot, 0xFF, sizeof(int32_t) * (size_t)(c.m + 1), s));
   CAS_CUDA(ctx, cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), s));
   k_split_dense_rows<<<grid_for(n, 256, ctx->sm_count * 4), 256, 0, s>>>(rows, n, c.row_flp, cap, heavy, light, counts,
@@ -1016,6 +1031,7 @@ cas_status symb_split_heavy(cas_ctx* ctx, Call& c, int32_t*& rows, int64_t& n, i
   CAS_TRY(alloc((void**)&hp.parts, sizeof(int64_t) * (size_t)(nh + 1)));
   CAS_TRY(alloc((void**)&hp.apre, sizeof(int64_t) * (size_t)(c.A.nnz > 0 ? c.A.nnz : 1)));
   CAS_TRY(alloc((void**)&hp.ticket, sizeof(unsigned long long)));
+  CAS_TRY(scratch_ready(ctx, s));
   c.hbits = hp.bits;
   CAS_CUDA(ctx, cudaMemsetAsync(hp.ticket, 0, sizeof(unsigned long long), s));
   k_heavy_plan<512><<<(unsigned)nh, 512, 0, s>>>(hp, c.A.csr, c.B.csr, c.ncol, c.b_sorted ? 1 : 0, ctx->d_status);
@@ -1064,11 +1080,7 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
           return set_err(ctx, CAS_ERR_BAD_INPUT, "heavy rows over more than %d columns need B rows sorted by column", kDenseChunkBits);
         int32_t* drows = const_cast<int32_t*>(rows);
         int64_t nd = n;
-        if (ctx->heavy_split) {
-          CAS_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
-          CAS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_fork, 0));
-          CAS_TRY(symb_split_heavy(ctx, c, drows, nd, row_nz, s));
-        }
+        if (ctx->heavy_split) CAS_TRY(symb_split_heavy(ctx, c, drows, nd, row_nz, s));
         if (nd == 0) break;
         // bitmaps kept for the numeric kernel: every slice of each row when that fits a quarter
         // of the free device memory, at most 24 GiB (and at least kSavedBitmapBytes), else
@@ -1081,8 +1093,7 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
           CAS_TRY(dev_alloc(ctx, (void**)&c.dbits, (size_t)nd * c.saved_slices * (kRankCols / 8)));
           CAS_TRY(dev_alloc(ctx, (void**)&c.dslot, sizeof(int32_t) * (c.m + 1)));
           CAS_CUDA(ctx, cudaMemsetAsync(c.dslot, 0xFF, sizeof(int32_t) * (c.m + 1), ctx->stream));
-          CAS_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
-          CAS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_fork, 0));
+          CAS_TRY(scratch_ready(ctx, s));
         }
         k_symb_dense<512><<<(unsigned)nd, 512, smem_symb_dense<512>(), s>>>(drows, c.A.csr, c.B.csr, c.ncol,
                                                                              c.b_sorted ? 1 : 0, row_nz, c.dbits,
@@ -1183,10 +1194,9 @@ void launch_esc_bin(int esc_form, bool rank, int64_t n, cudaStream_t s, const in
 }
 
 // The heaviest dense rows over several blocks (k_dense_setup, then
-// k_dense_acc; see cas_kernels.cu), on stream s, with scratch allocated and
-// freed on s: the slice bitmaps (64 KiB per row and slice), the per-row
-// plan and the product prefix of every A entry.
-
+// k_dense_acc; see cas_kernels.cu), on stream s.  Scratch: the
+// slice bitmaps (64 KiB per row and slice), the per-row plan and the product
+// prefix of every A entry.
 template <typename VIn>
 cas_status launch_heavy_split(cas_ctx* ctx, Call& c, const int32_t* rows, int64_t n, const int64_t* crp, int32_t* ccol,
                               typename cas::Acc<VIn>::T* cval, cudaStream_t s) {
@@ -1195,41 +1205,37 @@ cas_status launch_heavy_split(cas_ctx* ctx, Call& c, const int32_t* rows, int64_
   hp.rows = rows;
   hp.n = n;
   hp.max_slices = (int)((c.ncol + kRankCols - 1) / kRankCols);
-  std::vector<void*> tmp;
   auto alloc = [&](void** p, size_t bytes) -> cas_status {
-    CAS_TRY(dev_alloc(ctx, p, bytes, s));
-    tmp.push_back(*p);
+    CAS_TRY(dev_alloc(ctx, p, bytes));
+    c.heavy_tmp.push_back(*p);
     return CAS_OK;
   };
-  cas_status rc = [&]() -> cas_status {
-    CAS_TRY(alloc((void**)&hp.bits, (size_t)n * hp.max_slices * (kRankCols / 8)));
-    CAS_TRY(alloc((void**)&hp.slice_base, sizeof(int64_t) * (size_t)n * hp.max_slices));
-    CAS_TRY(alloc((void**)&hp.lo, sizeof(int64_t) * (size_t)n));
-    CAS_TRY(alloc((void**)&hp.hi, sizeof(int64_t) * (size_t)n));
-    CAS_TRY(alloc((void**)&hp.nslices, sizeof(int32_t) * (size_t)n));
-    CAS_TRY(alloc((void**)&hp.products, sizeof(int64_t) * (size_t)n));
-    CAS_TRY(alloc((void**)&hp.nparts, sizeof(int64_t) * (size_t)n));
-    CAS_TRY(alloc((void**)&hp.parts, sizeof(int64_t) * (size_t)(n + 1)));
-    CAS_TRY(alloc((void**)&hp.apre, sizeof(int64_t) * (size_t)(c.A.nnz > 0 ? c.A.nnz : 1)));
-    CAS_TRY(alloc((void**)&hp.ticket, sizeof(unsigned long long)));
-    CAS_CUDA(ctx, cudaMemsetAsync(hp.ticket, 0, sizeof(unsigned long long), s));
-    const int words = dense_words(c.ncol);
-    const size_t smem = DenseSmem<VIn>::bytes(words);
-    k_dense_setup<512, VIn><<<(unsigned)n, 512, smem, s>>>(
-        hp, c.A.csr, c.B.csr, c.ncol, c.b_sorted ? 1 : 0, words, crp, ccol, cval, c.dbits, c.dslot, c.saved_slices, c.hbits,
-        c.hslot, ctx->d_status);
-    CAS_TRY(check_launch(ctx, "k_dense_setup"));
-    k_scan_one_block<<<1, 1024, 0, s>>>(hp.nparts, n, hp.parts);
-    CAS_TRY(check_launch(ctx, "k_scan_one_block"));
-    int per_sm = 0;
-    CAS_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_acc<512, VIn>, 512, smem));
-    const int grid = std::max(1, per_sm) * ctx->sm_count;
-    k_dense_acc<512, VIn><<<grid, 512, smem, s>>>(hp, c.A.csr, c.B.csr, words, crp, cval, ctx->d_status);
-    CAS_TRY(check_launch(ctx, "k_dense_acc"));
-    return CAS_OK;
-  }();
-  for (void* p : tmp) cudaFreeAsync(p, s);
-  return rc;
+  CAS_TRY(alloc((void**)&hp.bits, (size_t)n * hp.max_slices * (kRankCols / 8)));
+  CAS_TRY(alloc((void**)&hp.slice_base, sizeof(int64_t) * (size_t)n * hp.max_slices));
+  CAS_TRY(alloc((void**)&hp.lo, sizeof(int64_t) * (size_t)n));
+  CAS_TRY(alloc((void**)&hp.hi, sizeof(int64_t) * (size_t)n));
+  CAS_TRY(alloc((void**)&hp.nslices, sizeof(int32_t) * (size_t)n));
+  CAS_TRY(alloc((void**)&hp.products, sizeof(int64_t) * (size_t)n));
+  CAS_TRY(alloc((void**)&hp.nparts, sizeof(int64_t) * (size_t)n));
+  CAS_TRY(alloc((void**)&hp.parts, sizeof(int64_t) * (size_t)(n + 1)));
+  CAS_TRY(alloc((void**)&hp.apre, sizeof(int64_t) * (size_t)(c.A.nnz > 0 ? c.A.nnz : 1)));
+  CAS_TRY(alloc((void**)&hp.ticket, sizeof(unsigned long long)));
+  CAS_TRY(scratch_ready(ctx, s));
+  CAS_CUDA(ctx, cudaMemsetAsync(hp.ticket, 0, sizeof(unsigned long long), s));
+  const int words = dense_words(c.ncol);
+  const size_t smem = DenseSmem<VIn>::bytes(words);
+  k_dense_setup<512, VIn><<<(unsigned)n, 512, smem, s>>>(
+      hp, c.A.csr, c.B.csr, c.ncol, c.b_sorted ? 1 : 0, words, crp, ccol, cval, c.dbits, c.dslot, c.saved_slices, c.hbits,
+      c.hslot, ctx->d_status);
+  CAS_TRY(check_launch(ctx, "k_dense_setup"));
+  k_scan_one_block<<<1, 1024, 0, s>>>(hp.nparts, n, hp.parts);
+  CAS_TRY(check_launch(ctx, "k_scan_one_block"));
+  int per_sm = 0;
+  CAS_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_acc<512, VIn>, 512, smem));
+  const int grid = std::max(1, per_sm) * ctx->sm_count;
+  k_dense_acc<512, VIn><<<grid, 512, smem, s>>>(hp, c.A.csr, c.B.csr, words, crp, cval, ctx->d_status);
+  CAS_TRY(check_launch(ctx, "k_dense_acc"));
+  return CAS_OK;
 }
 
 template <typename VIn>
@@ -1634,6 +1640,7 @@ cas_status run_blocked(cas_ctx* ctx, cas_accum accum, const cas_csr* A, Call& fu
       st = check_launch(ctx, "k_rebase_to");
     }
     if (st != CAS_OK) {
+      quiesce(ctx);
       scratch_free(ctx, ck);
       free_dev_c(o, ctx->stream);
       break;
@@ -1772,6 +1779,7 @@ cas_status run_spgemm(cas_ctx* ctx, cas_accum accum, const cas_csr* A, const cas
   });
   if (st != CAS_OK) {
     free_host();
+    quiesce(ctx);
     scratch_free(ctx, c);
     free_dev_c(o, ctx->stream);
     return finish(st);
