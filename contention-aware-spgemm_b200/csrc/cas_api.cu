@@ -39,14 +39,14 @@ constexpr int kAux = 4;          // auxiliary streams for concurrent bins
 constexpr int kMaxOutBlocks = 64;  // row blocks of a C returned in host memory, at most
 constexpr double kOutBlockMin = double(1ull << 30);    // host C under this: one block
 constexpr double kOutBlockBytes = double(2ull << 30);  // else a block per this many bytes of C
-constexpr int kCountSlots = 256; // device/pinned counter block
+constexpr int kCountSlots = 258; // device/pinned counter block
 constexpr int kMiscWords = 8;    // pinned words of other small results
 
 // Layout of the counter block (unsigned long long slots).
 constexpr int kSlotSymb = 0;     // [0, 9)   symbolic bin counts
 constexpr int kSlotNumc = 10;    // [10, 23) numeric bin counts
 constexpr int kSlotTotals = 24;  // [24]    products, [25] max row products
-constexpr int kSlotCursor = 28;  // [28, 41) bin cursors
+constexpr int kSlotCursor = 28;  // [28, 41) numeric bin cursors
 constexpr int kSlotNnz = 44;     // [44]    nnz(C) from the scan
 constexpr int kSlotCheck = 48;   // [48, 52) input check flags
 constexpr int kSlotBinSums = 64; // [64, 103) per numeric bin: products, nnz(C), nnz(A)
@@ -54,6 +54,8 @@ constexpr int kSlotOvf = 110;    // [110]   rows handed to the radix-sort ESC ke
 constexpr int kSlotFused = 112;  // [112, 116) fused rows: count, products, output bound, nnz(A); [116] ticket
 constexpr int kSlotHeavy = 128;  // [128, 176) dense rows per size class
 constexpr int kSlotHeavyCur = 176;  // [176, 224) their cursors
+constexpr int kSlotSymbCur = 228;   // [228, 237) symbolic bin cursors
+constexpr int kSlotStatus = 256;    // [256, 258) the device status, behind the counters
 constexpr size_t kStageBytes = size_t(64) << 20;  // pinned staging chunk for host copies
 constexpr double kSavedBitmapBytes = 8.0 * (1ull << 30);  // heavy-row bitmaps kept between the phases
 
@@ -95,11 +97,10 @@ struct cas_ctx {
   cas::DevStatus* d_status = nullptr;
   unsigned long long* d_counts = nullptr;
   unsigned long long* h_counts = nullptr;  // pinned mirror
-  cas::DevStatus* h_status = nullptr;      // pinned mirror
+  cas::DevStatus* h_status = nullptr;      // in the mirror, as d_status in d_counts
   unsigned long long* h_misc = nullptr;    // pinned words for other small results
   // the mirrors' device-side addresses (the device writes them by k_fetch_words)
   unsigned long long* h_counts_dev = nullptr;
-  unsigned long long* h_status_dev = nullptr;
   unsigned long long* h_misc_dev = nullptr;
   void* h_stage[3] = {};                   // pinned staging for large host copies
   cudaEvent_t ev_stage[3] = {};
@@ -167,20 +168,36 @@ const char* dev_err_name(int code) {
 // n words (8 bytes each) from device memory into a pinned mirror, written
 // by a one-block kernel on s through the mirror's device-side address
 // (mirror_dev); the caller synchronises s before reading the mirror.
-static_assert(sizeof(cas::DevStatus) % 8 == 0, "the status is fetched in 8-byte words");
+static_assert(sizeof(cas::DevStatus) == 8 * (kCountSlots - kSlotStatus), "the status is fetched with the counters");
 cas_status fetch_words(cas_ctx* ctx, unsigned long long* mirror_dev, const void* src, int n, cudaStream_t s) {
   cas::k_fetch_words<<<1, 256, 0, s>>>(mirror_dev, static_cast<const unsigned long long*>(src), n);
   return check_launch(ctx, "k_fetch_words");
 }
 
-cas_status check_status(cas_ctx* ctx) {
-  CAS_TRY(fetch_words(ctx, ctx->h_status_dev, ctx->d_status, (int)(sizeof(cas::DevStatus) / 8), ctx->stream));
+// Counters and status to the host, in one launch, and a wait for them.
+cas_status fetch_counts(cas_ctx* ctx) {
+  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev, ctx->d_counts, kCountSlots, ctx->stream));
   CAS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return CAS_OK;
+}
+
+// Counters and status cleared, before a call's first kernel.
+cas_status clear_counts(cas_ctx* ctx) {
+  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts, 0, sizeof(unsigned long long) * kCountSlots, ctx->stream));
+  return CAS_OK;
+}
+
+cas_status status_of(cas_ctx* ctx) {
   if (ctx->h_status->err != 0) {
     return set_err(ctx, CAS_ERR_DEVICE, "device check failed in kernel %d at row %lld: %s", ctx->h_status->kernel,
                    (long long)ctx->h_status->row, dev_err_name(ctx->h_status->err));
   }
   return CAS_OK;
+}
+
+cas_status check_status(cas_ctx* ctx) {
+  CAS_TRY(fetch_counts(ctx));
+  return status_of(ctx);
 }
 
 template <typename K>
@@ -732,31 +749,6 @@ cas_status to_device(cas_ctx* ctx, const cas_csr* M, DevMat& out, double& h2d) {
 
 }  // namespace
 
-// ============================================================ input check
-namespace cas {
-// One warp per row: row pointers non-decreasing and within [0, nnz], column
-// indices in [0, ncol); flags[1] is set when some row is not sorted.
-__global__ void k_check_csr(Csr M, int64_t nnz, unsigned long long* flags) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < M.nrow; r += nw) {
-    const int64_t s = M.rp[r], e = M.rp[r + 1];
-    if (s < 0 || e < s || e > nnz) {
-      if (lane == 0) atomicOr(&flags[0], 1ull);
-      continue;
-    }
-    bool bad = false, unsorted = false;
-    for (int64_t j = s + lane; j < e; j += 32) {
-      const int32_t c = M.col[j];
-      bad |= (uint64_t)c >= (uint64_t)M.ncol;
-      if (j + 1 < e) unsorted |= M.col[j + 1] < c;
-    }
-    if (__any_sync(kFull, bad) && lane == 0) atomicOr(&flags[0], 1ull);
-    if (__any_sync(kFull, unsorted) && lane == 0) atomicOr(&flags[1], 1ull);
-  }
-}
-}  // namespace cas
-
 namespace {
 
 struct Call {
@@ -780,7 +772,6 @@ struct Call {
   int32_t* frows = nullptr;
   int64_t* fpos = nullptr;
   unsigned long long* fstatus = nullptr;
-  bool ovf_preset = false;
   bool may_defer = false;  // some kernel launched may hand rows to the radix-sort ESC kernel
   // bitmaps of heavy rows kept by the symbolic kernel for the numeric one
   uint32_t* dbits = nullptr;
@@ -854,6 +845,10 @@ cas_status launch_scan(cas_ctx* ctx, int64_t* out, const int64_t* in, int64_t n,
   if (n <= 0) return CAS_OK;
   const int64_t n_in = n - 1;
   const int64_t nparts = (n + kScanTile - 1) / kScanTile;
+  if (nparts == 1) {
+    k_scan_tile<<<1, kScanBlock, 0, ctx->stream>>>(in, n_in, out, n, total_out);
+    return check_launch(ctx, "k_scan_tile");
+  }
   k_scan_partials<<<(unsigned)nparts, kScanBlock, 0, ctx->stream>>>(in, n_in, partial);
   CAS_TRY(check_launch(ctx, "k_scan_partials"));
   k_scan_top<<<1, kScanBlock, 0, ctx->stream>>>(partial, nparts, total_out);
@@ -864,62 +859,86 @@ cas_status launch_scan(cas_ctx* ctx, int64_t* out, const int64_t* in, int64_t n,
 }
 
 // ------------------------------------------------------------------ INIT
-// Row pointers and column indices of A and B in range (an error if not), and
-// whether B's rows are sorted by column (c.b_sorted).  Synchronises.
-cas_status check_inputs(cas_ctx* ctx, Call& c) {
-  using namespace cas;
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts + kSlotCheck, 0, sizeof(unsigned long long) * 4, ctx->stream));
-  const int g = grid_for(std::max<int64_t>(c.A.csr.nrow, c.B.csr.nrow) * 32, 256, ctx->sm_count * 16);
-  Csr a = c.A.csr;
-  a.ncol = c.B.csr.nrow;  // A's columns index B's rows
-  k_check_csr<<<g, 256, 0, ctx->stream>>>(a, c.A.nnz, ctx->d_counts + kSlotCheck);
-  CAS_TRY(check_launch(ctx, "k_check_csr"));
-  k_check_csr<<<g, 256, 0, ctx->stream>>>(c.B.csr, c.B.nnz, ctx->d_counts + kSlotCheck + 2);
-  CAS_TRY(check_launch(ctx, "k_check_csr"));
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev + kSlotCheck, ctx->d_counts + kSlotCheck, 4, ctx->stream));
-  CAS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+// Lanes that walk a row, by the rows' mean length: enough for most rows in one
+// go.  Row products of 500,009 rows of 4: 88 us with a warp a row, 37 with 4
+// lanes; of 131,072 skewed rows of 16 (and hubs, which blocks take): 289 and 76.
+template <typename F>
+void with_lanes(int64_t nnz, int64_t rows, F&& f) {
+  const int64_t mean = nnz / std::max<int64_t>(1, rows);
+  if (mean <= 6) f(std::integral_constant<int, 4>());
+  else if (mean <= 24) f(std::integral_constant<int, 16>());
+  else f(std::integral_constant<int, 32>());
+}
+
+cas_status launch_check(cas_ctx* ctx, const Csr& M, int64_t nnz, unsigned long long* flags) {
+  if (M.nrow <= 0) return CAS_OK;
+  with_lanes(nnz, M.nrow, [&](auto g) {
+    constexpr int G = decltype(g)::value;
+    cas::k_check_csr<256, G><<<grid_for(M.nrow * G, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(M, nnz, flags);
+  });
+  return check_launch(ctx, "k_check_csr");
+}
+
+// The row products and the symbolic bins' counts; with `check`, A is checked too.
+cas_status launch_flp(cas_ctx* ctx, const Call& c, bool check, bool a_is_b, int64_t* row_flp, int fuse) {
+  if (c.m <= 0) return CAS_OK;
+  unsigned long long* k = ctx->d_counts;
+  with_lanes(c.A.nnz, c.m, [&](auto g) {
+    constexpr int G = decltype(g)::value;
+    const int grid = grid_for(c.m * G, 256, ctx->sm_count * 16);
+    auto kern = check ? cas::k_flp<256, G, true> : cas::k_flp<256, G, false>;
+    kern<<<grid, 256, 0, ctx->stream>>>(c.A.csr, c.B.csr, c.A.nnz, a_is_b ? 1 : 0, c.ncol, row_flp, k + kSlotTotals,
+                                        k + kSlotSymb, k + kSlotCheck, ctx->d_status, fuse, k + kSlotFused);
+  });
+  return check_launch(ctx, "k_flp");
+}
+
+cas_status check_flags(cas_ctx* ctx, Call& c) {
   if (ctx->h_counts[kSlotCheck] || ctx->h_counts[kSlotCheck + 2])
     return set_err(ctx, CAS_ERR_BAD_INPUT, "invalid CSR input: row pointers or column indices out of range");
   c.b_sorted = ctx->h_counts[kSlotCheck + 3] == 0;
   return CAS_OK;
 }
 
-// With `validate`, checks the inputs first (check_inputs); without, c.b_sorted
-// is the caller's (a row block of a checked product).
+// Row pointers and column indices of A and B in range (an error if not), and
+// whether B's rows are sorted by column (c.b_sorted).  Synchronises.
+cas_status check_inputs(cas_ctx* ctx, Call& c) {
+  CAS_TRY(clear_counts(ctx));
+  Csr a = c.A.csr;
+  a.ncol = c.B.csr.nrow;  // A's columns index B's rows
+  CAS_TRY(launch_check(ctx, a, c.A.nnz, ctx->d_counts + kSlotCheck));
+  CAS_TRY(launch_check(ctx, c.B.csr, c.B.nnz, ctx->d_counts + kSlotCheck + 2));
+  CAS_TRY(fetch_counts(ctx));
+  return check_flags(ctx, c);
+}
+
+// With `validate`, the inputs are checked as in check_inputs, on the way:
+// nothing reads past a row pointer or column before it was looked at, and the
+// products and bins of a faulty input are never used.  Without, c.b_sorted is
+// the caller's (a row block of a checked product).
 cas_status phase_init(cas_ctx* ctx, Call& c, bool validate) {
   using namespace cas;
-  if (validate) CAS_TRY(check_inputs(ctx, c));
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts, 0, sizeof(unsigned long long) * kCountSlots, ctx->stream));
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(DevStatus), ctx->stream));
+  CAS_TRY(clear_counts(ctx));
   CAS_TRY(scratch_alloc(ctx, c));
+  const Csr &a = c.A.csr, &b = c.B.csr;
+  const bool a_is_b = a.rp == b.rp && a.col == b.col && a.nrow == b.nrow && a.ncol == b.ncol && c.A.nnz == c.B.nnz;
+  if (validate && !a_is_b) CAS_TRY(launch_check(ctx, b, c.B.nnz, ctx->d_counts + kSlotCheck + 2));
+  CAS_TRY(launch_flp(ctx, c, validate, a_is_b, c.row_flp, c.fuse));
   if (c.m > 0) {
-    k_flp<256><<<grid_for(c.m * 32, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-        c.A.csr, c.B.csr, c.ncol, c.row_flp, ctx->d_counts + kSlotTotals, ctx->d_counts + kSlotSymb, ctx->d_status,
-        c.fuse, ctx->d_counts + kSlotFused);
-    CAS_TRY(check_launch(ctx, "k_flp"));
+    k_bin_scatter_symb<<<grid_for(c.m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
+        c.m, c.row_flp, c.ncol, ctx->d_counts + kSlotSymb, ctx->d_counts + kSlotSymbCur, c.rows, c.fuse);
+    CAS_TRY(check_launch(ctx, "k_bin_scatter_symb"));
   }
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev, ctx->d_counts, kCountSlots, ctx->stream));
-  CAS_TRY(check_status(ctx));  // synchronises
+  CAS_TRY(fetch_counts(ctx));
+  if (validate) CAS_TRY(check_flags(ctx, c));
+  CAS_TRY(status_of(ctx));
   c.flop = (int64_t)ctx->h_counts[kSlotTotals];
   c.max_flp = (int64_t)ctx->h_counts[kSlotTotals + 1];
   c.nf = (int64_t)ctx->h_counts[kSlotFused];
   c.f_flop = (int64_t)ctx->h_counts[kSlotFused + 1];
   c.f_bound = (int64_t)ctx->h_counts[kSlotFused + 2];
   c.f_nnza = (int64_t)ctx->h_counts[kSlotFused + 3];
-  unsigned long long* cur = ctx->h_counts + kSlotCursor;
-  unsigned long long off = 0;
-  for (int b = 0; b < kSymbBins; ++b) {
-    c.symb_count[b] = (int64_t)ctx->h_counts[kSlotSymb + b];
-    cur[b] = off;
-    off += ctx->h_counts[kSlotSymb + b];
-  }
-  if (c.m > 0) {
-    CAS_CUDA(ctx, cudaMemcpyAsync(ctx->d_counts + kSlotCursor, cur, sizeof(unsigned long long) * kSymbBins,
-                                  cudaMemcpyHostToDevice, ctx->stream));
-    k_bin_scatter_symb<<<grid_for(c.m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-        c.m, c.row_flp, c.ncol, ctx->d_counts + kSlotCursor, c.rows, c.fuse);
-    CAS_TRY(check_launch(ctx, "k_bin_scatter_symb"));
-  }
+  for (int b = 0; b < kSymbBins; ++b) c.symb_count[b] = (int64_t)ctx->h_counts[kSlotSymb + b];
   if (c.nf > 0) {
     // the fused rows in ascending order: marks (in row_nz, cleared before the
     // symbolic kernels), their scan, the scatter
@@ -946,10 +965,7 @@ cas_status launch_fused(cas_ctx* ctx, Call& c, const int64_t* known, int32_t* cc
   using AT = typename Acc<VIn>::T;
   if (c.nf == 0) return CAS_OK;
   unsigned int* ovf_count = reinterpret_cast<unsigned int*>(ctx->d_counts + kSlotOvf);
-  CAS_CUDA(ctx, cudaMemsetAsync(ovf_count, 0, sizeof(unsigned int), ctx->stream));
-  c.ovf_preset = true;
   CAS_CUDA(ctx, cudaMemsetAsync(c.fstatus, 0, sizeof(unsigned long long) * c.nf, ctx->stream));
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts + kSlotFused + 4, 0, sizeof(unsigned long long), ctx->stream));
   Fused fu{c.frows, ctx->d_counts + kSlotFused + 4, c.fstatus, known, c.row_nz, cap};
   if (ctx->profile) CAS_CUDA(ctx, cudaEventRecord(ctx->ev_fused[0], ctx->stream));
   // Fewer fused rows than SMs keep the index form: which rows it hands to the
@@ -1109,49 +1125,23 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
 }
 
 // ------------------------------------------------------------------ MGMT
-cas_status numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int mode) {
+// The numeric bins' counts and lists; numc_counts reads the counts once the
+// host has them.
+cas_status launch_numc_count(cas_ctx* ctx, Call& c, const int64_t* crp, int mode) {
   using namespace cas;
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts + kSlotNumc, 0, sizeof(unsigned long long) * kNumcBins, ctx->stream));
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts + kSlotBinSums, 0, sizeof(unsigned long long) * 3 * kNumcBins,
-                                ctx->stream));
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts + kSlotHeavy, 0, sizeof(unsigned long long) * kHeavyClasses,
-                                ctx->stream));
-  if (c.m > 0) {
-    k_bin_count_numc<<<grid_for(c.m, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(
-        c.m, c.row_flp, crp, c.A.csr.rp, mode, ctx->acc_thres, ctx->esc_max, ctx->hash_max,
-        ctx->d_counts + kSlotNumc, ctx->d_counts + kSlotBinSums, ctx->d_counts + kSlotHeavy);
-    CAS_TRY(check_launch(ctx, "k_bin_count_numc"));
-  }
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev + kSlotNumc, ctx->d_counts + kSlotNumc, kNumcBins, ctx->stream));
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev + kSlotBinSums, ctx->d_counts + kSlotBinSums, 3 * kNumcBins, ctx->stream));
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev + kSlotHeavy, ctx->d_counts + kSlotHeavy, kHeavyClasses, ctx->stream));
-  CAS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  unsigned long long* cur = ctx->h_counts + kSlotCursor;
-  unsigned long long off = 0;
-  for (int b = 0; b < kNumcBins; ++b) {
-    c.numc_count[b] = (int64_t)ctx->h_counts[kSlotNumc + b];
-    cur[b] = off;
-    if (b == kNB_Dense) {  // heaviest size class first
-      unsigned long long* hc = ctx->h_counts + kSlotHeavyCur;
-      unsigned long long o = off;
-      for (int k = 0; k < kHeavyClasses; ++k) {
-        hc[k] = o;
-        o += ctx->h_counts[kSlotHeavy + k];
-      }
-    }
-    off += ctx->h_counts[kSlotNumc + b];
-  }
-  if (c.m > 0) {
-    CAS_CUDA(ctx, cudaMemcpyAsync(ctx->d_counts + kSlotCursor, cur, sizeof(unsigned long long) * kNumcBins,
-                                  cudaMemcpyHostToDevice, ctx->stream));
-    CAS_CUDA(ctx, cudaMemcpyAsync(ctx->d_counts + kSlotHeavyCur, ctx->h_counts + kSlotHeavyCur,
-                                  sizeof(unsigned long long) * kHeavyClasses, cudaMemcpyHostToDevice, ctx->stream));
-    k_bin_scatter_numc<<<grid_for(c.m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-        c.m, c.row_flp, crp, mode, ctx->acc_thres, ctx->esc_max, ctx->hash_max, ctx->d_counts + kSlotCursor,
-        ctx->d_counts + kSlotHeavyCur, c.rows);
-    CAS_TRY(check_launch(ctx, "k_bin_scatter_numc"));
-  }
-  return CAS_OK;
+  if (c.m <= 0) return CAS_OK;
+  unsigned long long* k = ctx->d_counts;
+  k_bin_count_numc<256><<<grid_for(c.m, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(
+      c.m, c.row_flp, crp, c.A.csr.rp, mode, ctx->acc_thres, ctx->esc_max, ctx->hash_max, k + kSlotNumc,
+      k + kSlotBinSums, k + kSlotHeavy);
+  CAS_TRY(check_launch(ctx, "k_bin_count_numc"));
+  k_bin_scatter_numc<<<grid_for(c.m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
+      c.m, c.row_flp, crp, mode, ctx->acc_thres, ctx->esc_max, ctx->hash_max, k + kSlotNumc, k + kSlotHeavy,
+      k + kSlotCursor, k + kSlotHeavyCur, c.rows);
+  return check_launch(ctx, "k_bin_scatter_numc");
+}
+void numc_counts(cas_ctx* ctx, Call& c) {
+  for (int b = 0; b < cas::kNumcBins; ++b) c.numc_count[b] = (int64_t)ctx->h_counts[kSlotNumc + b];
 }
 
 // ------------------------------------------------------------------ NUMC
@@ -1262,7 +1252,6 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
                          kNB_E3K, kNB_E2K, kNB_E1K, kNB_Tiny};
   const int* order = ctx->bin_order == 1 ? grouped : interleaved;
   unsigned int* ovf_count = reinterpret_cast<unsigned int*>(ctx->d_counts + kSlotOvf);
-  if (!c.ovf_preset) CAS_CUDA(ctx, cudaMemsetAsync(ovf_count, 0, sizeof(unsigned int), ctx->stream));
   CAS_TRY(fork(ctx));
   const bool rank = rank_form(ctx, c.ncol);
   int64_t esc_rows = c.nf;  // fused rows may have handed rows to the radix-sort kernel too
@@ -1406,19 +1395,19 @@ cas_status compute_dev(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, De
   CAS_TRY(launch_symb_bins(ctx, c, c.row_nz));
   CAS_TRY(launch_scan(ctx, o.crp, c.row_nz, c.m + 1, c.partial,
                       reinterpret_cast<int64_t*>(ctx->d_counts + kSlotNnz)));
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev + kSlotNnz, ctx->d_counts + kSlotNnz, 1, ctx->stream));
+  CAS_CUDA(ctx, cudaEventRecord(ctx->ev_phase[2], ctx->stream));
+  // MGMT: the numeric bins, then one wait for them and for nnz(C)
+  CAS_TRY(launch_numc_count(ctx, c, o.crp, mode_of(accum)));
   CAS_TRY(check_status(ctx));
+  numc_counts(ctx, c);
   // counts of the rows that had a symbolic pass; the fused rows add theirs
   // in NUMC, within the bound min(products, columns) each
   o.nnz_known = (int64_t)ctx->h_counts[kSlotNnz];
   o.nnz = o.nnz_known;
   const int64_t cap = o.nnz_known + (c.nf > 0 ? c.f_bound : 0);
-  CAS_CUDA(ctx, cudaEventRecord(ctx->ev_phase[2], ctx->stream));
-  // MGMT
   CAS_TRY(out_alloc(ctx, (void**)&o.ccol, sizeof(int32_t) * cap));
   CAS_TRY(out_alloc(ctx, &o.cval, vbytes * cap));
   CAS_TRY(at_cap(cap));
-  CAS_TRY(numc_bins(ctx, c, o.crp, mode_of(accum)));
   CAS_CUDA(ctx, cudaEventRecord(ctx->ev_phase[3], ctx->stream));
   // NUMC: the fused rows first (they place themselves after the known
   // counts), then the scan of all counts, which the other kernels write by
@@ -1432,8 +1421,6 @@ cas_status compute_dev(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, De
   else CAS_TRY(launch_numc_bins<int32_t>(ctx, c, o.crp, o.ccol, o.cval));
   CAS_TRY(scratch_free(ctx, c));
   CAS_CUDA(ctx, cudaEventRecord(ctx->ev_phase[4], ctx->stream));
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev + kSlotOvf, ctx->d_counts + kSlotOvf, 1, ctx->stream));
-  CAS_TRY(fetch_words(ctx, ctx->h_counts_dev + kSlotNnz, ctx->d_counts + kSlotNnz, 1, ctx->stream));
   CAS_TRY(check_status(ctx));
   o.nnz = (int64_t)ctx->h_counts[kSlotNnz];
   return CAS_OK;
@@ -1858,13 +1845,12 @@ cas_status cas_create(int device, cas_ctx** out) {
       for (int b = 0; b < cas::kSymbBins; ++b) CAS_CUDA(ctx, cudaEventCreate(&ctx->ev_symb[i][b]));
       for (int b = 0; b < cas::kNumcBins; ++b) CAS_CUDA(ctx, cudaEventCreate(&ctx->ev_numc[i][b]));
     }
-    CAS_CUDA(ctx, cudaMalloc(&ctx->d_status, sizeof(cas::DevStatus)));
     CAS_CUDA(ctx, cudaMalloc(&ctx->d_counts, sizeof(unsigned long long) * kCountSlots));
     CAS_CUDA(ctx, cudaMallocHost(&ctx->h_counts, sizeof(unsigned long long) * kCountSlots));
-    CAS_CUDA(ctx, cudaMallocHost(&ctx->h_status, sizeof(cas::DevStatus)));
+    ctx->d_status = reinterpret_cast<cas::DevStatus*>(ctx->d_counts + kSlotStatus);
+    ctx->h_status = reinterpret_cast<cas::DevStatus*>(ctx->h_counts + kSlotStatus);
     CAS_CUDA(ctx, cudaMallocHost(&ctx->h_misc, sizeof(unsigned long long) * kMiscWords));
     CAS_CUDA(ctx, cudaHostGetDevicePointer((void**)&ctx->h_counts_dev, ctx->h_counts, 0));
-    CAS_CUDA(ctx, cudaHostGetDevicePointer((void**)&ctx->h_status_dev, ctx->h_status, 0));
     CAS_CUDA(ctx, cudaHostGetDevicePointer((void**)&ctx->h_misc_dev, ctx->h_misc, 0));
     // keep freed device memory in the stream-ordered pool between calls
     cudaMemPool_t pool;
@@ -1910,10 +1896,8 @@ void cas_destroy(cas_ctx* ctx) {
     for (int b = 0; b < cas::kNumcBins; ++b)
       if (ctx->ev_numc[i][b]) cudaEventDestroy(ctx->ev_numc[i][b]);
   }
-  if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->d_counts) cudaFree(ctx->d_counts);
   if (ctx->h_counts) cudaFreeHost(ctx->h_counts);
-  if (ctx->h_status) cudaFreeHost(ctx->h_status);
   if (ctx->h_misc) cudaFreeHost(ctx->h_misc);
   for (int i = 0; i < kStageBufs; ++i) {
     if (ctx->h_stage[i]) cudaFreeHost(ctx->h_stage[i]);
@@ -2045,14 +2029,8 @@ cas_status cas_flp_populate(cas_ctx* ctx, const cas_csr* A, const cas_csr* B, in
   Call c;
   double h2d = 0;
   CAS_TRY(prepare(ctx, A, B, c, h2d));
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts, 0, sizeof(unsigned long long) * kCountSlots, ctx->stream));
-  CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(cas::DevStatus), ctx->stream));
-  if (c.m > 0) {
-    cas::k_flp<256><<<grid_for(c.m * 32, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-        c.A.csr, c.B.csr, c.ncol, d_row_flp, ctx->d_counts + kSlotTotals, ctx->d_counts + kSlotSymb, ctx->d_status,
-        0, ctx->d_counts + kSlotFused);
-    CAS_TRY(check_launch(ctx, "k_flp"));
-  }
+  CAS_TRY(clear_counts(ctx));
+  CAS_TRY(launch_flp(ctx, c, false, false, d_row_flp, 0));
   return check_status(ctx);
 }
 
@@ -2068,6 +2046,17 @@ cas_status cas_scan(cas_ctx* ctx, int64_t* d_out, const int64_t* d_in, int64_t n
   return st;
 }
 
+// The end of a phase call: its scratch freed, the kernels' status.
+static cas_status phase_end(cas_ctx* ctx, Call& c, cas_status st) {
+  if (st != CAS_OK) {
+    quiesce(ctx);
+    scratch_free(ctx, c);
+    return st;
+  }
+  CAS_TRY(scratch_free(ctx, c));
+  return check_status(ctx);
+}
+
 cas_status cas_hash_symb(cas_ctx* ctx, const cas_csr* A, const cas_csr* B, const int64_t* d_row_flp,
                          int64_t* d_row_nz) {
   if (!ctx || !d_row_nz) return CAS_ERR_BAD_INPUT;
@@ -2077,10 +2066,11 @@ cas_status cas_hash_symb(cas_ctx* ctx, const cas_csr* A, const cas_csr* B, const
   Call c;
   double h2d = 0;
   CAS_TRY(prepare(ctx, A, B, c, h2d));
-  CAS_TRY(phase_init(ctx, c, true));
-  CAS_TRY(launch_symb_bins(ctx, c, d_row_nz));
-  CAS_TRY(scratch_free(ctx, c));
-  return check_status(ctx);
+  const cas_status st = [&]() -> cas_status {
+    CAS_TRY(phase_init(ctx, c, true));
+    return launch_symb_bins(ctx, c, d_row_nz);
+  }();
+  return phase_end(ctx, c, st);
 }
 
 static cas_status numc_entry(cas_ctx* ctx, cas_accum accum, const cas_csr* A, const cas_csr* B, cas_csr* C) {
@@ -2090,14 +2080,16 @@ static cas_status numc_entry(cas_ctx* ctx, cas_accum accum, const cas_csr* A, co
   Call c;
   double h2d = 0;
   CAS_TRY(prepare(ctx, A, B, c, h2d));
-  CAS_TRY(phase_init(ctx, c, true));
-  CAS_TRY(numc_bins(ctx, c, C->row_ptrs, mode_of(accum)));
-  if (c.vt == CAS_VAL_F64)
-    CAS_TRY(launch_numc_bins<double>(ctx, c, C->row_ptrs, static_cast<int32_t*>(C->cols), C->rats));
-  else
-    CAS_TRY(launch_numc_bins<int32_t>(ctx, c, C->row_ptrs, static_cast<int32_t*>(C->cols), C->rats));
-  CAS_TRY(scratch_free(ctx, c));
-  return check_status(ctx);
+  const cas_status st = [&]() -> cas_status {
+    CAS_TRY(phase_init(ctx, c, true));
+    CAS_TRY(launch_numc_count(ctx, c, C->row_ptrs, mode_of(accum)));
+    CAS_TRY(fetch_counts(ctx));
+    numc_counts(ctx, c);
+    if (c.vt == CAS_VAL_F64)
+      return launch_numc_bins<double>(ctx, c, C->row_ptrs, static_cast<int32_t*>(C->cols), C->rats);
+    return launch_numc_bins<int32_t>(ctx, c, C->row_ptrs, static_cast<int32_t*>(C->cols), C->rats);
+  }();
+  return phase_end(ctx, c, st);
 }
 
 cas_status cas_hash_numc(cas_ctx* ctx, const cas_csr* A, const cas_csr* B, const int64_t* d_row_flp, cas_csr* C) {

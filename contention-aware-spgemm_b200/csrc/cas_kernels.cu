@@ -6,15 +6,83 @@ namespace cas {
 
 // ===================================================================== INIT
 
-// One warp per row of A: row_flp[i] = sum over A_i of |B_k|, the symbolic
-// bin histogram, and the block-reduced total and maximum.  Columns outside
-// [0, B.nrow) are reported and skipped.
-template <int BLOCK>
+// Walks the rows of a CSR: G lanes a row, and the whole block for rows of
+// more than 64 G entries, after the others (one row of a skewed graph's hub
+// kept a warp busy for most of the kernel's time).  begin(r, s, e) says whether
+// the row's entries are looked at, entry(r, c, next) is summed over them (the
+// column and the next one of the row, or the largest int32), end(r, s, e, sum)
+// runs in one thread.  The columns of four entries a lane are loaded before any
+// is used.  next is loaded where `pairs` says so.
+constexpr int kLongRows = 128;  // listed per block; more are walked by their lanes
+template <int BLOCK, int G, typename Begin, typename Entry, typename End>
+__device__ __forceinline__ void for_rows(int64_t nrow, const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                                         bool pairs, Begin&& begin, Entry&& entry, End&& end) {
+  constexpr int U = 4;
+  // entries s + first, s + first + step, ... of row r
+  auto walk = [&](int64_t r, int64_t s, int64_t e, int first, int step) -> long long {
+    long long sum = 0;
+    for (int64_t j = s + first; j < e; j += (int64_t)U * step) {
+      int32_t c[U], next[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = j + (int64_t)u * step;
+        c[u] = i < e ? col[i] : -1;
+        next[u] = pairs && i + 1 < e ? col[i + 1] : 0x7FFFFFFF;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (j + (int64_t)u * step < e) sum += entry(r, c[u], next[u]);
+    }
+    return sum;
+  };
+  __shared__ int s_nlong;
+  __shared__ int64_t s_long[kLongRows];
+  __shared__ long long s_tmp[BLOCK / 32 + 1];
+  if (threadIdx.x == 0) s_nlong = 0;
+  __syncthreads();
+  const int sub = threadIdx.x & (G - 1);
+  const unsigned lanes = (G == 32 ? kFull : ((1u << (G & 31)) - 1u) << (threadIdx.x & 31 & ~(G - 1)));
+  // a warp takes 32 / G consecutive rows, a block's warps rows far apart: the
+  // hubs of a graph, and the popular columns of a join, lie side by side
+  const int64_t groups = (int64_t)gridDim.x * (BLOCK / G);
+  const int64_t chunk = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  for (int64_t r = chunk * (32 / G) + (threadIdx.x & 31) / G; r < nrow; r += groups) {
+    const int64_t s = rp[r], e = rp[r + 1];
+    if (!begin(r, s, e)) continue;
+    if (e - s > 64 * G) {
+      int at = 0;
+      if (sub == 0) at = atomicAdd(&s_nlong, 1);
+      at = __shfl_sync(lanes, at, 0, G);
+      if (at < kLongRows) {
+        if (sub == 0) s_long[at] = r;
+        continue;
+      }
+    }
+    long long sum = walk(r, s, e, sub, G);
+#pragma unroll
+    for (int d = G / 2; d > 0; d >>= 1) sum += __shfl_xor_sync(lanes, sum, d, G);
+    if (sub == 0) end(r, s, e, sum);
+  }
+  __syncthreads();
+  const int nlong = s_nlong < kLongRows ? s_nlong : kLongRows;
+  for (int i = 0; i < nlong; ++i) {
+    const int64_t r = s_long[i], s = rp[r], e = rp[r + 1];
+    const long long sum = block_sum<BLOCK, long long>(walk(r, s, e, threadIdx.x, BLOCK), s_tmp);
+    if (threadIdx.x == 0) end(r, s, e, sum);
+  }
+}
+
+// Row products: row_flp[i] = sum over A_i of |B_k|, the symbolic bin
+// histogram, and the total and maximum.  With CHECK, A is checked on the way
+// (flags[0]: row pointers or columns out of range; flags[3]: rows not sorted,
+// where A is also B), and its faulty rows and entries are skipped; without, a
+// column outside [0, B.nrow) is reported.
+template <int BLOCK, int G, bool CHECK>
 __global__ void __launch_bounds__(BLOCK)
-k_flp(Csr A, Csr B, int64_t c_ncol, int64_t* __restrict__ row_flp,
+k_flp(Csr A, Csr B, int64_t a_nnz, int a_is_b, int64_t c_ncol, int64_t* __restrict__ row_flp,
       unsigned long long* __restrict__ totals, unsigned long long* __restrict__ bin_count,
-      DevStatus* st, int fuse, unsigned long long* __restrict__ fused_sums) {
-  __shared__ unsigned long long s_cnt[kSymbBins];
+      unsigned long long* __restrict__ flags, DevStatus* st, int fuse, unsigned long long* __restrict__ fused_sums) {
+  __shared__ unsigned int s_cnt[kSymbBins];
   __shared__ unsigned long long s_tot, s_max, s_f[4];
   unsigned long long my_f[4] = {0, 0, 0, 0};
   if (threadIdx.x < kSymbBins) s_cnt[threadIdx.x] = 0;
@@ -22,45 +90,84 @@ k_flp(Csr A, Csr B, int64_t c_ncol, int64_t* __restrict__ row_flp,
   if (threadIdx.x == 0) { s_tot = 0; s_max = 0; }
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int64_t nw = ((int64_t)gridDim.x * BLOCK) >> 5;
   unsigned long long my_tot = 0, my_max = 0;
-  for (int64_t r = ((int64_t)blockIdx.x * BLOCK + threadIdx.x) >> 5; r < A.nrow; r += nw) {
-    const int64_t s = A.rp[r], e = A.rp[r + 1];
-    long long sum = 0;
-    for (int64_t j = s + lane; j < e; j += 32) {
-      const int32_t k = A.col[j];
-      if ((uint64_t)k >= (uint64_t)B.nrow) {
-        dev_report(st, kDevBadIndex, 0, r);
-        continue;
-      }
-      sum += B.rp[k + 1] - B.rp[k];
-    }
-    sum = warp_sum(sum);
-    if (lane == 0) {
-      row_flp[r] = sum;
-      my_tot += (unsigned long long)sum;
-      my_max = max(my_max, (unsigned long long)sum);
-      atomicAdd(&s_cnt[symb_bin_of(sum, c_ncol, fuse)], 1ull);
-      if (fused_row(sum, fuse)) {  // fused rows: count, products, output bound, nnz(A)
-        my_f[0] += 1;
-        my_f[1] += (unsigned long long)sum;
-        my_f[2] += (unsigned long long)(sum < c_ncol ? sum : c_ncol);
-        my_f[3] += (unsigned long long)(e - s);
-      }
-    }
-  }
-  if (lane == 0 && my_f[0])
+  bool bad = false, unsorted = false;
+  for_rows<BLOCK, G>(
+      A.nrow, A.rp, A.col, CHECK && a_is_b,
+      [&](int64_t r, int64_t s, int64_t e) {
+        if (!CHECK || (s >= 0 && e >= s && e <= a_nnz)) return true;
+        bad = true;
+        if ((threadIdx.x & (G - 1)) == 0) {
+          row_flp[r] = 0;
+          atomicAdd(&s_cnt[kSB_Zero], 1u);
+        }
+        return false;
+      },
+      [&](int64_t r, int32_t c, int32_t next) -> long long {
+        const bool ok = (uint64_t)c < (uint64_t)B.nrow;
+        const int32_t k = ok ? c : 0;
+        if (CHECK) {
+          bad |= !ok;
+          unsorted |= next < c;
+        } else if (!ok) {
+          dev_report(st, kDevBadIndex, 0, r);
+        }
+        return ok ? B.rp[k + 1] - B.rp[k] : 0;
+      },
+      [&](int64_t r, int64_t s, int64_t e, long long sum) {
+        row_flp[r] = sum;
+        my_tot += (unsigned long long)sum;
+        my_max = max(my_max, (unsigned long long)sum);
+        atomicAdd(&s_cnt[symb_bin_of(sum, c_ncol, fuse)], 1u);
+        if (fused_row(sum, fuse)) {  // fused rows: count, products, output bound, nnz(A)
+          my_f[0] += 1;
+          my_f[1] += (unsigned long long)sum;
+          my_f[2] += (unsigned long long)(sum < c_ncol ? sum : c_ncol);
+          my_f[3] += (unsigned long long)(e - s);
+        }
+      });
+  if (my_f[0])
     for (int i = 0; i < 4; ++i) atomicAdd(&s_f[i], my_f[i]);
+  my_tot = warp_sum(my_tot);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) my_max = max(my_max, __shfl_xor_sync(kFull, my_max, d));
   if (lane == 0) {
     atomicAdd(&s_tot, my_tot);
     atomicMax(&s_max, my_max);
   }
-  __syncthreads();
-  if (threadIdx.x < kSymbBins && s_cnt[threadIdx.x]) atomicAdd(&bin_count[threadIdx.x], s_cnt[threadIdx.x]);
+  const int any_bad = __syncthreads_or(bad), any_unsorted = __syncthreads_or(unsorted);
+  if (threadIdx.x < kSymbBins && s_cnt[threadIdx.x]) atomicAdd(&bin_count[threadIdx.x], (unsigned long long)s_cnt[threadIdx.x]);
   if (threadIdx.x < 4 && s_f[threadIdx.x]) atomicAdd(&fused_sums[threadIdx.x], s_f[threadIdx.x]);
   if (threadIdx.x == 0) {
     atomicAdd(&totals[0], s_tot);
     atomicMax(&totals[1], s_max);
+    if (any_bad) atomicOr(&flags[0], 1ull);
+    if (any_unsorted) atomicOr(&flags[3], 1ull);
+  }
+}
+
+// Row pointers non-decreasing and within [0, nnz], column indices in [0,
+// ncol) (flags[0]); flags[1] is set when some row is not sorted.
+template <int BLOCK, int G>
+__global__ void __launch_bounds__(BLOCK) k_check_csr(Csr M, int64_t nnz, unsigned long long* __restrict__ flags) {
+  bool bad = false, unsorted = false;
+  for_rows<BLOCK, G>(
+      M.nrow, M.rp, M.col, true,
+      [&](int64_t, int64_t s, int64_t e) {
+        const bool ok = s >= 0 && e >= s && e <= nnz;
+        bad |= !ok;
+        return ok;
+      },
+      [&](int64_t, int32_t c, int32_t next) -> long long {
+        bad |= (uint64_t)c >= (uint64_t)M.ncol;
+        unsorted |= next < c;
+        return 0;
+      },
+      [](int64_t, int64_t, int64_t, long long) {});
+  const int any_bad = __syncthreads_or(bad), any_unsorted = __syncthreads_or(unsorted);
+  if (threadIdx.x == 0) {
+    if (any_bad) atomicOr(&flags[0], 1ull);
+    if (any_unsorted) atomicOr(&flags[1], 1ull);
   }
 }
 
@@ -107,14 +214,22 @@ __global__ void k_fetch_words(unsigned long long* __restrict__ dst, const unsign
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
-// Rows into per-bin lists.  cursor[b] starts at the bin's offset; lanes that
-// hit the same bin share one atomic (warp-aggregated).
+// Rows into per-bin lists: the bins follow each other in `rows` by their
+// counts, cursor[b] (zero before) counts the rows placed; lanes that hit the
+// same bin share one atomic (warp-aggregated).
 __global__ void k_bin_scatter_symb(int64_t m, const int64_t* __restrict__ row_flp, int64_t c_ncol,
+                                   const unsigned long long* __restrict__ bin_count,
                                    unsigned long long* __restrict__ cursor, int32_t* __restrict__ rows, int fuse) {
+  __shared__ unsigned long long s_off[kSymbBins];
+  if (threadIdx.x < kSymbBins) {
+    unsigned long long off = 0;
+    for (int b = 0; b < (int)threadIdx.x; ++b) off += bin_count[b];
+    s_off[threadIdx.x] = off;
+  }
+  __syncthreads();
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
     const int b = symb_bin_of(row_flp[r], c_ncol, fuse);
-    const unsigned long long pos = warp_aggregated_add(cursor, b);
-    rows[pos] = (int32_t)r;
+    rows[s_off[b] + warp_aggregated_add(cursor, b)] = (int32_t)r;
   }
 }
 
@@ -140,40 +255,85 @@ __device__ __forceinline__ int heavy_class(int64_t flp) {  // 0 for the heaviest
   return l >= kHeavyClasses ? 0 : kHeavyClasses - 1 - l;
 }
 
-__global__ void k_bin_count_numc(int64_t m, const int64_t* __restrict__ row_flp, const int64_t* __restrict__ crp,
-                                 const int64_t* __restrict__ arp, int mode, double thres, int esc_max, int hash_max,
-                                 unsigned long long* __restrict__ bin_count, unsigned long long* __restrict__ bin_sums,
-                                 unsigned long long* __restrict__ heavy_count) {
-  __shared__ unsigned long long s_cnt[4 * kNumcBins];
-  __shared__ unsigned long long s_heavy[kHeavyClasses];
-  if (threadIdx.x < 4 * kNumcBins) s_cnt[threadIdx.x] = 0;
+// The sums go by warp, once for each bin that its rows fall into (one to
+// three, as a rule): four 64-bit shared atomics a row on a handful of
+// addresses took 95 us for 500,000 rows (22 us for 256), this takes 11 (5).
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK)
+k_bin_count_numc(int64_t m, const int64_t* __restrict__ row_flp, const int64_t* __restrict__ crp,
+                 const int64_t* __restrict__ arp, int mode, double thres, int esc_max, int hash_max,
+                 unsigned long long* __restrict__ bin_count, unsigned long long* __restrict__ bin_sums,
+                 unsigned long long* __restrict__ heavy_count) {
+  __shared__ unsigned long long s_sum[BLOCK / 32][4 * kNumcBins];  // per warp: rows, products, nnz(C), nnz(A)
+  __shared__ unsigned int s_heavy[kHeavyClasses];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < (BLOCK / 32) * 4 * kNumcBins; i += BLOCK) (&s_sum[0][0])[i] = 0;
   if (threadIdx.x < kHeavyClasses) s_heavy[threadIdx.x] = 0;
   __syncthreads();
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t flp = row_flp[r], nz = crp[r + 1] - crp[r];
-    const int b = numc_bin_of(flp, nz, mode, thres, esc_max, hash_max);
-    if (b == kNB_Dense) atomicAdd(&s_heavy[heavy_class(flp)], 1ull);
-    atomicAdd(&s_cnt[b], 1ull);
-    atomicAdd(&s_cnt[kNumcBins + b], (unsigned long long)flp);
-    atomicAdd(&s_cnt[2 * kNumcBins + b], (unsigned long long)nz);
-    atomicAdd(&s_cnt[3 * kNumcBins + b], (unsigned long long)(arp[r + 1] - arp[r]));
+  const int64_t stride = (int64_t)gridDim.x * BLOCK;
+  for (int64_t r0 = (int64_t)blockIdx.x * BLOCK + warp * 32; r0 < m; r0 += stride) {
+    const int64_t r = r0 + lane;
+    int b = -1;
+    long long flp = 0, nz = 0, nza = 0;
+    if (r < m) {
+      flp = row_flp[r];
+      nz = crp[r + 1] - crp[r];
+      nza = arp[r + 1] - arp[r];
+      b = numc_bin_of(flp, nz, mode, thres, esc_max, hash_max);
+      if (b == kNB_Dense) atomicAdd(&s_heavy[heavy_class(flp)], 1u);
+    }
+    for (unsigned left = __ballot_sync(kFull, b >= 0); left;) {
+      const int cur = __shfl_sync(kFull, b, __ffs(left) - 1);
+      const bool mine = b == cur;
+      const unsigned in = __ballot_sync(kFull, mine);
+      const long long f = warp_sum(mine ? flp : 0ll), c = warp_sum(mine ? nz : 0ll), a = warp_sum(mine ? nza : 0ll);
+      if (lane == 0) {
+        unsigned long long* t = s_sum[warp] + cur;
+        t[0] += __popc(in);
+        t[kNumcBins] += (unsigned long long)f;
+        t[2 * kNumcBins] += (unsigned long long)c;
+        t[3 * kNumcBins] += (unsigned long long)a;
+      }
+      left &= ~in;
+    }
   }
   __syncthreads();
-  if (threadIdx.x < kNumcBins && s_cnt[threadIdx.x]) atomicAdd(&bin_count[threadIdx.x], s_cnt[threadIdx.x]);
-  if (threadIdx.x >= kNumcBins && threadIdx.x < 4 * kNumcBins && s_cnt[threadIdx.x])
-    atomicAdd(&bin_sums[threadIdx.x - kNumcBins], s_cnt[threadIdx.x]);
-  if (threadIdx.x < kHeavyClasses && s_heavy[threadIdx.x]) atomicAdd(&heavy_count[threadIdx.x], s_heavy[threadIdx.x]);
+  if (threadIdx.x < 4 * kNumcBins) {
+    unsigned long long t = 0;
+    for (int w = 0; w < BLOCK / 32; ++w) t += s_sum[w][threadIdx.x];
+    if (t) atomicAdd(threadIdx.x < kNumcBins ? &bin_count[threadIdx.x] : &bin_sums[threadIdx.x - kNumcBins], t);
+  }
+  if (threadIdx.x < kHeavyClasses && s_heavy[threadIdx.x])
+    atomicAdd(&heavy_count[threadIdx.x], (unsigned long long)s_heavy[threadIdx.x]);
 }
 
+// Rows into their numeric bins' lists, as k_bin_scatter_symb; the dense rows by
+// size class, the heaviest first.
 __global__ void k_bin_scatter_numc(int64_t m, const int64_t* __restrict__ row_flp, const int64_t* __restrict__ crp,
                                    int mode, double thres, int esc_max, int hash_max,
+                                   const unsigned long long* __restrict__ bin_count,
+                                   const unsigned long long* __restrict__ heavy_count,
                                    unsigned long long* __restrict__ cursor,
                                    unsigned long long* __restrict__ heavy_cursor, int32_t* __restrict__ rows) {
+  __shared__ unsigned long long s_off[kNumcBins], s_heavy[kHeavyClasses];
+  if (threadIdx.x < kNumcBins) {
+    unsigned long long off = 0;
+    for (int b = 0; b < (int)threadIdx.x; ++b) off += bin_count[b];
+    s_off[threadIdx.x] = off;
+  }
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + kHeavyClasses) {
+    unsigned long long off = 0;
+    for (int b = 0; b < kNB_Dense; ++b) off += bin_count[b];
+    for (int k = 0; k < (int)threadIdx.x - 64; ++k) off += heavy_count[k];
+    s_heavy[threadIdx.x - 64] = off;
+  }
+  __syncthreads();
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
     const int64_t flp = row_flp[r];
     const int b = numc_bin_of(flp, crp[r + 1] - crp[r], mode, thres, esc_max, hash_max);
-    const unsigned long long pos =
-        b == kNB_Dense ? warp_aggregated_add(heavy_cursor, heavy_class(flp)) : warp_aggregated_add(cursor, b);
+    const int h = b == kNB_Dense ? heavy_class(flp) : 0;
+    const unsigned long long pos = b == kNB_Dense ? s_heavy[h] + warp_aggregated_add(heavy_cursor, h)
+                                                  : s_off[b] + warp_aggregated_add(cursor, b);
     rows[pos] = (int32_t)r;
   }
 }
@@ -198,6 +358,29 @@ k_scan_partials(const int64_t* __restrict__ in, int64_t n_in, int64_t* __restric
   }
   s = block_sum<kScanBlock, long long>(s, tmp);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+
+// a scan of one tile in one launch
+__global__ void __launch_bounds__(kScanBlock)
+k_scan_tile(const int64_t* __restrict__ in, int64_t n_in, int64_t* __restrict__ out, int64_t n_out,
+            int64_t* __restrict__ total_out) {
+  __shared__ long long tmp[kScanBlock / 32 + 1];
+  const int64_t base = (int64_t)threadIdx.x * kScanItems;
+  long long v[kScanItems];
+  long long s = 0;
+#pragma unroll
+  for (int u = 0; u < kScanItems; ++u) {
+    v[u] = base + u < n_in ? in[base + u] : 0;
+    s += v[u];
+  }
+  long long tot;
+  long long run = block_exclusive_sum<kScanBlock, long long>(s, tmp, tot);
+#pragma unroll
+  for (int u = 0; u < kScanItems; ++u) {
+    if (base + u < n_out) out[base + u] = run;
+    run += v[u];
+  }
+  if (threadIdx.x == 0 && total_out) *total_out = tot;
 }
 
 // single block: exclusive scan of the tile partials (any count, in rounds)

@@ -311,9 +311,7 @@ extern "C" cas_status cas_csr_transpose(cas_ctx* ctx, const cas_csr* A, cas_csr*
     CAS_CUDA(ctx, cudaMemsetAsync(ctx->d_counts, 0, sizeof(unsigned long long) * kCountSlots, ctx->stream));
     cas::Csr a = dA.csr;
     if (a.nrow > 0) {
-      cas::k_check_csr<<<grid_for(a.nrow * 32, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-          a, A->num_nnz, ctx->d_counts + kSlotCheck);
-      rc = check_launch(ctx, "k_check_csr");
+      rc = launch_check(ctx, a, A->num_nnz, ctx->d_counts + kSlotCheck);
       if (rc == CAS_OK) {
         unsigned long long bad = 0;
         if (cudaMemcpyAsync(&bad, ctx->d_counts + kSlotCheck, sizeof(bad), cudaMemcpyDeviceToHost, ctx->stream) !=
