@@ -46,7 +46,7 @@ constexpr int kMiscWords = 8;    // pinned words of other small results
 constexpr int kSlotSymb = 0;     // [0, 9)   symbolic bin counts
 constexpr int kSlotNumc = 10;    // [10, 23) numeric bin counts
 constexpr int kSlotTotals = 24;  // [24]    products, [25] max row products
-constexpr int kSlotCursor = 28;  // [28, 41) numeric bin cursors
+constexpr int kSlotCursor = 28;  // [28, 43) numeric bin cursors
 constexpr int kSlotNnz = 44;     // [44]    nnz(C) from the scan
 constexpr int kSlotCheck = 48;   // [48, 52) input check flags
 constexpr int kSlotBinSums = 64; // [64, 103) per numeric bin: products, nnz(C), nnz(A)
@@ -55,6 +55,7 @@ constexpr int kSlotFused = 112;  // [112, 116) fused rows: count, products, outp
 constexpr int kSlotHeavy = 128;  // [128, 176) dense rows per size class
 constexpr int kSlotHeavyCur = 176;  // [176, 224) their cursors
 constexpr int kSlotSymbCur = 228;   // [228, 237) symbolic bin cursors
+constexpr int kSlotSmall = 240;     // [240, 242) rows of the kNB_E1K and kNB_H256 bins that a warp takes
 constexpr int kSlotStatus = 256;    // [256, 258) the device status, behind the counters
 constexpr size_t kStageBytes = size_t(64) << 20;  // pinned staging chunk for host copies
 constexpr double kSavedBitmapBytes = 8.0 * (1ull << 30);  // heavy-row bitmaps kept between the phases
@@ -270,6 +271,11 @@ constexpr size_t smem_numc_esc_idx() {
   X(256, 3, 6144)          \
   X(256, 2, 8192)
 
+// Enough rows for a warp each: with fewer than fill the chip's blocks, one
+// row's own time counts, and a block is done with it sooner (185 rows of up to
+// 512 products: 12 us by blocks, 32 by warps).
+bool many_rows(const cas_ctx* ctx, int64_t rows) { return rows >= 8 * (int64_t)ctx->sm_count; }
+
 // The ranked bitmap (esc_form 2) takes matrices of at most 2^kRankBits
 // columns, what its two levels can tell apart; wider ones take
 // k_numc_esc_idx with the keys in registers.
@@ -294,6 +300,8 @@ cas_status setup_numc_kernels(cas_ctx* ctx) {
 #define CAS_SETUP_RANK(BLOCK, MINB, CAP)                                                                   \
   CAS_TRY(allow_smem(ctx, k_numc_rank<BLOCK, MINB, CAP, VIn, false>, smem_numc_rank<BLOCK, CAP, VIn>(kRankCellBits)));
   CAS_RANK_SHAPES(CAS_SETUP_RANK)
+  CAS_TRY(allow_smem(ctx, k_numc_warp<VIn>,
+                     kWarpsPerBlock * smem_numc_warp<VIn>(rank_cell_bits<kWarpProducts>(int64_t(1) << kRankBits))));
 #undef CAS_SETUP_RANK
   CAS_TRY(allow_smem(ctx, k_numc_rank<256, 4, (int)kFusedHi, VIn, true>,
                      smem_numc_rank<256, (int)kFusedHi, VIn>(kRankCellBits)));
@@ -313,6 +321,7 @@ cas_status setup_kernels(cas_ctx* ctx) {
 #define CAS_SETUP_SYMB(bin, BLK, TB, SEG) CAS_TRY(allow_smem(ctx, k_symb_hash<BLK, TB, SEG>, smem_symb_hash<BLK, TB, SEG>()));
   CAS_SYMB_SHAPES(CAS_SETUP_SYMB)
 #undef CAS_SETUP_SYMB
+  CAS_TRY(allow_smem(ctx, k_symb_warp<10>, kWarpsPerBlock * sizeof(SymbWarp<10>)));
   CAS_TRY(allow_smem(ctx, k_symb_dense<512>, smem_symb_dense<512>()));
   CAS_TRY(allow_smem(ctx, k_heavy_bits<512>, smem_symb_dense<512>()));
   CAS_TRY(setup_numc_kernels<double>(ctx));
@@ -1086,6 +1095,14 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
         break;
 #define CAS_SYMB_CASE(bin, BLK, TB, SEG)                                                              \
       case bin:                                                                                     \
+        if constexpr (TB == 10) { /* a warp per row, where their products fit its table */          \
+          if (c.ncol > kWarpProducts && many_rows(ctx, n)) {                                        \
+            k_symb_warp<10><<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock),                \
+                              32 * kWarpsPerBlock, kWarpsPerBlock * sizeof(SymbWarp<10>), s>>>(     \
+                rows, n, c.A.csr, c.B.csr, row_nz, ctx->d_status);                                  \
+            break;                                                                                  \
+          }                                                                                         \
+        }                                                                                           \
         k_symb_hash<BLK, TB, SEG><<<(unsigned)n, BLK, smem_symb_hash<BLK, TB, SEG>(), s>>>(          \
             rows, c.A.csr, c.B.csr, row_nz, ctx->d_status);                                         \
         break;
@@ -1133,11 +1150,11 @@ cas_status launch_numc_count(cas_ctx* ctx, Call& c, const int64_t* crp, int mode
   unsigned long long* k = ctx->d_counts;
   k_bin_count_numc<256><<<grid_for(c.m, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(
       c.m, c.row_flp, crp, c.A.csr.rp, mode, ctx->acc_thres, ctx->esc_max, ctx->hash_max, k + kSlotNumc,
-      k + kSlotBinSums, k + kSlotHeavy);
+      k + kSlotBinSums, k + kSlotHeavy, k + kSlotSmall);
   CAS_TRY(check_launch(ctx, "k_bin_count_numc"));
   k_bin_scatter_numc<<<grid_for(c.m, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-      c.m, c.row_flp, crp, mode, ctx->acc_thres, ctx->esc_max, ctx->hash_max, k + kSlotNumc, k + kSlotHeavy,
-      k + kSlotCursor, k + kSlotHeavyCur, c.rows);
+      c.m, c.row_flp, crp, c.A.csr.rp, mode, ctx->acc_thres, ctx->esc_max, ctx->hash_max, k + kSlotNumc,
+      k + kSlotHeavy, k + kSlotSmall, k + kSlotCursor, k + kSlotHeavyCur, c.rows);
   return check_launch(ctx, "k_bin_scatter_numc");
 }
 void numc_counts(cas_ctx* ctx, Call& c) {
@@ -1254,17 +1271,39 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
   unsigned int* ovf_count = reinterpret_cast<unsigned int*>(ctx->d_counts + kSlotOvf);
   CAS_TRY(fork(ctx));
   const bool rank = rank_form(ctx, c.ncol);
+  // The warps' rows lead their two bins.  Wider than 2^kWarpBits columns a
+  // warp's bitmap is much for it to clear and scan, and leaves fewer warps on an
+  // SM: 192,500 join rows over 6e5 columns take 1.33 ms by warps and 0.97 by
+  // k_numc_rank, 131,000 uniform rows over 1.3e5 0.50 and 0.72.  The hash rows,
+  // whose other kernel sorts, go by warps at any width.
+  auto by_warps = [&](int b, int64_t ws) {
+    return rank && many_rows(ctx, ws) && (b == kNB_H256 || (b == kNB_E1K && c.ncol <= (int64_t(1) << kWarpBits)));
+  };
+  auto launch_warp = [&](const int32_t* wrows, int64_t n, cudaStream_t s) -> cas_status {
+    const int cell_bits = rank_cell_bits<kWarpProducts>(c.ncol);
+    k_numc_warp<VIn><<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), 32 * kWarpsPerBlock,
+                       kWarpsPerBlock * smem_numc_warp<VIn>(cell_bits), s>>>(
+        wrows, n, c.A.csr, c.B.csr, c.b_sorted ? 1 : 0, cell_bits, crp, ccol, cval, ctx->d_status);
+    return check_launch(ctx, "k_numc_warp");
+  };
   int64_t esc_rows = c.nf;  // fused rows may have handed rows to the radix-sort kernel too
   int si = 0;
   for (int oi = 0; oi < 12; ++oi) {
     const int b = order[oi];
-    const int64_t n = c.numc_count[b];
+    int64_t n = c.numc_count[b];
     if (n == 0) continue;
     const int32_t* rows = c.rows + off[b];
     cudaStream_t s = ctx->profile ? ctx->stream : ctx->aux[si++ % kAux];  // profiling: one bin at a time
     if (ctx->profile) CAS_CUDA(ctx, cudaEventRecord(ctx->ev_numc[0][b], s));
+    const int64_t ws = (int64_t)ctx->h_counts[kSlotSmall + (b == kNB_H256)];
+    if ((b == kNB_E1K || b == kNB_H256) && by_warps(b, ws)) {
+      CAS_TRY(launch_warp(rows, ws, s));
+      rows += ws;
+      n -= ws;
+    }
     const Csr& A = c.A.csr;
     const Csr& B = c.B.csr;
+    if (n > 0)
     switch (b) {
       case kNB_Tiny:
         k_numc_tiny<256, VIn><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(rows, n, A, B, crp, ccol, cval, ctx->d_status);
@@ -1310,7 +1349,7 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
         break;
       }
     }
-    CAS_TRY(check_launch(ctx, "numeric bin"));
+    if (n > 0) CAS_TRY(check_launch(ctx, "numeric bin"));
     if (ctx->profile) CAS_CUDA(ctx, cudaEventRecord(ctx->ev_numc[1][b], s));
   }
   CAS_TRY(join(ctx));

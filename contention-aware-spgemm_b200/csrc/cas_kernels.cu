@@ -244,6 +244,11 @@ __global__ void k_fused_scatter(int64_t m, const int64_t* __restrict__ row_flp, 
     if (fused_row(row_flp[r], fuse)) frows[pos[r]] = (int32_t)r;
 }
 
+// Rows a warp takes (k_symb_warp, k_numc_warp): products, and A entries.
+constexpr int kWarpProducts = 512;
+constexpr int kWarpEntries = 128;
+constexpr int kWarpBits = 18;  // log2 of the matrix's columns, at most, for the ESC rows
+
 // Numeric bin histogram plus, per bin, the sums of products, nnz(C) and
 // nnz(A) of its rows (for the per-kernel algorithmic byte count).
 // Heavy rows launch heaviest first (longest-processing-time order, so the
@@ -255,6 +260,12 @@ __device__ __forceinline__ int heavy_class(int64_t flp) {  // 0 for the heaviest
   return l >= kHeavyClasses ? 0 : kHeavyClasses - 1 - l;
 }
 
+// The rows of the kNB_E1K and kNB_H256 bins that a warp takes (warp_row) lead
+// their bins' lists; small_count has their numbers.
+__device__ __forceinline__ bool warp_row(int b, int64_t flp, int64_t nza) {
+  return (b == kNB_E1K || b == kNB_H256) && flp <= kWarpProducts && nza <= kWarpEntries;
+}
+
 // The sums go by warp, once for each bin that its rows fall into (one to
 // three, as a rule): four 64-bit shared atomics a row on a handful of
 // addresses took 95 us for 500,000 rows (22 us for 256), this takes 11 (5).
@@ -263,12 +274,14 @@ __global__ void __launch_bounds__(BLOCK)
 k_bin_count_numc(int64_t m, const int64_t* __restrict__ row_flp, const int64_t* __restrict__ crp,
                  const int64_t* __restrict__ arp, int mode, double thres, int esc_max, int hash_max,
                  unsigned long long* __restrict__ bin_count, unsigned long long* __restrict__ bin_sums,
-                 unsigned long long* __restrict__ heavy_count) {
+                 unsigned long long* __restrict__ heavy_count, unsigned long long* __restrict__ small_count) {
+  __shared__ unsigned int s_small[2];
   __shared__ unsigned long long s_sum[BLOCK / 32][4 * kNumcBins];  // per warp: rows, products, nnz(C), nnz(A)
   __shared__ unsigned int s_heavy[kHeavyClasses];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < (BLOCK / 32) * 4 * kNumcBins; i += BLOCK) (&s_sum[0][0])[i] = 0;
   if (threadIdx.x < kHeavyClasses) s_heavy[threadIdx.x] = 0;
+  if (threadIdx.x < 2) s_small[threadIdx.x] = 0;
   __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * BLOCK;
   for (int64_t r0 = (int64_t)blockIdx.x * BLOCK + warp * 32; r0 < m; r0 += stride) {
@@ -286,6 +299,8 @@ k_bin_count_numc(int64_t m, const int64_t* __restrict__ row_flp, const int64_t* 
       const int cur = __shfl_sync(kFull, b, __ffs(left) - 1);
       const bool mine = b == cur;
       const unsigned in = __ballot_sync(kFull, mine);
+      const unsigned small = __ballot_sync(kFull, mine && warp_row(b, flp, nza));
+      if (small && lane == 0) atomicAdd(&s_small[cur == kNB_H256], (unsigned)__popc(small));
       const long long f = warp_sum(mine ? flp : 0ll), c = warp_sum(mine ? nz : 0ll), a = warp_sum(mine ? nza : 0ll);
       if (lane == 0) {
         unsigned long long* t = s_sum[warp] + cur;
@@ -305,20 +320,28 @@ k_bin_count_numc(int64_t m, const int64_t* __restrict__ row_flp, const int64_t* 
   }
   if (threadIdx.x < kHeavyClasses && s_heavy[threadIdx.x])
     atomicAdd(&heavy_count[threadIdx.x], (unsigned long long)s_heavy[threadIdx.x]);
+  if (threadIdx.x < 2 && s_small[threadIdx.x]) atomicAdd(&small_count[threadIdx.x], (unsigned long long)s_small[threadIdx.x]);
 }
 
 // Rows into their numeric bins' lists, as k_bin_scatter_symb; the dense rows by
 // size class, the heaviest first.
 __global__ void k_bin_scatter_numc(int64_t m, const int64_t* __restrict__ row_flp, const int64_t* __restrict__ crp,
-                                   int mode, double thres, int esc_max, int hash_max,
+                                   const int64_t* __restrict__ arp, int mode, double thres, int esc_max, int hash_max,
                                    const unsigned long long* __restrict__ bin_count,
                                    const unsigned long long* __restrict__ heavy_count,
+                                   const unsigned long long* __restrict__ small_count,
                                    unsigned long long* __restrict__ cursor,
                                    unsigned long long* __restrict__ heavy_cursor, int32_t* __restrict__ rows) {
-  __shared__ unsigned long long s_off[kNumcBins], s_heavy[kHeavyClasses];
+  // a bin's rows, with the warps' rows of the two bins as bins of their own
+  __shared__ unsigned long long s_off[kNumcBins + 2], s_heavy[kHeavyClasses];
   if (threadIdx.x < kNumcBins) {
     unsigned long long off = 0;
     for (int b = 0; b < (int)threadIdx.x; ++b) off += bin_count[b];
+    const int small = threadIdx.x == kNB_E1K ? 0 : threadIdx.x == kNB_H256 ? 1 : -1;
+    if (small >= 0) {
+      s_off[kNumcBins + small] = off;
+      off += small_count[small];
+    }
     s_off[threadIdx.x] = off;
   }
   if (threadIdx.x >= 64 && threadIdx.x < 64 + kHeavyClasses) {
@@ -330,7 +353,8 @@ __global__ void k_bin_scatter_numc(int64_t m, const int64_t* __restrict__ row_fl
   __syncthreads();
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
     const int64_t flp = row_flp[r];
-    const int b = numc_bin_of(flp, crp[r + 1] - crp[r], mode, thres, esc_max, hash_max);
+    int b = numc_bin_of(flp, crp[r + 1] - crp[r], mode, thres, esc_max, hash_max);
+    if (warp_row(b, flp, arp[r + 1] - arp[r])) b = kNumcBins + (b == kNB_H256);
     const int h = b == kNB_Dense ? heavy_class(flp) : 0;
     const unsigned long long pos = b == kNB_Dense ? s_heavy[h] + warp_aggregated_add(heavy_cursor, h)
                                                   : s_off[b] + warp_aggregated_add(cursor, b);
@@ -2679,6 +2703,350 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
   }
   __syncthreads();
   for (int i = threadIdx.x; i < distinct; i += BLOCK) ccol[c0 + i] = (int32_t)scol[i];
+}
+
+// ---- a warp per row ---------------------------------------------------------
+// Rows of at most kWarpProducts products.  A block per row spends most of its
+// time at barriers between steps of a few hundred instructions; a warp needs
+// none, and some 30 rows are in flight on an SM.  Bound: issue slots and the
+// shared-memory pipe, each about 60% busy, and instruction fetches (the loops
+// over a lane's products are unrolled).  63,897 rows of 39 products over 5e5
+// columns: symbolic 167 us by blocks, 34 by warps; 130,923 rows of 272 over
+// 1.3e5: symbolic 436 and 240, numeric 725 and 504; 63,897 hash rows of 39 over
+// 5e5 columns took 671 us.
+constexpr int kWarpsPerBlock = 4;
+
+// Entry of this lane's product t + lane among ne entries with first products
+// pre[0..ne), pre[ne] their total: e0 is the first entry that starts at or
+// after t, and moves on to the next group.
+__device__ __forceinline__ int warp_entry(const uint32_t* pre, int ne, uint32_t t, int& e0, unsigned upto) {
+  const uint32_t d = pre[min(e0 + (int)(threadIdx.x & 31), ne)] - t;
+  const unsigned starts = __reduce_or_sync(kFull, d < 32u ? 1u << d : 0u);
+  const int e = e0 + __popc(starts & upto) - 1;
+  e0 += __popc(starts);
+  return min(e, ne - 1);
+}
+
+// The distinct columns of rows of at most 2^TBITS / 2 products: the hash of
+// k_symb_hash, a table and 32 staged A entries per warp.
+template <int TBITS>
+struct alignas(16) SymbWarp {
+  uint32_t tab[1 << TBITS];
+  int64_t off[32];
+  uint32_t pre[36];
+};
+template <int TBITS>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+k_symb_warp(const int32_t* __restrict__ rows, int64_t nrows, Csr A, Csr B, int64_t* __restrict__ row_nz, DevStatus* st) {
+  constexpr int T = 1 << TBITS;
+  extern __shared__ __align__(16) uint8_t smem[];
+  SymbWarp<TBITS>& sw = reinterpret_cast<SymbWarp<TBITS>*>(smem)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const unsigned upto = 0xFFFFFFFFu >> (31 - lane);
+  const int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (w >= nrows) return;
+  const int64_t r = rows[w];
+  for (int i = lane; i < T / 4; i += 32) reinterpret_cast<uint4*>(sw.tab)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  const int64_t as = A.rp[r], ae = A.rp[r + 1];
+  int cnt = 0;
+  uint32_t seen = 0;
+  for (int64_t a0 = as; a0 < ae; a0 += 32) {
+    int64_t bs = 0;
+    uint32_t len = 0;
+    if (a0 + lane < ae) {
+      const int32_t k = A.col[a0 + lane];
+      bs = B.rp[k];
+      len = (uint32_t)(B.rp[k + 1] - bs);
+    }
+    const uint32_t inc = warp_inclusive_sum(len);
+    const uint32_t total = __shfl_sync(kFull, inc, 31);
+    const unsigned some = __ballot_sync(kFull, len > 0);
+    const int ne = __popc(some);
+    seen += total;
+    if (seen > (uint32_t)(T / 2)) break;  // uniform: the bin bound was violated
+    if (len > 0) {
+      const int e = __popc(some & lanemask_lt());
+      sw.off[e] = bs - (int64_t)(inc - len);
+      sw.pre[e] = inc - len;
+    }
+    if (lane == 0) sw.pre[ne] = total;
+    __syncwarp();
+    int e0 = 0;
+    for (uint32_t t = 0; t < total; t += 32 * 4) {
+      int32_t key[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t p = t + 32 * u + lane;
+        key[u] = -1;
+        if (t + 32 * u < total) {
+          const int e = warp_entry(sw.pre, ne, t + 32 * u, e0, upto);
+          if (p < total) key[u] = __ldg(B.col + (sw.off[e] + p));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (key[u] < 0) continue;
+        uint32_t h = hash_slot((uint32_t)key[u], TBITS);
+        for (;;) {  // at most half the slots are taken: a free one comes up
+          const uint32_t old = atomicCAS(&sw.tab[h], kEmptyKey, (uint32_t)key[u]);
+          if (old == kEmptyKey) ++cnt;
+          if (old == kEmptyKey || old == (uint32_t)key[u]) break;
+          h = (h + 1) & (T - 1);
+        }
+      }
+    }
+    __syncwarp();
+  }
+  cnt = warp_sum(cnt);
+  if (lane == 0) {
+    row_nz[r] = cnt;
+    if (seen > (uint32_t)(T / 2)) dev_report(st, kDevCapacity, 18, r);
+  }
+}
+
+// k_numc_rank by warps: rows of at most kWarpProducts products and
+// kWarpEntries A entries.  The words of the scans are a warp's: no barrier.
+template <typename VIn>
+struct alignas(16) NumcWarp {
+  int64_t off[kWarpEntries];
+  VIn av[kWarpEntries];
+  uint32_t pre[kWarpEntries + 4];
+};
+template <typename VIn>
+__host__ __device__ constexpr size_t smem_numc_warp(int cell_bits) {  // of one warp
+  return rank_arena<kWarpProducts>(cell_bits) + sizeof(NumcWarp<VIn>);
+}
+
+template <typename VIn>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 8)
+k_numc_warp(const int32_t* __restrict__ rows, int64_t nrows, Csr A, Csr B, int32_t b_sorted, int cell_bits,
+            const int64_t* __restrict__ crp, int32_t* __restrict__ ccol, typename Acc<VIn>::T* __restrict__ cval,
+            DevStatus* st) {
+  using AT = typename Acc<VIn>::T;
+  constexpr int NPT = kWarpProducts / 32;  // products per lane: lane + 32 u
+  constexpr int G = 4;
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int lane = threadIdx.x & 31;
+  const unsigned upto = 0xFFFFFFFFu >> (31 - lane);
+  const int words = 1 << (cell_bits - 5);
+  uint32_t* bits = reinterpret_cast<uint32_t*>(smem + (threadIdx.x >> 5) * smem_numc_warp<VIn>(cell_bits));
+  uint16_t* wpre = reinterpret_cast<uint16_t*>(bits + words);
+  uint32_t* slot = reinterpret_cast<uint32_t*>(wpre + words);
+  AT* sval = reinterpret_cast<AT*>(bits);
+  NumcWarp<VIn>& sg = *reinterpret_cast<NumcWarp<VIn>*>(reinterpret_cast<uint8_t*>(bits) + rank_arena<kWarpProducts>(cell_bits));
+  const int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (w >= nrows) return;
+  const int64_t r = rows[w];
+  const int64_t as = A.rp[r], ae = A.rp[r + 1];
+  for (int i = lane; i < words / 4; i += 32) reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
+  // the nonempty entries, their first products and the columns' range
+  uint32_t n = 0, kmin = b_sorted ? 0xFFFFFFFFu : 0u;
+  uint32_t kmax = b_sorted ? 0u : (uint32_t)(B.ncol > 0 ? B.ncol - 1 : 0);
+  int ne = 0;
+  bool fits = ae - as <= kWarpEntries;
+  for (int64_t a0 = as; a0 < ae && fits; a0 += 32) {
+    int64_t bs = 0;
+    uint32_t len = 0;
+    VIn av = VIn(0);
+    if (a0 + lane < ae) {
+      const int32_t k = A.col[a0 + lane];
+      bs = B.rp[k];
+      const int64_t l = B.rp[k + 1] - bs;
+      len = l > kWarpProducts ? kWarpProducts + 1 : (uint32_t)l;
+      av = static_cast<const VIn*>(A.val)[a0 + lane];
+      if (b_sorted && len > 0) {
+        kmin = min(kmin, (uint32_t)__ldg(B.col + bs));
+        kmax = max(kmax, (uint32_t)__ldg(B.col + bs + l - 1));
+      }
+    }
+    const uint32_t inc = warp_inclusive_sum(len);
+    const unsigned some = __ballot_sync(kFull, len > 0);
+    if (len > 0) {
+      const int e = ne + __popc(some & lanemask_lt());
+      const uint32_t first = n + inc - len;
+      sg.off[e] = bs - (int64_t)first;
+      sg.pre[e] = first;
+      sg.av[e] = av;
+    }
+    ne += __popc(some);
+    n += __shfl_sync(kFull, inc, 31);
+    fits = n <= kWarpProducts;
+  }
+  if (lane == 0) sg.pre[ne] = n;
+  const uint32_t lo = __reduce_min_sync(kFull, kmin), hi = __reduce_max_sync(kFull, kmax);
+  const uint32_t range = hi > lo ? hi - lo : 0u;
+  const int rbits = 32 - __clz(range);
+  const int shift = rbits > cell_bits ? rbits - cell_bits : 0;
+  const int64_t c0 = crp[r];
+  const int64_t nz = crp[r + 1] - c0;
+  if (!fits || shift > 4) {  // uniform: the bin's bounds were violated
+    if (lane == 0) dev_report(st, kDevCapacity, 18, r);
+    return;
+  }
+  __syncwarp();
+  // columns; `pos` holds each product's entry in its upper 7 bits of 16
+  uint32_t key[NPT], pos[NPT / 2];
+  int e0 = 0;
+#pragma unroll
+  for (int g = 0; g < NPT; g += G) {
+    if (32u * g >= n) break;
+    uint32_t e[G];
+#pragma unroll
+    for (int v = 0; v < G; ++v) {
+      const uint32_t t = 32u * (g + v);
+      // a group past the last product reads as the last one
+      e[v] = t < n ? (uint32_t)warp_entry(sg.pre, ne, t, e0, upto) : (uint32_t)(ne - 1);
+      key[g + v] = (uint32_t)__ldg(B.col + (sg.off[e[v]] + min(t + lane, n - 1)));
+    }
+#pragma unroll
+    for (int v = 0; v < G; v += 2) pos[(g + v) >> 1] = (e[v] << 9) | (e[v + 1] << 25);
+  }
+  const uint32_t valid = n > (uint32_t)lane ? 0xFFFFFFFFu >> (32 - ((n - lane + 31) >> 5)) : 0u;
+  uint32_t own = 0;
+#pragma unroll
+  for (int g = 0; g < NPT; g += G) {
+    if (32u * g >= n) break;
+#pragma unroll
+    for (int u = g; u < g + G; ++u) {
+      key[u] -= lo;
+      const uint32_t c = key[u] >> shift, bit = 1u << (c & 31);
+      const uint32_t old = atomic_or_if((valid >> u) & 1u, &bits[c >> 5], bit, bit);
+      if (!(old & bit)) own |= 1u << u;
+    }
+  }
+  __syncwarp();
+  // ranks of the occupied cells, four chunks of 128 words in one scan
+  const int nwords = (int)((range >> shift) >> 5) + 1;
+  uint32_t distinct = 0;
+  for (int w0 = 0; w0 < nwords; w0 += 512) {
+    uint2 pc[4];
+    unsigned long long packed = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = (w0 >> 2) + k * 32 + lane;
+      pc[k] = make_uint2(0, 0);
+      if (i * 4 < nwords) {
+        const uint4 x = reinterpret_cast<const uint4*>(bits)[i];
+        const uint32_t a = __popc(x.x), b = a + __popc(x.y), c = b + __popc(x.z);
+        pc[k] = make_uint2(a << 16, b | (c << 16));
+        packed |= (unsigned long long)(c + __popc(x.w)) << (16 * k);
+      }
+    }
+    const unsigned long long inc = warp_inclusive_sum(packed);
+    const unsigned long long total = __shfl_sync(kFull, inc, 31), ex = inc - packed;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = (w0 >> 2) + k * 32 + lane;
+      if (i * 4 < nwords) {
+        const uint32_t b = distinct + (uint32_t)((ex >> (16 * k)) & 0xFFFFu);
+        reinterpret_cast<uint2*>(wpre)[i] = make_uint2(pc[k].x + b * 0x10001u, pc[k].y + b * 0x10001u);
+      }
+      distinct += (uint32_t)((total >> (16 * k)) & 0xFFFFu);
+    }
+  }
+  const uint32_t submask = (1u << shift) - 1u;
+  if (shift > 0) {
+    own = 0;
+    for (int i = lane; i < (int)((distinct + 3) >> 2); i += 32) reinterpret_cast<uint4*>(slot)[i] = make_uint4(0, 0, 0, 0);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int g = 0; g < NPT; g += G) {
+    if (32u * g >= n) break;
+    uint32_t q[G];
+#pragma unroll
+    for (int v = 0; v < G; ++v) {
+      const uint32_t c = key[g + v] >> shift, x = c >> 5;
+      q[v] = wpre[x] + __popc(bits[x] & ((1u << (c & 31)) - 1u));
+      if (shift > 0) {
+        const uint32_t bit = 1u << (key[g + v] & submask);
+        const uint32_t old = atomic_or_if((valid >> (g + v)) & 1u, &slot[q[v]], bit, bit);
+        if (!(old & bit)) own |= 1u << (g + v);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < G; v += 2) pos[(g + v) >> 1] |= q[v] | (q[v + 1] << 16);
+  }
+  __syncwarp();
+  if (shift > 0) {  // the distinct columns before each slot, and the places
+    const uint32_t nocc = distinct;
+    uint4 m[4];
+    unsigned long long packed = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      m[k] = make_uint4(0, 0, 0, 0);
+      if ((uint32_t)(k * 128 + lane * 4) < nocc) m[k] = reinterpret_cast<const uint4*>(slot)[k * 32 + lane];
+      packed |= (unsigned long long)(__popc(m[k].x | (m[k].y << 16)) + __popc(m[k].z | (m[k].w << 16))) << (16 * k);
+    }
+    const unsigned long long inc = warp_inclusive_sum(packed);
+    const unsigned long long total = __shfl_sync(kFull, inc, 31), ex = inc - packed;
+    distinct = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t b0 = distinct + (uint32_t)((ex >> (16 * k)) & 0xFFFFu);
+      const uint32_t b1 = b0 + __popc(m[k].x), b2 = b1 + __popc(m[k].y), b3 = b2 + __popc(m[k].z);
+      if ((uint32_t)(k * 128 + lane * 4) < nocc)
+        reinterpret_cast<uint4*>(slot)[k * 32 + lane] =
+            make_uint4(m[k].x | (b0 << 16), m[k].y | (b1 << 16), m[k].z | (b2 << 16), m[k].w | (b3 << 16));
+      distinct += (uint32_t)((total >> (16 * k)) & 0xFFFFu);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int g = 0; g < NPT; g += G) {
+      if (32u * g >= n) break;
+#pragma unroll
+      for (int u = g; u < g + G; u += 2) {
+        const uint32_t s0 = slot[pos[u >> 1] & 0x1FFu], s1 = slot[(pos[u >> 1] >> 16) & 0x1FFu];
+        const uint32_t q0 = (s0 >> 16) + __popc(s0 & ((1u << (key[u] & submask)) - 1u));
+        const uint32_t q1 = (s1 >> 16) + __popc(s1 & ((1u << (key[u + 1] & submask)) - 1u));
+        pos[u >> 1] = (pos[u >> 1] & 0xFE00FE00u) | q0 | (q1 << 16);
+      }
+    }
+    __syncwarp();
+  }
+  if ((int64_t)distinct != nz) {  // uniform
+    if (lane == 0) dev_report(st, (int64_t)distinct > nz ? kDevRowOverflow : kDevRowUnderflow, 18, r);
+    return;
+  }
+  // values: owners store, the others add
+  const VIn* __restrict__ bval = static_cast<const VIn*>(B.val);
+  auto half = [&](int u) -> uint32_t { return (u & 1) ? pos[u >> 1] >> 16 : pos[u >> 1] & 0xFFFFu; };
+  auto values = [&](uint32_t which, bool owners) {
+#pragma unroll
+    for (int g = 0; g < NPT; g += G) {
+      if (32u * g >= n) break;
+      if (!owners && !__any_sync(kFull, (which >> g) & ((1u << G) - 1u))) continue;
+      VIn bv[G];
+#pragma unroll
+      for (int v = 0; v < G; ++v)
+        bv[v] = __ldg(bval + (sg.off[half(g + v) >> 9] + min(32u * (g + v) + lane, n - 1)));
+#pragma unroll
+      for (int v = 0; v < G; ++v) {
+        const uint32_t h = half(g + v);
+        const AT x = Acc<VIn>::mul(sg.av[h >> 9], bv[v]);
+        const bool on = (which >> (g + v)) & 1u;
+        if (owners) sts_if(on, &sval[h & 0x1FFu], x);
+        else if (on) atomic_add_sh(&sval[h & 0x1FFu], x);
+      }
+    }
+  };
+  values(own, true);
+  if (distinct < n) {
+    __syncwarp();
+    values(valid & ~own, false);
+  }
+  __syncwarp();
+  for (uint32_t i = lane; i < distinct; i += 32) cval[c0 + i] = sval[i];
+  __syncwarp();
+  uint32_t* scol = bits;
+#pragma unroll
+  for (int g = 0; g < NPT; g += G) {
+    if (32u * g >= n) break;
+#pragma unroll
+    for (int u = g; u < g + G; ++u) sts_if((own >> u) & 1u, &scol[half(u) & 0x1FFu], key[u] + lo);
+  }
+  __syncwarp();
+  for (uint32_t i = lane; i < distinct; i += 32) ccol[c0 + i] = (int32_t)scol[i];
 }
 
 // Hash accumulator for rows with at most 2^TBITS / 2 distinct columns: linear

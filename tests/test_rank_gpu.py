@@ -85,6 +85,31 @@ def test_small_bins(ctx, products, ncol):
     check(ctx, A, B)
 
 
+@pytest.mark.parametrize("products", [33, 64, 127, 128, 129, 384, 511, 512, 513])
+@pytest.mark.parametrize("entries", [1, 31, 32, 33, 128, 129])
+@pytest.mark.parametrize("algo", ["hash", "hsersc"])
+def test_warp_rows(ctx, products, entries, algo):
+    """Rows at the bounds of what a warp takes: products, A entries (empty B rows among them), widths of one and two
+    levels, few and many repeats, both value types (1300 rows: enough for a warp each)."""
+    rng = np.random.default_rng(products + entries)
+    rows, ncol = 1300, [300, 14000, 16385, 262144, 262145, 2000000][(products + entries) % 6]
+    live = max(1, min(entries, products, int(rng.integers(1, entries + 1))) if products > 33 else min(entries, products))
+    live = max(live, -(-products // min(ncol, 300)))
+    entries = max(entries, live)
+    per = np.full(live, products // live)
+    per[:products % live] += 1
+    lens = np.zeros(entries, np.int64)
+    lens[rng.choice(entries, live, replace=False)] = per
+    A = from_coo(rows, entries, np.repeat(np.arange(rows), entries), np.tile(np.arange(entries), rows),
+                 rng.integers(1, 8, rows * entries), np.int32 if products % 2 else np.float64)
+    cols = np.concatenate([np.sort(rng.choice(min(ncol, 20000), n, replace=False)) for n in lens]) if products else []
+    if ncol > 20000:
+        cols = cols * (ncol // 20000)
+    B = from_coo(entries, ncol, np.repeat(np.arange(entries), lens), cols, rng.integers(1, 8, products),
+                 np.int32 if products % 2 else np.float64)
+    check(ctx, A, B, algo)
+
+
 @pytest.mark.parametrize("span", [300, 5000])
 @pytest.mark.parametrize("dtype", [np.float64, np.int32])
 def test_crowded_columns(ctx, span, dtype):
