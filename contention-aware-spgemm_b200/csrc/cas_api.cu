@@ -210,8 +210,7 @@ cas_status allow_smem(cas_ctx* ctx, K kernel, size_t bytes) {
 // ------------------------------------------------ kernel shapes and memory
 template <int BLOCK, int TBITS, int SEGCAP>
 constexpr size_t smem_symb_hash() { return (size_t(1) << TBITS) * 4 + SEGCAP + sizeof(cas::StageB<double>); }
-template <int BLOCK>
-constexpr size_t smem_symb_dense() { return size_t(cas::kDenseChunkBits / 32) * 4 + sizeof(cas::Stage<double>); }
+constexpr size_t smem_symb_dense(int words) { return size_t(words) * 4 + sizeof(cas::Stage<double>); }
 template <int BLOCK, int CAP, typename VIn>
 constexpr size_t smem_numc_esc() {
   return size_t(CAP) * 16 + size_t(CAP) * sizeof(typename cas::Acc<VIn>::T) + sizeof(cas::SortScratch<BLOCK>) +
@@ -222,12 +221,6 @@ constexpr size_t smem_numc_hash() {
   return (size_t(1) << TBITS) * (4 + sizeof(typename cas::Acc<VIn>::T)) + (size_t(1) << (TBITS - 1)) * 8 +
          sizeof(cas::SortScratch<BLOCK>) + sizeof(cas::Stage<VIn>);
 }
-// Bitmap words of the widest slice of a matrix of ncol columns.
-int dense_words(int64_t ncol) {
-  const int64_t cols = std::min<int64_t>(std::max<int64_t>(ncol, 1), cas::kRankCols);
-  return (int)((cols + 255) / 256) * 8;
-}
-
 template <int CAP, int NBB, typename VIn>
 constexpr size_t smem_numc_esc_msd() {
   return size_t(CAP) * (sizeof(typename cas::Acc<VIn>::T) + 4) + (size_t(1) << NBB) * 2 + size_t(CAP / 32) * 4 +
@@ -239,6 +232,12 @@ template <int CAP, int NBB, typename VIn>
 constexpr size_t smem_numc_esc_idx() {
   return size_t(CAP) * 8 + (size_t(1) << NBB) * 2 + size_t((CAP / 32 + 3) & ~3) * 8 +
          ((size_t(CAP) + 15) & ~size_t(15)) + sizeof(cas::StageB<VIn>);
+}
+
+// Bitmap words of the widest slice of a matrix of ncol columns.
+int dense_words(int64_t ncol) {
+  const int64_t cols = std::min<int64_t>(std::max<int64_t>(ncol, 1), cas::kRankCols);
+  return (int)((cols + 255) / 256) * 8;
 }
 
 // symbolic hash shape of each symbolic bin: threads, log2(table slots), byte
@@ -322,8 +321,10 @@ cas_status setup_kernels(cas_ctx* ctx) {
   CAS_SYMB_SHAPES(CAS_SETUP_SYMB)
 #undef CAS_SETUP_SYMB
   CAS_TRY(allow_smem(ctx, k_symb_warp<10>, kWarpsPerBlock * sizeof(SymbWarp<10>)));
-  CAS_TRY(allow_smem(ctx, k_symb_dense<512>, smem_symb_dense<512>()));
-  CAS_TRY(allow_smem(ctx, k_heavy_bits<512>, smem_symb_dense<512>()));
+  CAS_TRY(allow_smem(ctx, k_symb_dense<128>, smem_symb_dense(kRankCols / 32)));
+  CAS_TRY(allow_smem(ctx, k_symb_dense<256>, smem_symb_dense(kRankCols / 32)));
+  CAS_TRY(allow_smem(ctx, k_symb_dense<512>, smem_symb_dense(kRankCols / 32)));
+  CAS_TRY(allow_smem(ctx, k_heavy_bits<512>, smem_symb_dense(kRankCols / 32)));
   CAS_TRY(setup_numc_kernels<double>(ctx));
   CAS_TRY(setup_numc_kernels<int32_t>(ctx));
   return CAS_OK;
@@ -1064,8 +1065,9 @@ cas_status symb_split_heavy(cas_ctx* ctx, Call& c, int32_t*& rows, int64_t& n, i
   k_scan_one_block<<<1, 1024, 0, s>>>(hp.nparts, nh, hp.parts);
   CAS_TRY(check_launch(ctx, "k_scan_one_block"));
   int per_sm = 0;
-  CAS_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_heavy_bits<512>, 512, smem_symb_dense<512>()));
-  k_heavy_bits<512><<<std::max(1, per_sm) * ctx->sm_count, 512, smem_symb_dense<512>(), s>>>(hp, c.A.csr, c.B.csr,
+  const int words = dense_words(c.ncol);
+  CAS_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_heavy_bits<512>, 512, smem_symb_dense(words)));
+  k_heavy_bits<512><<<std::max(1, per_sm) * ctx->sm_count, 512, smem_symb_dense(words), s>>>(hp, c.A.csr, c.B.csr, words,
                                                                                              ctx->d_status);
   CAS_TRY(check_launch(ctx, "k_heavy_bits"));
   k_heavy_count<512><<<(unsigned)nh, 512, 0, s>>>(hp, row_nz);
@@ -1080,6 +1082,7 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
   CAS_TRY(fork(ctx));
   int64_t off[kSymbBins + 1] = {0};
   for (int b = 0; b < kSymbBins; ++b) off[b + 1] = off[b] + c.symb_count[b];
+  const int words = dense_words(c.ncol);
   // heaviest bins first, each on its own stream
   const int order[] = {kSB_Dense, kSB_H32K, kSB_H16K, kSB_H8K, kSB_H4K, kSB_H2K, kSB_H1K, kSB_Tiny};
   int si = 0;
@@ -1102,6 +1105,12 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
                 rows, n, c.A.csr, c.B.csr, row_nz, ctx->d_status);                                  \
             break;                                                                                  \
           }                                                                                         \
+        }                                                                                           \
+        if (words <= (1 << TB) && c.ncol <= kDenseChunkBits) {                                          \
+          k_symb_dense<BLK><<<(unsigned)n, BLK, smem_symb_dense(words), s>>>(                       \
+              rows, c.A.csr, c.B.csr, c.ncol, c.b_sorted ? 1 : 0, words, row_nz, nullptr, nullptr, 0, \
+              ctx->d_status);                                                                       \
+          break;                                                                                    \
         }                                                                                           \
         k_symb_hash<BLK, TB, SEG><<<(unsigned)n, BLK, smem_symb_hash<BLK, TB, SEG>(), s>>>(          \
             rows, c.A.csr, c.B.csr, row_nz, ctx->d_status);                                         \
@@ -1128,9 +1137,9 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
           CAS_CUDA(ctx, cudaMemsetAsync(c.dslot, 0xFF, sizeof(int32_t) * (c.m + 1), ctx->stream));
           CAS_TRY(scratch_ready(ctx, s));
         }
-        k_symb_dense<512><<<(unsigned)nd, 512, smem_symb_dense<512>(), s>>>(drows, c.A.csr, c.B.csr, c.ncol,
-                                                                             c.b_sorted ? 1 : 0, row_nz, c.dbits,
-                                                                             c.dslot, c.saved_slices, ctx->d_status);
+        k_symb_dense<512><<<(unsigned)nd, 512, smem_symb_dense(words), s>>>(drows, c.A.csr, c.B.csr, c.ncol,
+                                                                            c.b_sorted ? 1 : 0, words, row_nz, c.dbits,
+                                                                            c.dslot, c.saved_slices, ctx->d_status);
         break;
       }
     }

@@ -683,19 +683,23 @@ __device__ __forceinline__ void row_col_range(const Csr& A, const Csr& B, int64_
   __syncthreads();
 }
 
-// Heavy rows: a bitmap over kDenseChunkBits columns at a time, one pass per
+// Heavy rows, and the rows whose hash table would be no smaller than the
+// matrix's bitmap: a bitmap over kDenseChunkBits columns at a time (`words`
+// words of it, the matrix's widest slice; a bit set costs one shared-memory
+// atomic, a hash insertion a compare-and-swap or more: 9,858 rows of 8193 to
+// 16384 products over 1.3e5 columns 0.77 -> 0.25 ms, 19,313 of about 5400 over
+// 5.2e5 0.61 -> 0.53), one pass per
 // chunk of the row's column range; the count is the population count.  B
 // rows are cut to each column chunk by binary search when there is more than
 // one chunk.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
-k_symb_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted,
+k_symb_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, int words,
              int64_t* __restrict__ row_nz, uint32_t* __restrict__ saved, int32_t* __restrict__ saved_slot,
              int saved_slices, DevStatus* st) {
-  constexpr int W = kDenseChunkBits / 32;
   extern __shared__ __align__(16) uint8_t smem[];
   uint32_t* bm = reinterpret_cast<uint32_t*>(smem);
-  Stage<double>& sg = *reinterpret_cast<Stage<double>*>(smem + W * sizeof(uint32_t));
+  Stage<double>& sg = *reinterpret_cast<Stage<double>*>(smem + words * sizeof(uint32_t));
   const int64_t r = rows[blockIdx.x];
   int64_t lo, hi;
   row_col_range<BLOCK>(A, B, r, b_sorted != 0, c_ncol, lo, hi);
@@ -710,7 +714,7 @@ k_symb_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
     expand_row<BLOCK, false, double>(A, B, r, sg, multi, (int32_t)c0, (int32_t)c1,
                                      [&](int32_t key, double, double, int64_t) {
       const uint32_t idx = (uint32_t)key - (uint32_t)c0;
-      if (idx >= kDenseChunkBits) { bad = true; return; }
+      if (idx >= (uint32_t)(c1 - c0)) { bad = true; return; }
       atomicOr(&bm[idx >> 5], 1u << (idx & 31));
     });
     if (bad && !multi) dev_report(st, kDevBadIndex, 3, r);
@@ -3582,11 +3586,11 @@ k_heavy_plan(HeavyPlan hp, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, DevSt
 }
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
-k_heavy_bits(HeavyPlan hp, Csr A, Csr B, DevStatus* st) {
-  constexpr int NWORD = kRankCols / 32;
+k_heavy_bits(HeavyPlan hp, Csr A, Csr B, int words, DevStatus* st) {
+  constexpr int NWORD = kRankCols / 32;  // of a slice kept in memory
   extern __shared__ __align__(16) uint8_t smem[];
   uint32_t* bm = reinterpret_cast<uint32_t*>(smem);
-  Stage<double>& sg = *reinterpret_cast<Stage<double>*>(smem + NWORD * sizeof(uint32_t));
+  Stage<double>& sg = *reinterpret_cast<Stage<double>*>(smem + words * sizeof(uint32_t));
   __shared__ long long s_t, s_i;
   const int64_t total = hp.parts[hp.n];
   for (;;) {

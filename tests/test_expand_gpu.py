@@ -59,3 +59,22 @@ def test_dense_row_columns_leave_in_tiles(ctx, ncol, nnz):
     np.testing.assert_array_equal(out.csr.row_ptrs, rp)
     np.testing.assert_array_equal(out.csr.cols.astype(np.int64), cols)
     np.testing.assert_array_equal(out.csr.vals.astype(np.float64), vals)
+
+
+@pytest.mark.parametrize("ncol", [40, 4096, 32768, 32769, 131072, 131073, 524288, 524289])
+@pytest.mark.parametrize("products", [700, 1500, 3000, 6000, 12000, 17000])
+def test_symbolic_counts_by_bitmap_and_hash(ctx, ncol, products):
+    """Every symbolic bin at the widths where its rows go by bitmap and by hash."""
+    rng = np.random.default_rng(ncol + products)
+    rows, per = 40, min(ncol, 97)
+    entries = -(-products // per)
+    A = from_coo(rows, entries + 5, np.repeat(np.arange(rows), entries),
+                 np.concatenate([rng.choice(entries + 5, entries, replace=False) for _ in range(rows)]))
+    cols = np.concatenate([np.sort(rng.choice(ncol, per, replace=False)) for _ in range(entries + 5)])
+    B = from_coo(entries + 5, ncol, np.repeat(np.arange(entries + 5), per), cols)
+    for algo in ("hash", "hybacc"):
+        out = ctx.spgemm(A, B, algo)
+        rp, c, v, _ = oracle.oracle_spgemm(A, B, algo)
+        np.testing.assert_array_equal(out.csr.row_ptrs, rp)
+        np.testing.assert_array_equal(out.csr.cols.astype(np.int64), c)
+        np.testing.assert_array_equal(out.csr.vals.astype(np.float64), v)
