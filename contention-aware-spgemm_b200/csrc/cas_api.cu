@@ -86,6 +86,9 @@ struct cas_ctx {
   int hash_max = 4096;                     // hash rows: at most this many distinct columns
   int out_blocks = 0;                      // C in host memory: row blocks (0: by C's size)
   cudaMemPool_t scratch = nullptr;         // the device's scratch pool (scratch_pool_get)
+  char* ws = nullptr;                      // workspace that products take their scratch from (ws_alloc):
+  size_t ws_cap = 0, ws_used = 0;          // its bytes, and those the current product has taken
+  size_t ws_need = 0;                      // what the current product has asked for
   double mem_share = 1.0;                  // share of the free device memory this context sizes
                                            // its optional scratch by (a batch worker's: 1 / workers)
   double acc_thres = 2.0;
@@ -366,6 +369,8 @@ constexpr int kMaxDevices = 64;
 struct ScratchPool {
   cudaMemPool_t pool = nullptr;
   int users = 0;
+  size_t total = 0;    // bytes of the device's memory
+  size_t ws_bytes = 0; // of the contexts' workspaces
 };
 std::mutex g_scratch_mu;
 ScratchPool g_scratch[kMaxDevices];
@@ -378,6 +383,7 @@ cas_status scratch_pool_get(cas_ctx* ctx) {
   if (!sp.pool) {
     size_t free_b = 0, total_b = 0;
     CAS_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
+    sp.total = total_b;
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -409,8 +415,8 @@ void scratch_pool_put(cas_ctx* ctx) {
 }
 
 // Device memory a stream-ordered allocation can still get: the device's free
-// memory plus what the pools hold reserved but unused (freed allocations they
-// keep).  cudaMemGetInfo alone would count the pools' idle reserve as taken, so
+// memory, what the pools hold reserved but unused (freed allocations they
+// keep), and the rest of the context's workspace.  cudaMemGetInfo alone would count the pools' idle reserve as taken, so
 // sizes chosen from it would shrink after every large product.
 double free_device_bytes(cas_ctx* ctx) {
   size_t free_b = 0, total_b = 0;
@@ -418,7 +424,7 @@ double free_device_bytes(cas_ctx* ctx) {
     cudaGetLastError();
     return 0.0;
   }
-  double idle = 0.0;
+  double idle = (double)(ctx->ws_cap - ctx->ws_used);
   cudaMemPool_t pools[2] = {nullptr, ctx->scratch};
   if (cudaDeviceGetDefaultMemPool(&pools[0], ctx->device) != cudaSuccess) pools[0] = nullptr;
   for (cudaMemPool_t pool : pools) {
@@ -465,6 +471,56 @@ cas_status scratch_ready(cas_ctx* ctx, cudaStream_t s) {
   if (s == ctx->stream) return CAS_OK;
   CAS_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
   CAS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_fork, 0));
+  return CAS_OK;
+}
+
+// A product's scratch comes from a workspace that its context keeps: from the
+// second product of a size on, no call of the allocator is left in it (the
+// pool, for all its order, now and then mapped the largest blocks anew: 1 to 60
+// ms beside a 10 ms product).  What does not fit is allocated, and the
+// workspace grows to the product's need before the next one starts, while the
+// contexts of a device together keep at most kWorkspaceKeep of its memory.
+// Only one product at a time uses it, on the context's stream and the
+// auxiliary streams that join it.
+constexpr double kWorkspaceKeep = 1.0 / 16;
+void ws_drop(cas_ctx* ctx) {
+  if (!ctx->ws) return;
+  cudaFreeAsync(ctx->ws, ctx->stream);
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  g_scratch[ctx->device].ws_bytes -= ctx->ws_cap;
+  ctx->ws = nullptr;
+  ctx->ws_cap = ctx->ws_used = 0;
+}
+void ws_begin(cas_ctx* ctx) {
+  const size_t need = (ctx->ws_need + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
+  ctx->ws_used = ctx->ws_need = 0;
+  if (need <= ctx->ws_cap) return;
+  ws_drop(ctx);
+  {
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    ScratchPool& sp = g_scratch[ctx->device];
+    if ((double)(sp.ws_bytes + need) > kWorkspaceKeep * (double)sp.total) return;
+    sp.ws_bytes += need;
+  }
+  ctx->ws_cap = need;
+  if (pool_alloc(ctx, ctx->scratch, (void**)&ctx->ws, need, ctx->stream) != cudaSuccess) {
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    g_scratch[ctx->device].ws_bytes -= need;
+    ctx->ws = nullptr;
+    ctx->ws_cap = 0;
+  }
+}
+// `spill` gets what was allocated, to be freed after the product.
+cas_status ws_alloc(cas_ctx* ctx, std::vector<void*>& spill, void** p, size_t bytes) {
+  bytes = (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
+  ctx->ws_need += bytes;
+  if (ctx->ws_used + bytes <= ctx->ws_cap) {
+    *p = ctx->ws + ctx->ws_used;
+    ctx->ws_used += bytes;
+    return CAS_OK;
+  }
+  CAS_TRY(dev_alloc(ctx, p, bytes));
+  spill.push_back(*p);
   return CAS_OK;
 }
 
@@ -791,7 +847,7 @@ struct Call {
   // in them (-1 for other rows); kept for the numeric setup of split rows
   uint32_t* hbits = nullptr;
   int32_t* hslot = nullptr;
-  std::vector<void*> heavy_tmp;  // the rest of the symbolic split's scratch
+  std::vector<void*> spill;  // scratch that the context's workspace had no room for
 };
 
 cas_status fork(cas_ctx* ctx) {
@@ -820,7 +876,7 @@ cas_status scratch_alloc(cas_ctx* ctx, Call& c) {
   const size_t rows4 = (sizeof(int32_t) * (size_t)(c.m + 1) + 255) & ~size_t(255);
   c.nparts = (c.m + 1 + cas::kScanTile - 1) / cas::kScanTile;
   char* p = nullptr;
-  CAS_TRY(dev_alloc(ctx, (void**)&p, 2 * rows8 + 2 * rows4 + sizeof(int64_t) * (size_t)(c.nparts + 1)));
+  CAS_TRY(ws_alloc(ctx, c.spill, (void**)&p, 2 * rows8 + 2 * rows4 + sizeof(int64_t) * (size_t)(c.nparts + 1)));
   c.row_flp = reinterpret_cast<int64_t*>(p);
   c.row_nz = reinterpret_cast<int64_t*>(p + rows8);
   c.rows = reinterpret_cast<int32_t*>(p + 2 * rows8);
@@ -830,9 +886,8 @@ cas_status scratch_alloc(cas_ctx* ctx, Call& c) {
 }
 
 cas_status scratch_free(cas_ctx* ctx, Call& c) {
-  void* ps[] = {c.row_flp, c.frows, c.fpos, c.fstatus, c.dbits, c.dslot};
-  for (void* p : ps)
-    if (p) CAS_CUDA(ctx, cudaFreeAsync(p, ctx->stream));
+  for (void* p : c.spill) CAS_CUDA(ctx, cudaFreeAsync(p, ctx->stream));
+  c.spill.clear();
   c.row_flp = c.row_nz = nullptr;
   c.rows = c.ovf = nullptr;
   c.partial = nullptr;
@@ -841,8 +896,6 @@ cas_status scratch_free(cas_ctx* ctx, Call& c) {
   c.fstatus = nullptr;
   c.dbits = nullptr;
   c.dslot = nullptr;
-  for (void* p : c.heavy_tmp) CAS_CUDA(ctx, cudaFreeAsync(p, ctx->stream));
-  c.heavy_tmp.clear();
   c.hbits = nullptr;
   c.hslot = nullptr;
   return CAS_OK;
@@ -929,6 +982,7 @@ cas_status check_inputs(cas_ctx* ctx, Call& c) {
 cas_status phase_init(cas_ctx* ctx, Call& c, bool validate) {
   using namespace cas;
   CAS_TRY(clear_counts(ctx));
+  ws_begin(ctx);
   CAS_TRY(scratch_alloc(ctx, c));
   const Csr &a = c.A.csr, &b = c.B.csr;
   const bool a_is_b = a.rp == b.rp && a.col == b.col && a.nrow == b.nrow && a.ncol == b.ncol && c.A.nnz == c.B.nnz;
@@ -952,9 +1006,9 @@ cas_status phase_init(cas_ctx* ctx, Call& c, bool validate) {
   if (c.nf > 0) {
     // the fused rows in ascending order: marks (in row_nz, cleared before the
     // symbolic kernels), their scan, the scatter
-    CAS_TRY(dev_alloc(ctx, (void**)&c.fpos, sizeof(int64_t) * (c.m + 1)));
-    CAS_TRY(dev_alloc(ctx, (void**)&c.frows, sizeof(int32_t) * c.nf));
-    CAS_TRY(dev_alloc(ctx, (void**)&c.fstatus, sizeof(unsigned long long) * c.nf));
+    CAS_TRY(ws_alloc(ctx, c.spill, (void**)&c.fpos, sizeof(int64_t) * (c.m + 1)));
+    CAS_TRY(ws_alloc(ctx, c.spill, (void**)&c.frows, sizeof(int32_t) * c.nf));
+    CAS_TRY(ws_alloc(ctx, c.spill, (void**)&c.fstatus, sizeof(unsigned long long) * c.nf));
     const int g = grid_for(c.m, 256, ctx->sm_count * 8);
     k_fused_mark<<<g, 256, 0, ctx->stream>>>(c.m, c.row_flp, c.fuse, c.row_nz);
     CAS_TRY(check_launch(ctx, "k_fused_mark"));
@@ -1019,11 +1073,7 @@ cas_status symb_split_heavy(cas_ctx* ctx, Call& c, int32_t*& rows, int64_t& n, i
   using namespace cas;
   const int64_t max_slices = (c.ncol + kRankCols - 1) / kRankCols;
   const int64_t cap = (int64_t)((double)kSplitScratch * ctx->mem_share) / (max_slices * (kRankCols / 8));
-  auto alloc = [&](void** p, size_t bytes) -> cas_status {
-    CAS_TRY(dev_alloc(ctx, p, bytes));
-    c.heavy_tmp.push_back(*p);
-    return CAS_OK;
-  };
+  auto alloc = [&](void** p, size_t bytes) { return ws_alloc(ctx, c.spill, p, bytes); };
   int32_t *heavy = nullptr, *light = nullptr;
   unsigned long long* counts = nullptr;
   CAS_TRY(alloc((void**)&c.hslot, sizeof(int32_t) * (size_t)(c.m + 1)));
@@ -1132,8 +1182,8 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
         const int64_t max_slices = (c.ncol + kRankCols - 1) / kRankCols;
         c.saved_slices = (double)nd * max_slices * (kRankCols / 8) <= cap ? (int)max_slices : 1;
         if ((double)nd * c.saved_slices * (kRankCols / 8) <= cap) {
-          CAS_TRY(dev_alloc(ctx, (void**)&c.dbits, (size_t)nd * c.saved_slices * (kRankCols / 8)));
-          CAS_TRY(dev_alloc(ctx, (void**)&c.dslot, sizeof(int32_t) * (c.m + 1)));
+          CAS_TRY(ws_alloc(ctx, c.spill, (void**)&c.dbits, (size_t)nd * c.saved_slices * (kRankCols / 8)));
+          CAS_TRY(ws_alloc(ctx, c.spill, (void**)&c.dslot, sizeof(int32_t) * (c.m + 1)));
           CAS_CUDA(ctx, cudaMemsetAsync(c.dslot, 0xFF, sizeof(int32_t) * (c.m + 1), ctx->stream));
           CAS_TRY(scratch_ready(ctx, s));
         }
@@ -1221,11 +1271,7 @@ cas_status launch_heavy_split(cas_ctx* ctx, Call& c, const int32_t* rows, int64_
   hp.rows = rows;
   hp.n = n;
   hp.max_slices = (int)((c.ncol + kRankCols - 1) / kRankCols);
-  auto alloc = [&](void** p, size_t bytes) -> cas_status {
-    CAS_TRY(dev_alloc(ctx, p, bytes));
-    c.heavy_tmp.push_back(*p);
-    return CAS_OK;
-  };
+  auto alloc = [&](void** p, size_t bytes) { return ws_alloc(ctx, c.spill, p, bytes); };
   CAS_TRY(alloc((void**)&hp.bits, (size_t)n * hp.max_slices * (kRankCols / 8)));
   CAS_TRY(alloc((void**)&hp.slice_base, sizeof(int64_t) * (size_t)n * hp.max_slices));
   CAS_TRY(alloc((void**)&hp.lo, sizeof(int64_t) * (size_t)n));
@@ -1474,6 +1520,21 @@ cas_status compute_dev(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, De
   return CAS_OK;
 }
 
+// compute_dev, once more without the workspace when memory runs out beside it.
+template <typename F>
+cas_status compute(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, DevC& o, F&& at_cap) {
+  cas_status st = compute_dev(ctx, accum, c, validate, o, at_cap);
+  if (st == CAS_ERR_OOM && ctx->ws) {
+    quiesce(ctx);
+    CAS_TRY(scratch_free(ctx, c));
+    free_dev_c(o, ctx->stream);
+    ws_drop(ctx);
+    ctx->ws_need = 0;
+    st = compute_dev(ctx, accum, c, validate, o, at_cap);
+  }
+  return st;
+}
+
 // The counters of one product just computed (its phases' events and counts
 // are still in the context); kernel launches and copied bytes are the
 // caller's.
@@ -1665,7 +1726,7 @@ cas_status run_blocked(cas_ctx* ctx, cas_accum accum, const cas_csr* A, Call& fu
     ck.fuse = full.fuse;
     ck.b_sorted = full.b_sorted;
     DevC o;
-    st = compute_dev(ctx, accum, ck, false, o, [](int64_t) { return CAS_OK; });
+    st = compute(ctx, accum, ck, false, o, [](int64_t) { return CAS_OK; });
     if (st == CAS_OK && o.nnz > bound - base)
       st = set_err(ctx, CAS_ERR_DEVICE, "row block %d: %lld entries past the output bound", k,
                    (long long)(base + o.nnz - bound));
@@ -1803,9 +1864,12 @@ cas_status run_spgemm(cas_ctx* ctx, cas_accum accum, const cas_csr* A, const cas
     host_give(ctx, h_rp);
     host_give(ctx, h_col);
     host_give(ctx, h_val);
+    h_rp = nullptr;
+    h_col = h_val = nullptr;
   };
-  cas_status st = compute_dev(ctx, accum, c, !checked, o, [&](int64_t cap) -> cas_status {
+  cas_status st = compute(ctx, accum, c, !checked, o, [&](int64_t cap) -> cas_status {
     if (c_on_device) return CAS_OK;
+    free_host();  // of a first try
     h_rp = static_cast<int64_t*>(host_take(ctx, sizeof(int64_t) * (c.m + 1)));
     h_col = host_take(ctx, (size_t)c_col_bytes * (size_t)(cap > 0 ? cap : 1));
     h_val = host_take(ctx, vbytes * (size_t)(cap > 0 ? cap : 1));
@@ -1962,6 +2026,8 @@ void cas_destroy(cas_ctx* ctx) {
     for (auto& b : ctx->host_blocks) g_host_owner.erase(b.first);
     for (auto& b : ctx->host_free) free(b.first);
   }
+  ctx->stream = ctx->own_stream;
+  ws_drop(ctx);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   scratch_pool_put(ctx);
   delete ctx;
