@@ -1326,6 +1326,16 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
   unsigned int* ovf_count = reinterpret_cast<unsigned int*>(ctx->d_counts + kSlotOvf);
   CAS_TRY(fork(ctx));
   const bool rank = rank_form(ctx, c.ncol);
+  // The dense kernel also takes the larger hash rows where the matrix's bitmap
+  // has no more words than their table slots: it neither probes nor sorts
+  // (14,591 rows of at most 4096 columns and 7,000 products, over 1e5 columns:
+  // 3.52 ms by hash, 1.5 here).
+  const int words = dense_words(c.ncol);
+  auto launch_dense = [&](const int32_t* drows, int64_t n, cudaStream_t s) {
+    k_numc_dense<512, VIn><<<(unsigned)n, 512, DenseSmem<VIn>::bytes(words), s>>>(
+        drows, c.A.csr, c.B.csr, c.ncol, c.b_sorted ? 1 : 0, words, crp, ccol, cval, c.dbits, c.dslot, c.saved_slices,
+        ctx->d_status);
+  };
   // The warps' rows lead their two bins.  Wider than 2^kWarpBits columns a
   // warp's bitmap is much for it to clear and scan, and leaves fewer warps on an
   // SM: 192,500 join rows over 6e5 columns take 1.33 ms by warps and 0.97 by
@@ -1376,10 +1386,12 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
         k_numc_hash<256, 9, VIn><<<(unsigned)n, 256, smem_numc_hash<256, 9, VIn>(), s>>>(rows, A, B, crp, ccol, cval, ctx->d_status);
         break;
       case kNB_H1K:
-        k_numc_hash<256, 11, VIn><<<(unsigned)n, 256, smem_numc_hash<256, 11, VIn>(), s>>>(rows, A, B, crp, ccol, cval, ctx->d_status);
+        if (words <= (1 << 11)) launch_dense(rows, n, s);
+        else k_numc_hash<256, 11, VIn><<<(unsigned)n, 256, smem_numc_hash<256, 11, VIn>(), s>>>(rows, A, B, crp, ccol, cval, ctx->d_status);
         break;
       case kNB_H4K:
-        k_numc_hash<512, 13, VIn><<<(unsigned)n, 512, smem_numc_hash<512, 13, VIn>(), s>>>(rows, A, B, crp, ccol, cval, ctx->d_status);
+        if (words <= (1 << 13)) launch_dense(rows, n, s);
+        else k_numc_hash<512, 13, VIn><<<(unsigned)n, 512, smem_numc_hash<512, 13, VIn>(), s>>>(rows, A, B, crp, ccol, cval, ctx->d_status);
         break;
       case kNB_Dense: {
         if (!c.b_sorted && c.ncol > kRankCols)
@@ -1395,12 +1407,7 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
         if (!ctx->heavy_split) n_split = 0;
         ctx->stats.split_rows = n_split;
         if (n_split > 0) CAS_TRY(launch_heavy_split<VIn>(ctx, c, rows, n_split, crp, ccol, cval, s));
-        if (n > n_split) {
-          const int words = dense_words(c.ncol);
-          k_numc_dense<512, VIn><<<(unsigned)(n - n_split), 512, DenseSmem<VIn>::bytes(words), s>>>(
-              rows + n_split, A, B, c.ncol, c.b_sorted ? 1 : 0, words, crp, ccol, cval, c.dbits, c.dslot,
-              c.saved_slices, ctx->d_status);
-        }
+        if (n > n_split) launch_dense(rows + n_split, n - n_split, s);
         break;
       }
     }
