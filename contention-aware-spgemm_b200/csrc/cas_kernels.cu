@@ -3148,13 +3148,18 @@ __device__ __forceinline__ long long slice_ranks(const uint32_t* __restrict__ bm
   for (int g0 = 0; g0 < ng; g0 += BLOCK) {
     const int g = g0 + threadIdx.x;
     int cnt = 0;
-    if (g < ng) {
+    if (g < ng) {  // 8 words in two loads: one by one, lanes 8 words apart met in the same banks
+      const uint4 lo = reinterpret_cast<const uint4*>(bm)[g * 2], hi = reinterpret_cast<const uint4*>(bm)[g * 2 + 1];
+      const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      uint32_t before[2] = {0u, 0u};
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int w = g * 8 + k;
-        wrank[w] = (uint8_t)cnt;
-        cnt += w < nw ? __popc(bm[w]) : 0;
+        before[k >> 2] |= (uint32_t)cnt << (8 * (k & 3));
+        cnt += g * 8 + k < nw ? __popc(v[k]) : 0;
       }
+      uint32_t* out = reinterpret_cast<uint32_t*>(wrank + g * 8);
+      out[0] = before[0];
+      out[1] = before[1];
     }
     long long tot;
     const long long ex = block_exclusive_sum<BLOCK, long long>((long long)cnt, tmp, tot);
