@@ -640,12 +640,20 @@ def main():
     dom_ms = bin_ms[dom]
     dom_bytes = bin_bytes[dom]
     achieved = dom_bytes / (dom_ms * 1e-3) / 1e9 if dom_ms > 0 else 0.0
-    kernel_name = {"tiny": "k_numc_tiny<256>", "hash256": "k_numc_hash<256,9>", "hash1k": "k_numc_hash<256,11>",
-                   "hash4k": "k_numc_hash<512,13>", "dense": "k_numc_dense<512>"}.get(dom)
-    # the index form runs the fused rows and the ESC bins over 4096 products when esc_form is 1
+    ncol = B.num_col
+    kernel_name = {"tiny": "k_numc_tiny<256>", "hash256": "k_numc_hash<256,9>",
+                   "hash1k": "k_numc_dense<512>" if ncol <= 1 << 16 else "k_numc_hash<256,11>",
+                   "hash4k": "k_numc_dense<512>" if ncol <= 1 << 18 else "k_numc_hash<512,13>",
+                   "dense": "k_numc_dense<512>"}.get(dom)
+    # the index form runs the fused rows and the ESC bins over 4096 products when esc_form is 1;
+    # the ranked bitmap runs them all when it is 2 and C has at most 2^21 columns
     form = ctx.get_tuning().get("esc_form", 1)
     idx_form = form >= 1
-    if dom == "fused":
+    rank_shape = {"fused": "256,4,5120,fused", "esc1k": "128,12,1024", "esc2k": "256,6,2048", "esc3k": "256,4,5120",
+                  "esc4k": "256,4,5120", "esc5k": "256,4,5120", "esc6k": "256,3,6144", "esc8k": "256,2,8192"}
+    if form == 2 and ncol <= 1 << 21 and dom in rank_shape:
+        kernel_name = "k_numc_rank<%s>" % rank_shape[dom]
+    elif dom == "fused":
         kernel_name = "k_numc_esc_%s<256,5120,11,fused%s>" % ("idx" if idx_form else "msd",
                                                             ",keys in registers" if form == 2 else "")
     if kernel_name is None and dom.startswith("esc"):

@@ -900,14 +900,6 @@ __device__ __forceinline__ void esc_radix_row(int64_t r, const Csr& A, const Csr
   if (threadIdx.x == 0 && carry != nz) dev_report(st, carry > nz ? kDevRowOverflow : kDevRowUnderflow, 11, r);
 }
 
-template <int BLOCK, int CAP, typename VIn>
-__global__ void __launch_bounds__(BLOCK)
-k_numc_esc(const int32_t* __restrict__ rows, Csr A, Csr B, const int64_t* __restrict__ crp,
-           int32_t* __restrict__ ccol, typename Acc<VIn>::T* __restrict__ cval, DevStatus* st) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  esc_radix_row<BLOCK, CAP, VIn>(rows[blockIdx.x], A, B, crp, ccol, cval, st, smem);
-}
-
 // Persistent form for the rows the bucketed ESC kernel hands back (their
 // keys fall unevenly into its buckets): the list length is read on the device.
 template <int BLOCK, int CAP, typename VIn>

@@ -26,6 +26,9 @@ namespace cas {
 // Symbolic bins by t = min(row_flp, num_col) (an upper bound on the row's
 // distinct columns); numeric bins by accumulator and size.
 // Hash tables hold at least twice the bound, so the load factor stays <= 1/2.
+// The bins say how much a row can hold; where there are enough rows a warp takes
+// each H1K, E1K and H256 row, and where the matrix's bitmap is no larger than the
+// table, H* rows take the bitmap kernels (the rules stand at the launches).
 enum SymbBin : int {
   kSB_Zero = 0,    // row_flp == 0
   kSB_Tiny = 1,    // row_flp <= 32: one warp, one product per lane
@@ -39,7 +42,7 @@ enum SymbBin : int {
   kSymbBins = 9
 };
 
-// ESC bins by products (bucketed ESC, 256 threads; capacity = the bound);
+// ESC bins by products (capacity = the bound; ranked bitmap or bucketed ESC);
 // hash bins by nnz of the row.
 enum NumcBin : int {
   kNB_Zero = 0,    // no products
@@ -61,7 +64,7 @@ enum NumcBin : int {
 enum AccumMode : int { kAccHash = 0, kAccEsc = 1, kAccHybrid = 2 };
 
 constexpr int kDenseChunkBits = 1 << 19;   // symbolic bitmap slice: 512 Ki columns (64 KiB)
-constexpr int kRankCols = 1 << 19;         // numeric dense slice: 512 Ki columns (64 + 32 + 8 KiB of bitmap and ranks)
+constexpr int kRankCols = 1 << 19;         // numeric dense slice: 512 Ki columns (64 + 16 + 8 KiB of bitmap and ranks)
 static_assert(kRankCols == kDenseChunkBits, "the symbolic and numeric slices coincide, so bitmaps carry over");
 
 struct Csr {
