@@ -456,14 +456,24 @@ k_scan_apply(const int64_t* __restrict__ in, int64_t n_in, const int64_t* __rest
 // products, and a product's entry is the running entry plus the marks up to
 // its lane.  So no product searches for its entry, the B rows' lengths do not
 // matter, and a warp's loads are consecutive.  Loads of four groups of 32 are
-// issued before any is consumed.  With `ranged`, every B row is cut to the
-// columns [c0, c1) by binary search (B rows sorted); otherwise f receives every
-// product.  (Finding each product's entry from an interpolated guess, checked
+// issued before any is consumed.  `cut` (cut_of) says whether B rows reach below
+// c0 or past c1 and are cut there by binary search (B rows sorted); otherwise f
+// receives every product.  A row of one chunk that is walked slice by slice
+// starts each slice where the last one ended (`next`, the thread's own): each
+// search is a chain of some 15 loads, and searching both ends of every slice
+// took most of the symbolic phase of a join matrix of 850000 rows, two slices
+// wide (28.0 ms, 17.4 now; the product of one of 600000 rows 26.8 and 25.5).
+// (Finding each product's entry from an interpolated guess, checked
 // and repaired by binary search, took 125 to 170 instructions per 32 products
 // in the dense kernels and bound them, issue slots 80% busy; the symbolic
 // dense kernels of Graph500 scale 17 took 4.4 ms that way and take 1.8, those
 // of a join matrix of 600000 rows 7.5 and 3.5.)
 constexpr int kAChunk = 256;
+constexpr int kCutLow = 1, kCutHigh = 2;
+// the cuts of slice [s0, s1) of a row whose columns lie in [lo, hi)
+__device__ __forceinline__ int cut_of(int64_t s0, int64_t s1, int64_t lo, int64_t hi) {
+  return (s0 > lo ? kCutLow : 0) | (s1 < hi ? kCutHigh : 0);
+}
 constexpr int kUnroll = 8;
 
 template <typename VIn>
@@ -476,7 +486,7 @@ struct alignas(16) Stage {
 
 template <int BLOCK, bool NEED_VAL, typename VIn, typename F>
 __device__ __forceinline__ int64_t expand_entries(const Csr& A, const Csr& B, int64_t as, int64_t ae, Stage<VIn>& sg,
-                                                  bool ranged, int32_t c0, int32_t c1, F&& f) {
+                                                  int cut, int32_t c0, int32_t c1, int64_t& next, F&& f) {
   const VIn* __restrict__ aval = static_cast<const VIn*>(A.val);
   const VIn* __restrict__ bval = static_cast<const VIn*>(B.val);
   constexpr int ACH = BLOCK < kAChunk ? BLOCK : kAChunk;  // one staged A entry per thread
@@ -496,10 +506,9 @@ __device__ __forceinline__ int64_t expand_entries(const Csr& A, const Csr& B, in
       const int32_t k = A.col[a0 + threadIdx.x];
       lo = B.rp[k];
       int64_t hi = B.rp[k + 1];
-      if (ranged) {
-        lo = lower_bound_g(B.col, lo, hi, c0);
-        hi = lower_bound_g(B.col, lo, hi, c1);
-      }
+      if (cut & kCutLow) lo = ae - as <= ACH ? next : lower_bound_g(B.col, lo, hi, c0);
+      if (cut & kCutHigh) hi = lower_bound_g(B.col, lo, hi, c1);
+      next = hi;
       len = hi - lo;
     }
     long long sum;
@@ -568,10 +577,8 @@ __device__ __forceinline__ int64_t expand_entries(const Csr& A, const Csr& B, in
       for (int i = 0; i < na; ++i) {
         const int32_t k = A.col[a0 + i];
         int64_t l = B.rp[k], h = B.rp[k + 1];
-        if (ranged) {
-          l = lower_bound_g(B.col, l, h, c0);
-          h = lower_bound_g(B.col, l, h, c1);
-        }
+        if (cut & kCutLow) l = lower_bound_g(B.col, l, h, c0);
+        if (cut & kCutHigh) h = lower_bound_g(B.col, l, h, c1);
         const VIn av = NEED_VAL ? aval[a0 + i] : VIn(0);
         for (int64_t j = l + threadIdx.x; j < h; j += BLOCK)
           f(__ldg(B.col + j), av, NEED_VAL ? __ldg(bval + j) : VIn(0), pbase + before + (j - l));
@@ -587,8 +594,14 @@ __device__ __forceinline__ int64_t expand_entries(const Csr& A, const Csr& B, in
 // The products of row r (its A entries [A.rp[r], A.rp[r + 1])).
 template <int BLOCK, bool NEED_VAL, typename VIn, typename F>
 __device__ __forceinline__ int64_t expand_row(const Csr& A, const Csr& B, int64_t r, Stage<VIn>& sg,
-                                              bool ranged, int32_t c0, int32_t c1, F&& f) {
-  return expand_entries<BLOCK, NEED_VAL, VIn>(A, B, A.rp[r], A.rp[r + 1], sg, ranged, c0, c1, f);
+                                              int cut, int32_t c0, int32_t c1, int64_t& next, F&& f) {
+  return expand_entries<BLOCK, NEED_VAL, VIn>(A, B, A.rp[r], A.rp[r + 1], sg, cut, c0, c1, next, f);
+}
+// All of them.
+template <int BLOCK, bool NEED_VAL, typename VIn, typename F>
+__device__ __forceinline__ int64_t expand_row(const Csr& A, const Csr& B, int64_t r, Stage<VIn>& sg, F&& f) {
+  int64_t next = 0;
+  return expand_entries<BLOCK, NEED_VAL, VIn>(A, B, A.rp[r], A.rp[r + 1], sg, 0, 0, 0, next, f);
 }
 
 // ================================================================ SYMBOLIC
@@ -705,13 +718,14 @@ k_symb_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
   row_col_range<BLOCK>(A, B, r, b_sorted != 0, c_ncol, lo, hi);
   const bool multi = hi - lo > kDenseChunkBits;
   long long cnt = 0;
+  int64_t next = 0;
   for (int64_t c0 = lo; c0 < hi; c0 += kDenseChunkBits) {
     const int64_t c1 = (hi < c0 + kDenseChunkBits ? hi : c0 + kDenseChunkBits);
     const int nw = (int)((c1 - c0 + 31) >> 5);  // words the slice uses
     for (int i = threadIdx.x; i < nw; i += BLOCK) bm[i] = 0u;
     __syncthreads();
     bool bad = false;
-    expand_row<BLOCK, false, double>(A, B, r, sg, multi, (int32_t)c0, (int32_t)c1,
+    expand_row<BLOCK, false, double>(A, B, r, sg, cut_of(c0, c1, lo, hi), (int32_t)c0, (int32_t)c1, next,
                                      [&](int32_t key, double, double, int64_t) {
       const uint32_t idx = (uint32_t)key - (uint32_t)c0;
       if (idx >= (uint32_t)(c1 - c0)) { bad = true; return; }
@@ -852,7 +866,7 @@ __device__ __forceinline__ void esc_radix_row(int64_t r, const Csr& A, const Csr
   __syncthreads();
   uint32_t kmin = 0xFFFFFFFFu, kmax = 0u;
   bool over = false;
-  const int64_t n = expand_row<BLOCK, true, VIn>(A, B, r, sg, false, 0, 0,
+  const int64_t n = expand_row<BLOCK, true, VIn>(A, B, r, sg,
                                                 [&](int32_t key, VIn av, VIn bv, int64_t p) {
     if (p >= CAP) { over = true; return; }
     items[p] = ((uint64_t)(uint32_t)key << 32) | (uint64_t)p;
@@ -3072,7 +3086,7 @@ k_numc_hash(const int32_t* __restrict__ rows, Csr A, Csr B, const int64_t* __res
   if (threadIdx.x == 0) { s_min = 0xFFFFFFFFu; s_max = 0u; s_cnt = 0; s_full = 0; }
   __syncthreads();
   bool full = false;
-  expand_row<BLOCK, true, VIn>(A, B, r, sg, false, 0, 0, [&](int32_t key, VIn av, VIn bv, int64_t) {
+  expand_row<BLOCK, true, VIn>(A, B, r, sg, [&](int32_t key, VIn av, VIn bv, int64_t) {
     const AT v = Acc<VIn>::mul(av, bv);
     uint32_t h = hash_slot((uint32_t)key, TBITS);
     for (int probe = 0; probe < T; ++probe) {
@@ -3263,8 +3277,7 @@ k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
   const int64_t c0r = crp[r], nz = crp[r + 1] - c0r;
   int64_t lo, hi;
   row_col_range<BLOCK>(A, B, r, b_sorted != 0, c_ncol, lo, hi);
-  const bool multi = hi - lo > kRankCols;
-  int64_t written = 0;
+  int64_t written = 0, next_bits = 0, next = 0;
   for (int64_t s0 = lo; s0 < hi; s0 += kRankCols) {
     const int64_t s1 = hi < s0 + kRankCols ? hi : s0 + kRankCols;
     const int nw = (int)((s1 - s0 + 31) >> 5);
@@ -3276,7 +3289,7 @@ k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
     } else {
       for (int i = threadIdx.x; i < nw; i += BLOCK) bm[i] = 0u;
       __syncthreads();
-      expand_row<BLOCK, false, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1,
+      expand_row<BLOCK, false, VIn>(A, B, r, sg, cut_of(s0, s1, lo, hi), (int32_t)s0, (int32_t)s1, next_bits,
                                     [&](int32_t key, VIn, VIn, int64_t) {
         const uint32_t idx = (uint32_t)key - (uint32_t)s0;
         if (idx < (uint32_t)(s1 - s0)) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
@@ -3292,7 +3305,7 @@ k_numc_dense(const int32_t* __restrict__ rows, Csr A, Csr B, int64_t c_ncol, int
     for (uint32_t i = threadIdx.x; i < cnt; i += BLOCK) cval[base + i] = AT(0);
     emit_columns<BLOCK>(bm, nw, gbase, wrank, cnt, (int32_t)s0, sm.tile, ccol + base);
     __syncthreads();  // the zeroed values are visible to the block's atomic adds
-    expand_row<BLOCK, true, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1,
+    expand_row<BLOCK, true, VIn>(A, B, r, sg, cut_of(s0, s1, lo, hi), (int32_t)s0, (int32_t)s1, next,
                                  [&](int32_t key, VIn av, VIn bv, int64_t) {
       const uint32_t idx = (uint32_t)key - (uint32_t)s0;
       if (idx >= (uint32_t)(s1 - s0)) return;
@@ -3402,8 +3415,7 @@ k_dense_setup(HeavyPlan hp, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, int 
     hp.nslices[i] = ns;
     if (ns > hp.max_slices) dev_report(st, kDevCapacity, 14, r);
   }
-  const bool multi = ns > 1;
-  int64_t written = 0;
+  int64_t written = 0, next = 0;
   for (int sl = 0; sl < ns && sl < hp.max_slices; ++sl) {
     const int64_t s0 = lo + (int64_t)sl * kRankCols;
     const int64_t s1 = hi < s0 + kRankCols ? hi : s0 + kRankCols;
@@ -3421,7 +3433,8 @@ k_dense_setup(HeavyPlan hp, Csr A, Csr B, int64_t c_ncol, int32_t b_sorted, int 
     } else {
       for (int w = threadIdx.x; w < nw; w += BLOCK) bm[w] = 0u;
       __syncthreads();
-      expand_row<BLOCK, false, VIn>(A, B, r, sg, multi, (int32_t)s0, (int32_t)s1, [&](int32_t key, VIn, VIn, int64_t) {
+      expand_row<BLOCK, false, VIn>(A, B, r, sg, cut_of(s0, s1, lo, hi), (int32_t)s0, (int32_t)s1, next,
+                                    [&](int32_t key, VIn, VIn, int64_t) {
         const uint32_t idx = (uint32_t)key - (uint32_t)s0;
         if (idx < (uint32_t)(s1 - s0)) atomicOr(&bm[idx >> 5], 1u << (idx & 31));
       });
@@ -3493,6 +3506,7 @@ k_dense_acc(HeavyPlan hp, Csr A, Csr B, int words, const int64_t* __restrict__ c
     const int ns = hp.nslices[i];
     const int64_t lo = hp.lo[i], hi = hp.hi[i];
     const int64_t c0r = crp[r];
+    int64_t next = 0;
     for (int sl = 0; sl < ns && a1 > a0; ++sl) {
       const int64_t s0 = lo + (int64_t)sl * kRankCols;
       const int64_t s1 = hi < s0 + kRankCols ? hi : s0 + kRankCols;
@@ -3503,7 +3517,7 @@ k_dense_acc(HeavyPlan hp, Csr A, Csr B, int words, const int64_t* __restrict__ c
       __syncthreads();
       slice_ranks<BLOCK>(bm, nw, gbase, wrank, sg.tmp);
       const int64_t base = c0r + sb;
-      expand_entries<BLOCK, true, VIn>(A, B, a0, a1, sg, ns > 1, (int32_t)s0, (int32_t)s1,
+      expand_entries<BLOCK, true, VIn>(A, B, a0, a1, sg, cut_of(s0, s1, lo, hi), (int32_t)s0, (int32_t)s1, next,
                                        [&](int32_t key, VIn av, VIn bv, int64_t) {
         const uint32_t idx = (uint32_t)key - (uint32_t)s0;
         if (idx >= (uint32_t)(s1 - s0)) return;
@@ -3621,13 +3635,14 @@ k_heavy_bits(HeavyPlan hp, Csr A, Csr B, int words, DevStatus* st) {
     const int64_t a1 = q + 1 == K ? ae : first_at(P * (q + 1) / K);
     const int ns = hp.nslices[i] < hp.max_slices ? hp.nslices[i] : hp.max_slices;
     const int64_t lo = hp.lo[i], hi = hp.hi[i];
+    int64_t next = 0;
     for (int sl = 0; sl < ns && a1 > a0; ++sl) {
       const int64_t s0 = lo + (int64_t)sl * kRankCols;
       const int64_t s1 = hi < s0 + kRankCols ? hi : s0 + kRankCols;
       const int nw = (int)((s1 - s0 + 31) >> 5);
       for (int w = threadIdx.x; w < nw; w += BLOCK) bm[w] = 0u;
       __syncthreads();
-      expand_entries<BLOCK, false, double>(A, B, a0, a1, sg, ns > 1, (int32_t)s0, (int32_t)s1,
+      expand_entries<BLOCK, false, double>(A, B, a0, a1, sg, cut_of(s0, s1, lo, hi), (int32_t)s0, (int32_t)s1, next,
                                            [&](int32_t key, double, double, int64_t) {
         const uint32_t idx = (uint32_t)key - (uint32_t)s0;
         if (idx < (uint32_t)(s1 - s0)) atomicOr(&bm[idx >> 5], 1u << (idx & 31));

@@ -41,6 +41,29 @@ def test_walk(ctx, lengths, entries, algo, ncol, dtype):
     np.testing.assert_array_equal(out.csr.vals.astype(np.float64), vals)
 
 
+@pytest.mark.parametrize("per", [40, 700])  # products of a row on either side of 2^17, where rows are split
+@pytest.mark.parametrize("entries", [255, 256, 257, 600])
+def test_slices_follow_each_other(ctx, per, entries):
+    """Rows over four column slices, in one staged chunk and in several: B rows that reach all slices, one of them,
+    only the last, and none."""
+    rng = np.random.default_rng(entries)
+    ncol, mid, rows = 4 * 524288 - 3, 601, 5
+    spans = [(0, ncol), (524288, 2 * 524288), (ncol - 9000, ncol), (524280, 524300)]
+    cols = [np.zeros(0, np.int64) if k % 5 == 4 else
+            np.sort(rng.choice(np.arange(*spans[k % 5]), min(per, spans[k % 5][1] - spans[k % 5][0]), replace=False))
+            for k in range(mid)]
+    B = from_coo(mid, ncol, np.repeat(np.arange(mid), [len(c) for c in cols]), np.concatenate(cols),
+                 rng.integers(1, 8, sum(map(len, cols))))
+    A = from_coo(rows, mid, np.repeat(np.arange(rows), entries),
+                 np.concatenate([rng.choice(mid, entries, replace=False) for _ in range(rows)]),
+                 rng.integers(1, 8, rows * entries))
+    out = ctx.spgemm(A, B, "hash")
+    rp, want, vals, _ = oracle.oracle_spgemm(A, B, "hash")
+    np.testing.assert_array_equal(out.csr.row_ptrs, rp)
+    np.testing.assert_array_equal(out.csr.cols.astype(np.int64), want)
+    np.testing.assert_array_equal(out.csr.vals.astype(np.float64), vals)
+
+
 @pytest.mark.parametrize("ncol", [16385, 131072, 524288, 524289, 1100000])
 @pytest.mark.parametrize("nnz", [4097, 8192, 20000])
 def test_dense_row_columns_leave_in_tiles(ctx, ncol, nnz):
