@@ -10,7 +10,8 @@
 //   NUMC  numeric kernels per bin
 // Each phase boundary is a CUDA event; the phase times are what cas_runtime
 // reports, like the reference's runtime_t.  The host waits three times per
-// call, each to size the next phase (bin counts, nnz(C)).
+// call: for the symbolic bins' counts, for nnz(C) and the numeric bins' counts,
+// and for the end.
 #include <cuda_runtime.h>
 
 #include <immintrin.h>
