@@ -38,6 +38,9 @@ class CasCsr(ctypes.Structure):
         ("col_bytes", ctypes.c_int32), ("val_type", ctypes.c_int32),
         ("on_device", ctypes.c_int32), ("owned", ctypes.c_int32),
     ]
+    # bytes of a value, which val_type does not say: a product of int32 matrices
+    # has int64 values, their transpose (Context.transpose_device) int32 ones
+    value_bytes = 8
 
 
 class CasRuntime(ctypes.Structure):
@@ -391,6 +394,7 @@ class Context:
         cb = CasCsr()
         cb.on_device = 1
         self._check(self.lib.cas_csr_transpose(self.h, ctypes.byref(ca), ctypes.byref(cb)))
+        cb.value_bytes = 8 if cb.val_type == VAL_F64 else 4
         return cb
 
     def free(self, cc: CasCsr):
@@ -398,6 +402,8 @@ class Context:
 
     def digest(self, cc: CasCsr, rows: bool = False):
         """Digest of a device CSR (cas_csr_digest); with rows, also its row digests."""
+        if cc.value_bytes != 8:
+            raise ValueError("digests are of products: fp64 or int64 values")
         d = ctypes.c_uint64()
         rd = np.empty(cc.num_row, np.uint64) if rows else None
         self._check(self.lib.cas_csr_digest(self.h, ctypes.byref(cc), ctypes.byref(d), _ptr(rd)))
@@ -744,7 +750,8 @@ def device_tensors(cc: CasCsr):
             return torch.empty(0, dtype=dtype, device="cuda")
         return torch.as_tensor(_DeviceView(ptr, n, typestr), device="cuda")
 
-    vt = ("<f8", torch.float64) if cc.val_type == VAL_F64 else ("<i8", torch.int64)
+    vt = (("<f8", torch.float64) if cc.val_type == VAL_F64 else
+          ("<i8", torch.int64) if cc.value_bytes == 8 else ("<i4", torch.int32))
     return (view(cc.row_ptrs, cc.num_row + 1, "<i8", torch.int64), view(cc.cols, cc.num_nnz, "<i4", torch.int32),
             view(cc.rats, cc.num_nnz, *vt))
 
