@@ -2285,18 +2285,22 @@ __device__ __forceinline__ uint32_t atomic_or_if(bool c, uint32_t* p, uint32_t v
 }
 
 // Sum of x over the lanes of `peers` (the lanes with this lane's key), at
-// their lowest lane; the whole warp takes part.
+// their lowest lane, pairwise; the whole warp takes part.  List ranking by
+// pointer jumping (J. C. Wyllie, The Complexity of Parallel Computations,
+// 1979): x stands for the lane's peers up to, not including, lane `next`; each
+// turn it takes up what `next` stands for, so twice as many.
 template <typename T>
 __device__ __forceinline__ T peers_sum(unsigned peers, T x) {
   const int lane = threadIdx.x & 31;
-  int rel = __popc(peers & lanemask_lt());
-  peers &= 0xFFFFFFFEu << lane;  // the lanes above
-  while (__any_sync(kFull, peers != 0)) {
-    const int next = __ffs(peers);
-    const T y = __shfl_sync(kFull, x, next > 0 ? next - 1 : lane);
-    if (next > 0) x += y;
-    peers &= __ballot_sync(kFull, (rel & 1) == 0);
-    rel >>= 1;
+  int next = __ffs(peers & (0xFFFFFFFEu << lane)) - 1;  // -1: none above
+  while (__any_sync(kFull, next >= 0)) {
+    const int from = next >= 0 ? next : lane;
+    const T y = __shfl_sync(kFull, x, from);
+    const int beyond = __shfl_sync(kFull, next, from);
+    if (next >= 0) {
+      x += y;
+      next = beyond;
+    }
   }
   return x;
 }
