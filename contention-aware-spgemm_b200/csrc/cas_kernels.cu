@@ -1,4 +1,6 @@
 // casgemm kernel bodies (contracts in cas_kernels.cuh).
+#include <type_traits>
+
 #include "cas_kernels.cuh"
 #include "cas_sortnet.cuh"
 
@@ -2206,7 +2208,12 @@ k_numc_esc_idx(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted,
 //   4. values are loaded in product order (B's own): owners store
 //      a_ik * b_kj at their places, the repeats add theirs by shared-memory
 //      atomics (listed and summed per warp first when they are few: the
-//      diagonal of A*A^T brings one per A entry);
+//      diagonal of A*A^T brings one per A entry).  Real values in the bins up
+//      to 5120 products are all listed, behind the values (8 bytes a column
+//      and 4 a repeat are at most 8 a product), and each place's are summed by
+//      one warp, pairwise 32 at a time.  Added one by one, the error of a
+//      column of 64 products was 2.8 times a pairwise sum's; it is 0.7 to 1.1
+//      times, for 1.2% of the product of 70,001 ragged rows (839 to 849 us);
 //   5. the values, then the columns (still in registers), are copied to C in
 //      order.
 // The slots are scanned eight to a thread; rank_slot swaps every second pair
@@ -2305,6 +2312,30 @@ __device__ __forceinline__ T peers_sum(unsigned peers, T x) {
   return x;
 }
 
+// Sums of a column's repeats that come in several parts, one lane at a time:
+// *at += x, and what that rounds off (Knuth's TwoSum) is kept in the upper 16
+// bits of a double, to be added at the end by rest_of.
+template <typename AT>
+__device__ __forceinline__ void add_part(AT* at, AT x, uint16_t* rest) {
+  if constexpr (std::is_same<AT, double>::value) {
+    const double a = *at, s = a + x, t = s - a;
+    *at = s;
+    if (rest) {
+      const double e = __hiloint2double((int)*rest << 16, 0) + ((a - (s - t)) + (x - t));
+      if (isfinite(e)) *rest = (uint16_t)((uint32_t)__double2hiint(e) >> 16);
+    }
+  } else {
+    *at += x;
+  }
+}
+template <typename AT>
+__device__ __forceinline__ AT rest_of(AT x, uint16_t rest) {
+  if constexpr (std::is_same<AT, double>::value) {
+    if (rest) x += __hiloint2double((int)rest << 16, 0);
+  }
+  return x;
+}
+
 // log2 of the bitmap's cells for rows of up to `cap` products over ncol
 // columns.  Clearing and scanning the bitmap is work for every row, the
 // second level work for every product: one column per cell while that is at
@@ -2392,6 +2423,9 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
   constexpr int G = NPT >= 16 ? 4 : 2;            // products whose loads are in flight together
   constexpr int WCH = 4;                          // bitmap chunks of 4 words per thread in one scan
   constexpr int SCH = (CAP + 8 * BLOCK - 1) / (8 * BLOCK);  // slot chunks of 8 per thread
+  // Repeats summed pairwise by column: real values of the bins up to 5120
+  // products, which the bucketed form summed so too.
+  constexpr bool kPairs = !FUSED && CAP <= 5120 && std::is_same<VIn, double>::value;
   static_assert(CAP < 16384 && NPT % G == 0 && NPT <= 32, "places in 16 bits, whole groups, one flag per product");
   static_assert(WCH <= 4 && SCH <= 4, "four 16-bit counts in one word of a scan");
   static_assert(CAP % 16 == 0 && NW <= 16, "vector access to the slots; the scans' words");
@@ -2603,18 +2637,30 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
   // fused rows: the count goes out now; the look-back waits until the values
   // are in place, so the wait for earlier rows overlaps them
   if (FUSED && threadIdx.x == 0) lookback_publish(fu.status, tick, distinct);
-  const bool listed = n - distinct <= BLOCK;
+  const int nrep = n - distinct;
+  const bool listed = kPairs || nrep <= BLOCK;
   const uint32_t dup = valid & ~own;
+  // where the repeats are listed: in rep, or behind the values
+  const bool behind = kPairs && nrep > 32;
+  uint32_t* list = behind ? reinterpret_cast<uint32_t*>(sval + distinct) : rep;
+  uint16_t* rest = nullptr;  // add_part's, behind the list
+  if (behind) {
+    if ((size_t)distinct * 10 + (size_t)nrep * 4 <= rank_arena<CAP>(cell_bits))
+      rest = reinterpret_cast<uint16_t*>(list + nrep);
+    __syncthreads();  // the slots there are read
+    if (rest)
+      for (int i = threadIdx.x; i < distinct; i += BLOCK) rest[i] = 0;
+  }
   if (listed && dup) {
 #pragma unroll
     for (int g = 0; g < NPT; g += G) {
       if (((dup >> g) & ((1u << G) - 1u)) == 0) continue;
 #pragma unroll
       for (int u = g; u < g + G; ++u)
-        if ((dup >> u) & 1u) rep[atomicAdd(&sg.repeats, 1)] = (uint32_t)(threadIdx.x + u * BLOCK) | (get_pos(u) << 16);
+        if ((dup >> u) & 1u) list[atomicAdd(&sg.repeats, 1)] = (uint32_t)(threadIdx.x + u * BLOCK) | (get_pos(u) << 16);
     }
   }
-  __syncthreads();
+  if (!behind) __syncthreads();
   // 4. values
   auto values = [&](int p0, int p1, uint32_t which, auto&& put) {
 #pragma unroll
@@ -2643,9 +2689,62 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
   auto add = [](bool c, AT* p, AT v) {
     if (c) atomic_add_sh(p, v);
   };
+  // the listed repeats of [p0, p1), 32 at a time: at most 32 by one warp, else
+  // those whose places are the warp's (place modulo warps) through its words of rep
+  bool first_round = true;
+  auto add_pairs = [&](int p0, int p1) {
+    uint32_t* q = rep + warp * 32;
+    auto round = [&](uint32_t d, bool in) {
+      const unsigned peers = __match_any_sync(kFull, in ? d >> 16 : 0x10000u);
+      const bool first = in && lane == __ffs(peers) - 1;
+      AT* at = &sval[d >> 16];
+      AT x = AT(0);
+      if (in) {
+        const int p = (int)(d & 0xFFFFu), e = segof[p];
+        x = Acc<VIn>::mul(sg.av[e], __ldg(sg.vp[e] + p));
+      }
+      if (first && first_round) x += *at;
+      x = peers_sum(peers, x);
+      if (first) {
+        if (first_round) *at = x;
+        else add_part(at, x, rest ? rest + (d >> 16) : nullptr);
+      }
+      first_round = false;
+    };
+    if (!behind) {
+      if (warp > 0) return;
+      const uint32_t d = lane < nrep ? list[lane] : 0u;
+      round(d, lane < nrep && (int)(d & 0xFFFFu) >= p0 && (int)(d & 0xFFFFu) < p1);
+      return;
+    }
+    int have = 0;
+    for (int i0 = 0; i0 < nrep; i0 += 32) {
+      const uint32_t d = i0 + lane < nrep ? list[i0 + lane] : 0u;
+      const int p = (int)(d & 0xFFFFu);
+      const bool mine = i0 + lane < nrep && (d >> 16) % NW == warp && p >= p0 && p < p1;
+      const unsigned in = __ballot_sync(kFull, mine);
+      const int to = have + __popc(in & lanemask_lt());
+      if (mine && to < 32) q[to] = d;
+      have += __popc(in);
+      if (have >= 32) {
+        __syncwarp();
+        round(q[lane], true);
+        __syncwarp();
+        if (mine && to >= 32) q[to - 32] = d;
+        have -= 32;
+      }
+    }
+    __syncwarp();
+    if (have > 0) round(lane < have ? q[lane] : 0u, lane < have);
+    __syncwarp();
+  };
   auto add_listed = [&](int p0, int p1) {
-    if (warp * 32 >= n - distinct) return;
-    const uint32_t d = threadIdx.x < n - distinct ? rep[threadIdx.x] : 0xFFFFFFFFu;
+    if (kPairs) {
+      add_pairs(p0, p1);
+      return;
+    }
+    if (warp * 32 >= nrep) return;
+    const uint32_t d = threadIdx.x < nrep ? list[threadIdx.x] : 0xFFFFFFFFu;
     const int p = (int)(d & 0xFFFFu);
     const bool in = p >= p0 && p < p1;
     AT x = AT(0);
@@ -2707,7 +2806,10 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
     __syncthreads();
   }
   // 5. the row in order; the columns follow over the same shared memory
-  for (int i = threadIdx.x; i < distinct; i += BLOCK) cval[c0 + i] = sval[i];
+  if (kPairs && rest)
+    for (int i = threadIdx.x; i < distinct; i += BLOCK) cval[c0 + i] = rest_of(sval[i], rest[i]);
+  else
+    for (int i = threadIdx.x; i < distinct; i += BLOCK) cval[c0 + i] = sval[i];
   __syncthreads();
 #pragma unroll
   for (int g = 0; g < NPT; g += G) {
@@ -3022,35 +3124,64 @@ k_numc_warp(const int32_t* __restrict__ rows, int64_t nrows, Csr A, Csr B, int32
     if (lane == 0) dev_report(st, (int64_t)distinct > nz ? kDevRowOverflow : kDevRowUnderflow, 18, r);
     return;
   }
-  // values: owners store, the others add
+  // values: the owners store theirs
   const VIn* __restrict__ bval = static_cast<const VIn*>(B.val);
   auto half = [&](int u) -> uint32_t { return (u & 1) ? pos[u >> 1] >> 16 : pos[u >> 1] & 0xFFFFu; };
-  auto values = [&](uint32_t which, bool owners) {
 #pragma unroll
-    for (int g = 0; g < NPT; g += G) {
-      if (32u * g >= n) break;
-      if (!owners && !__any_sync(kFull, (which >> g) & ((1u << G) - 1u))) continue;
-      VIn bv[G];
+  for (int g = 0; g < NPT; g += G) {
+    if (32u * g >= n) break;
+    VIn bv[G];
 #pragma unroll
-      for (int v = 0; v < G; ++v)
-        bv[v] = __ldg(bval + (sg.off[half(g + v) >> 9] + min(32u * (g + v) + lane, n - 1)));
+    for (int v = 0; v < G; ++v)
+      bv[v] = __ldg(bval + (sg.off[half(g + v) >> 9] + min(32u * (g + v) + lane, n - 1)));
 #pragma unroll
-      for (int v = 0; v < G; ++v) {
-        const uint32_t h = half(g + v);
-        const AT x = Acc<VIn>::mul(sg.av[h >> 9], bv[v]);
-        const bool on = (which >> (g + v)) & 1u;
-        if (owners) sts_if(on, &sval[h & 0x1FFu], x);
-        else if (on) atomic_add_sh(&sval[h & 0x1FFu], x);
+    for (int v = 0; v < G; ++v) {
+      const uint32_t h = half(g + v);
+      sts_if((own >> (g + v)) & 1u, &sval[h & 0x1FFu], Acc<VIn>::mul(sg.av[h >> 9], bv[v]));
+    }
+  }
+  // The others are listed behind the values (8 bytes a column and 4 a repeat
+  // are at most 8 a product) and summed 32 at a time, pairwise by column, the
+  // owner's with the first.  Added one by one, the error of the diagonal of
+  // A*A^T (one product per A entry) was 1.5 times a pairwise sum's at 16
+  // products and 2.3 times at 65, that of a product of uniform rows of 256
+  // products 1.44 times; these are 1.0 now, and the product of 131072 such rows
+  // took 909 us then, 877 now (a 32-lane pass a list instead of one a group).
+  uint16_t* rest = nullptr;
+  if (distinct < n) {
+    uint32_t* rep = reinterpret_cast<uint32_t*>(sval + distinct);  // product, entry and place
+    const uint32_t dup = valid & ~own, nrep = n - distinct;
+    if (std::is_same<VIn, double>::value && nrep > 32 &&
+        distinct * 10 + nrep * 4 <= rank_arena<kWarpProducts>(cell_bits)) {
+      rest = reinterpret_cast<uint16_t*>(rep + nrep);
+      for (uint32_t i = lane; i < distinct; i += 32) rest[i] = 0;
+    }
+    uint32_t listed = 0;
+#pragma unroll
+    for (int u = 0; u < NPT; ++u) {
+      if (32u * u >= n) break;
+      const unsigned in = __ballot_sync(kFull, (dup >> u) & 1u);
+      sts_if((dup >> u) & 1u, &rep[listed + __popc(in & lanemask_lt())], (32u * u + lane) | (half(u) << 16));
+      listed += __popc(in);
+    }
+    for (uint32_t i0 = 0; i0 < nrep; i0 += 32) {
+      __syncwarp();
+      const bool in = i0 + lane < nrep;
+      const uint32_t d = in ? rep[i0 + lane] : 0u, e = d >> 25, at = (d >> 16) & 0x1FFu;
+      const unsigned peers = __match_any_sync(kFull, in ? at : (uint32_t)kWarpProducts);
+      const bool first = in && lane == __ffs(peers) - 1;
+      AT x = AT(0);
+      if (in) x = Acc<VIn>::mul(sg.av[e], __ldg(bval + (sg.off[e] + (d & 0xFFFFu))));
+      if (first && i0 == 0) x += sval[at];
+      x = peers_sum(peers, x);
+      if (first) {
+        if (i0 == 0) sval[at] = x;
+        else add_part(&sval[at], x, rest ? rest + at : nullptr);
       }
     }
-  };
-  values(own, true);
-  if (distinct < n) {
-    __syncwarp();
-    values(valid & ~own, false);
   }
   __syncwarp();
-  for (uint32_t i = lane; i < distinct; i += 32) cval[c0 + i] = sval[i];
+  for (uint32_t i = lane; i < distinct; i += 32) cval[c0 + i] = rest ? rest_of(sval[i], rest[i]) : sval[i];
   __syncwarp();
   uint32_t* scol = bits;
 #pragma unroll
