@@ -2264,6 +2264,9 @@ __device__ __forceinline__ T block_exclusive_sum1(T v, T* tmp, T& total) {
   return (warp > 0 ? before : T(0)) + inc - v;
 }
 
+// The lowest n bits, n from 0 to 32 (a shift by 32 is undefined).
+__host__ __device__ __forceinline__ uint32_t low_bits(int n) { return n >= 32 ? 0xFFFFFFFFu : (1u << n) - 1u; }
+
 // Shared-memory accesses under a predicate, without a branch.
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void sts_if(bool c, uint32_t* p, uint32_t v) {
@@ -2504,7 +2507,7 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
   }
   const int nwords = (int)((range >> shift) >> 5) + 1;
   const int cnt = n > (int)threadIdx.x ? (n - (int)threadIdx.x + BLOCK - 1) / BLOCK : 0;
-  const uint32_t valid = cnt >= 32 ? 0xFFFFFFFFu : (1u << cnt) - 1u;
+  const uint32_t valid = low_bits(cnt);
   uint32_t own = 0;  // bit u: the thread's product u set its cell's bit
 #pragma unroll
   for (int g = 0; g < NPT; g += G) {
@@ -2683,7 +2686,7 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
   auto within = [&](int p0, int p1) -> uint32_t {
     const int t = threadIdx.x;
     const int c1 = p1 > t ? (p1 - t + BLOCK - 1) / BLOCK : 0, c0 = p0 > t ? (p0 - t + BLOCK - 1) / BLOCK : 0;
-    return (c1 >= 32 ? 0xFFFFFFFFu : (1u << c1) - 1u) & ~((1u << c0) - 1u);
+    return low_bits(c1) & ~low_bits(c0);
   };
   auto store = [](bool c, AT* p, AT v) { sts_if(c, p, v); };
   auto add = [](bool c, AT* p, AT v) {
