@@ -319,6 +319,8 @@ cas_status setup_numc_kernels(cas_ctx* ctx) {
   return CAS_OK;
 }
 
+cas_status setup_transpose(cas_ctx* ctx);
+
 cas_status setup_kernels(cas_ctx* ctx) {
   using namespace cas;
 #define CAS_SETUP_SYMB(bin, BLK, TB, SEG) CAS_TRY(allow_smem(ctx, k_symb_hash<BLK, TB, SEG>, smem_symb_hash<BLK, TB, SEG>()));
@@ -331,7 +333,7 @@ cas_status setup_kernels(cas_ctx* ctx) {
   CAS_TRY(allow_smem(ctx, k_heavy_bits<512>, smem_symb_dense(kRankCols / 32)));
   CAS_TRY(setup_numc_kernels<double>(ctx));
   CAS_TRY(setup_numc_kernels<int32_t>(ctx));
-  return CAS_OK;
+  return setup_transpose(ctx);
 }
 
 int grid_for(int64_t items, int block, int cap) {

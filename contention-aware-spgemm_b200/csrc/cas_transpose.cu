@@ -384,7 +384,6 @@ cas_status transpose_rows(cas_ctx* ctx, const DevMat& A, int shift, const int64_
   if (m <= cas::kRankCols) {
     const int words = dense_words(m);
     const size_t smem = cas::DenseSmem<double>::ranks(words);
-    CAS_TRY(allow_smem(ctx, k_tr_rank<512, V>, smem));
     k_tr_rank<512, V><<<(unsigned)rest, 512, smem, ctx->stream>>>(m, shift, words, brp, big, key, aval, bcol, bval,
                                                                   big + rest, nagain);
     CAS_TRY(check_launch(ctx, "k_tr_rank"));
@@ -397,6 +396,15 @@ cas_status transpose_rows(cas_ctx* ctx, const DevMat& A, int shift, const int64_
   CAS_TRY(check_launch(ctx, "k_tr_sort_block"));
   k_tr_gather<V><<<(unsigned)rest, kTrBlock, 0, ctx->stream>>>(shift, brp, list, key, aval, bcol, bval);
   return check_launch(ctx, "k_tr_gather");
+}
+
+// The limit is the kernel's on the device, for all contexts and threads: set
+// once to the most a call may take, not to what each call does (a narrower
+// matrix on another thread would take it from a wide one's launch).
+cas_status setup_transpose(cas_ctx* ctx) {
+  const size_t smem = cas::DenseSmem<double>::ranks(cas::kRankCols / 32);
+  CAS_TRY(allow_smem(ctx, k_tr_rank<512, double>, smem));
+  return allow_smem(ctx, k_tr_rank<512, int32_t>, smem);
 }
 
 cas_status transpose_device(cas_ctx* ctx, const DevMat& A, int vt, cas_csr* B, bool to_host, double& d2h) {
