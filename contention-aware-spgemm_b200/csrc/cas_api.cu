@@ -866,10 +866,12 @@ cas_status join(cas_ctx* ctx) {
   return CAS_OK;
 }
 
-// After an error: kernels of the call that may still run on the auxiliary
-// streams end before its memory is freed.
+// After an error: kernels of the call that may still run, on its stream or the
+// auxiliary ones, end before its memory is freed.  The next call may come on
+// another stream (cas_set_stream) and uses the same workspace and counters.
 void quiesce(cas_ctx* ctx) {
   for (int i = 0; i < kAux; ++i) cudaStreamSynchronize(ctx->aux[i]);
+  cudaStreamSynchronize(ctx->stream);
   cudaGetLastError();
 }
 
