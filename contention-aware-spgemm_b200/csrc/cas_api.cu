@@ -33,6 +33,7 @@
 
 #include "casgemm.h"
 #include "cas_kernels.cu"
+#include "cas_workspace.h"
 
 namespace {
 
@@ -87,9 +88,7 @@ struct cas_ctx {
   int hash_max = 4096;                     // hash rows: at most this many distinct columns
   int out_blocks = 0;                      // C in host memory: row blocks (0: by C's size)
   cudaMemPool_t scratch = nullptr;         // the device's scratch pool (scratch_pool_get)
-  char* ws = nullptr;                      // workspace that products take their scratch from (ws_alloc):
-  size_t ws_cap = 0, ws_used = 0;          // its bytes, and those the current product has taken
-  size_t ws_need = 0;                      // what the current product has asked for
+  cas::Workspace ws;                       // what products take their scratch from (ws_alloc)
   double mem_share = 1.0;                  // share of the free device memory this context sizes
                                            // its optional scratch by (a batch worker's: 1 / workers)
   double acc_thres = 2.0;
@@ -372,8 +371,8 @@ constexpr int kMaxDevices = 64;
 struct ScratchPool {
   cudaMemPool_t pool = nullptr;
   int users = 0;
-  size_t total = 0;    // bytes of the device's memory
-  size_t ws_bytes = 0; // of the contexts' workspaces
+  size_t total = 0;         // bytes of the device's memory
+  cas::WorkspaceBook book;  // the contexts' workspaces
 };
 std::mutex g_scratch_mu;
 ScratchPool g_scratch[kMaxDevices];
@@ -403,6 +402,7 @@ cas_status scratch_pool_get(cas_ctx* ctx) {
   }
   ++sp.users;
   ctx->scratch = sp.pool;
+  sp.book.join(ctx->ws);
   return CAS_OK;
 }
 
@@ -427,7 +427,7 @@ double free_device_bytes(cas_ctx* ctx) {
     cudaGetLastError();
     return 0.0;
   }
-  double idle = (double)(ctx->ws_cap - ctx->ws_used);
+  double idle = (double)(ctx->ws.cap - ctx->ws.used);
   cudaMemPool_t pools[2] = {nullptr, ctx->scratch};
   if (cudaDeviceGetDefaultMemPool(&pools[0], ctx->device) != cudaSuccess) pools[0] = nullptr;
   for (cudaMemPool_t pool : pools) {
@@ -440,18 +440,26 @@ double free_device_bytes(cas_ctx* ctx) {
   return (double)free_b + idle;
 }
 
-// An allocation from `pool` on stream s.  Out of memory, both pools give
-// back what they hold idle, once the stream's pending frees are done, and the
-// allocation is tried again.
+// What the library holds idle on a device, given back to it: the workspaces that
+// no product runs in, whose contexts may be other threads' (nothing on the
+// device uses them: ws_end), then what the pools hold, once the stream's pending
+// frees are done.
+void give_back(cas_ctx* ctx, cudaStream_t s) {
+  g_scratch[ctx->device].book.reclaim([&](char* p) { cudaFreeAsync(p, s); });
+  cudaStreamSynchronize(s);
+  cudaMemPool_t def = nullptr;
+  if (cudaDeviceGetDefaultMemPool(&def, ctx->device) == cudaSuccess) cudaMemPoolTrimTo(def, 0);
+  cudaMemPoolTrimTo(ctx->scratch, 0);
+}
+
+// An allocation from `pool` on stream s, tried again after give_back when no
+// memory is left.
 cudaError_t pool_alloc(cas_ctx* ctx, cudaMemPool_t pool, void** p, size_t bytes, cudaStream_t s) {
   if (bytes == 0) bytes = 16;
   cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    cudaMemPool_t def = nullptr;
-    cudaStreamSynchronize(s);
-    if (cudaDeviceGetDefaultMemPool(&def, ctx->device) == cudaSuccess) cudaMemPoolTrimTo(def, 0);
-    cudaMemPoolTrimTo(ctx->scratch, 0);
+    give_back(ctx, s);
     e = cudaMallocFromPoolAsync(p, bytes, pool, s);
   }
   if (e != cudaSuccess) cudaGetLastError();
@@ -477,51 +485,32 @@ cas_status scratch_ready(cas_ctx* ctx, cudaStream_t s) {
   return CAS_OK;
 }
 
-// A product's scratch comes from a workspace that its context keeps: from the
-// second product of a size on, no call of the allocator is left in it (the
-// pool, for all its order, now and then mapped the largest blocks anew: 1 to 60
-// ms beside a 10 ms product).  What does not fit is allocated, and the
-// workspace grows to the product's need before the next one starts, while the
-// contexts of a device together keep at most kWorkspaceKeep of its memory.
-// Only one product at a time uses it, on the context's stream and the
-// auxiliary streams that join it.
+// A product's scratch comes from a workspace that its context keeps
+// (cas_workspace.h): the pool, for all its order, now and then mapped the
+// largest blocks anew, 1 to 60 ms beside a 10 ms product.  The contexts of a
+// device together keep at most kWorkspaceKeep of its memory.  One product at a
+// time uses a workspace, on the context's stream and the auxiliary streams that
+// join it; ws_end follows once the host has waited for all of it.
 constexpr double kWorkspaceKeep = 1.0 / 16;
 void ws_drop(cas_ctx* ctx) {
-  if (!ctx->ws) return;
-  cudaFreeAsync(ctx->ws, ctx->stream);
-  std::lock_guard<std::mutex> lock(g_scratch_mu);
-  g_scratch[ctx->device].ws_bytes -= ctx->ws_cap;
-  ctx->ws = nullptr;
-  ctx->ws_cap = ctx->ws_used = 0;
+  g_scratch[ctx->device].book.drop(ctx->ws, [&](char* p) { cudaFreeAsync(p, ctx->stream); });
 }
 void ws_begin(cas_ctx* ctx) {
-  const size_t need = (ctx->ws_need + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
-  ctx->ws_used = ctx->ws_need = 0;
-  if (need <= ctx->ws_cap) return;
-  ws_drop(ctx);
-  {
-    std::lock_guard<std::mutex> lock(g_scratch_mu);
-    ScratchPool& sp = g_scratch[ctx->device];
-    if ((double)(sp.ws_bytes + need) > kWorkspaceKeep * (double)sp.total) return;
-    sp.ws_bytes += need;
-  }
-  ctx->ws_cap = need;
-  if (pool_alloc(ctx, ctx->scratch, (void**)&ctx->ws, need, ctx->stream) != cudaSuccess) {
-    std::lock_guard<std::mutex> lock(g_scratch_mu);
-    g_scratch[ctx->device].ws_bytes -= need;
-    ctx->ws = nullptr;
-    ctx->ws_cap = 0;
-  }
+  ScratchPool& sp = g_scratch[ctx->device];
+  auto get = [&](size_t bytes) -> char* {  // as much as there is; not from the other contexts
+    void* p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes, ctx->scratch, ctx->stream) == cudaSuccess) return static_cast<char*>(p);
+    cudaGetLastError();
+    return nullptr;
+  };
+  sp.book.begin(ctx->ws, (size_t)(kWorkspaceKeep * (double)sp.total), get,
+                [&](char* p) { cudaFreeAsync(p, ctx->stream); });
 }
+void ws_end(cas_ctx* ctx) { g_scratch[ctx->device].book.end(ctx->ws); }
 // `spill` gets what was allocated, to be freed after the product.
 cas_status ws_alloc(cas_ctx* ctx, std::vector<void*>& spill, void** p, size_t bytes) {
-  bytes = (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
-  ctx->ws_need += bytes;
-  if (ctx->ws_used + bytes <= ctx->ws_cap) {
-    *p = ctx->ws + ctx->ws_used;
-    ctx->ws_used += bytes;
-    return CAS_OK;
-  }
+  *p = ctx->ws.take(bytes);
+  if (*p) return CAS_OK;
   CAS_TRY(dev_alloc(ctx, p, bytes));
   spill.push_back(*p);
   return CAS_OK;
@@ -1533,17 +1522,23 @@ cas_status compute_dev(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, De
 }
 
 // compute_dev, once more without the workspace when memory runs out beside it.
+// After an error nothing of the call is left, neither memory nor kernels.
 template <typename F>
 cas_status compute(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, DevC& o, F&& at_cap) {
-  cas_status st = compute_dev(ctx, accum, c, validate, o, at_cap);
-  if (st == CAS_ERR_OOM && ctx->ws) {
+  auto undo = [&] {
     quiesce(ctx);
-    CAS_TRY(scratch_free(ctx, c));
+    scratch_free(ctx, c);
     free_dev_c(o, ctx->stream);
+  };
+  cas_status st = compute_dev(ctx, accum, c, validate, o, at_cap);
+  if (st == CAS_ERR_OOM && ctx->ws.mem) {
+    undo();
     ws_drop(ctx);
-    ctx->ws_need = 0;
+    ctx->ws.need = 0;
     st = compute_dev(ctx, accum, c, validate, o, at_cap);
   }
+  if (st != CAS_OK) undo();
+  ws_end(ctx);
   return st;
 }
 
@@ -1748,8 +1743,6 @@ cas_status run_blocked(cas_ctx* ctx, cas_accum accum, const cas_csr* A, Call& fu
       st = check_launch(ctx, "k_rebase_to");
     }
     if (st != CAS_OK) {
-      quiesce(ctx);
-      scratch_free(ctx, ck);
       free_dev_c(o, ctx->stream);
       break;
     }
@@ -1890,9 +1883,6 @@ cas_status run_spgemm(cas_ctx* ctx, cas_accum accum, const cas_csr* A, const cas
   });
   if (st != CAS_OK) {
     free_host();
-    quiesce(ctx);
-    scratch_free(ctx, c);
-    free_dev_c(o, ctx->stream);
     return finish(st);
   }
   const int64_t nnz = o.nnz;
@@ -2039,7 +2029,7 @@ void cas_destroy(cas_ctx* ctx) {
     for (auto& b : ctx->host_free) free(b.first);
   }
   ctx->stream = ctx->own_stream;
-  ws_drop(ctx);
+  if (ctx->scratch) g_scratch[ctx->device].book.leave(ctx->ws, [&](char* p) { cudaFreeAsync(p, ctx->stream); });
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   scratch_pool_put(ctx);
   delete ctx;
@@ -2174,13 +2164,12 @@ cas_status cas_scan(cas_ctx* ctx, int64_t* d_out, const int64_t* d_in, int64_t n
 
 // The end of a phase call: its scratch freed, the kernels' status.
 static cas_status phase_end(cas_ctx* ctx, Call& c, cas_status st) {
-  if (st != CAS_OK) {
-    quiesce(ctx);
-    scratch_free(ctx, c);
-    return st;
-  }
-  CAS_TRY(scratch_free(ctx, c));
-  return check_status(ctx);
+  if (st != CAS_OK) quiesce(ctx);
+  const cas_status freed = scratch_free(ctx, c);
+  if (st == CAS_OK) st = freed;
+  if (st == CAS_OK) st = check_status(ctx);
+  ws_end(ctx);
+  return st;
 }
 
 cas_status cas_hash_symb(cas_ctx* ctx, const cas_csr* A, const cas_csr* B, const int64_t* d_row_flp,
