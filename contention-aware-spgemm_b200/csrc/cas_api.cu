@@ -87,6 +87,7 @@ struct cas_ctx {
   int esc_max = 8192;                      // ESC rows: at most this many products
   int hash_max = 4096;                     // hash rows: at most this many distinct columns
   int out_blocks = 0;                      // C in host memory: row blocks (0: by C's size)
+  cudaMemPool_t def_pool = nullptr;        // the device's default pool
   cudaMemPool_t scratch = nullptr;         // the device's scratch pool (scratch_pool_get)
   cas::Workspace ws;                       // what products take their scratch from (ws_alloc)
   double mem_share = 1.0;                  // share of the free device memory this context sizes
@@ -361,11 +362,13 @@ cas_status free_owned(cas_ctx* ctx, DevMat& m) {
 // were cut up by the next call's scratch, and the pool mapped its memory anew
 // for the next C: a program that keeps three Graph500 scale 17 products paid 6
 // to 25 ms beside each call's 19 for its first fifteen calls; with two pools
-// it pays for the first C of each product only.  Results (C, B = A^T) stay in the device's default pool, where
-// equal sizes find their holes again; scratch has a pool of its own per
-// device, which the contexts of a process share and the last one destroys.  It
-// keeps at most kScratchKeep of the device's memory when idle, and both pools
-// give their idle memory back before an allocation fails.
+// it pays for the first C of each product only.  Results (C, B = A^T) stay in
+// the device's default pool, where equal sizes find their holes again; scratch
+// has a pool of its own per device, which the contexts of a process share and
+// the last one destroys.  It keeps at most kScratchKeep of the device's memory
+// when idle, and both pools give their idle memory back before an allocation
+// fails.  A program that has made a pool of its own current on the device
+// (cudaDeviceSetMemPool) has both from there, and no workspace is kept.
 constexpr double kScratchKeep = 1.0 / 8;
 constexpr int kMaxDevices = 64;
 struct ScratchPool {
@@ -417,10 +420,20 @@ void scratch_pool_put(cas_ctx* ctx) {
   ctx->scratch = nullptr;
 }
 
+// The pool that cudaMallocAsync would take: the program's own where it has set
+// one, else the device's default.
+cudaMemPool_t current_pool(cas_ctx* ctx) {
+  cudaMemPool_t pool = nullptr;
+  if (cudaDeviceGetMemPool(&pool, ctx->device) == cudaSuccess) return pool;
+  cudaGetLastError();
+  return ctx->def_pool;
+}
+
 // Device memory a stream-ordered allocation can still get: the device's free
 // memory, what the pools hold reserved but unused (freed allocations they
-// keep), and the rest of the context's workspace.  cudaMemGetInfo alone would count the pools' idle reserve as taken, so
-// sizes chosen from it would shrink after every large product.
+// keep), and the rest of the context's workspace.  cudaMemGetInfo alone would
+// count the pools' idle reserve as taken, so sizes chosen from it would shrink
+// after every large product.
 double free_device_bytes(cas_ctx* ctx) {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
@@ -428,9 +441,8 @@ double free_device_bytes(cas_ctx* ctx) {
     return 0.0;
   }
   double idle = (double)(ctx->ws.cap - ctx->ws.used);
-  cudaMemPool_t pools[2] = {nullptr, ctx->scratch};
-  if (cudaDeviceGetDefaultMemPool(&pools[0], ctx->device) != cudaSuccess) pools[0] = nullptr;
-  for (cudaMemPool_t pool : pools) {
+  cudaMemPool_t own = current_pool(ctx);
+  for (cudaMemPool_t pool : {ctx->def_pool, ctx->scratch, own == ctx->def_pool ? nullptr : own}) {
     uint64_t reserved = 0, used = 0;  // 64-bit attribute values
     if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
@@ -447,9 +459,7 @@ double free_device_bytes(cas_ctx* ctx) {
 void give_back(cas_ctx* ctx, cudaStream_t s) {
   g_scratch[ctx->device].book.reclaim([&](char* p) { cudaFreeAsync(p, s); });
   cudaStreamSynchronize(s);
-  cudaMemPool_t def = nullptr;
-  if (cudaDeviceGetDefaultMemPool(&def, ctx->device) == cudaSuccess) cudaMemPoolTrimTo(def, 0);
-  cudaMemPoolTrimTo(ctx->scratch, 0);
+  for (cudaMemPool_t pool : {ctx->def_pool, ctx->scratch, current_pool(ctx)}) cudaMemPoolTrimTo(pool, 0);
 }
 
 // An allocation from `pool` on stream s, tried again after give_back when no
@@ -476,7 +486,9 @@ cas_status alloc_err(cas_ctx* ctx, cudaError_t e, size_t bytes) {
 // the pool's holes the same from call to call.  A kernel on another stream
 // waits for `scratch_ready` first.
 cas_status dev_alloc(cas_ctx* ctx, void** p, size_t bytes) {
-  return alloc_err(ctx, pool_alloc(ctx, ctx->scratch, p, bytes, ctx->stream), bytes);
+  cudaMemPool_t pool = current_pool(ctx);
+  if (pool == ctx->def_pool) pool = ctx->scratch;
+  return alloc_err(ctx, pool_alloc(ctx, pool, p, bytes, ctx->stream), bytes);
 }
 cas_status scratch_ready(cas_ctx* ctx, cudaStream_t s) {
   if (s == ctx->stream) return CAS_OK;
@@ -503,7 +515,9 @@ void ws_begin(cas_ctx* ctx) {
     cudaGetLastError();
     return nullptr;
   };
-  sp.book.begin(ctx->ws, (size_t)(kWorkspaceKeep * (double)sp.total), get,
+  const bool own = current_pool(ctx) != ctx->def_pool;  // the program's pool serves the scratch too
+  if (own) ws_drop(ctx);
+  sp.book.begin(ctx->ws, own ? 0 : (size_t)(kWorkspaceKeep * (double)sp.total), get,
                 [&](char* p) { cudaFreeAsync(p, ctx->stream); });
 }
 void ws_end(cas_ctx* ctx) { g_scratch[ctx->device].book.end(ctx->ws); }
@@ -518,9 +532,7 @@ cas_status ws_alloc(cas_ctx* ctx, std::vector<void*>& spill, void** p, size_t by
 
 // an array of a result, which outlives the call
 cas_status out_alloc(cas_ctx* ctx, void** p, size_t bytes) {
-  cudaMemPool_t pool = nullptr;
-  CAS_CUDA(ctx, cudaDeviceGetDefaultMemPool(&pool, ctx->device));
-  return alloc_err(ctx, pool_alloc(ctx, pool, p, bytes, ctx->stream), bytes);
+  return alloc_err(ctx, pool_alloc(ctx, current_pool(ctx), p, bytes, ctx->stream), bytes);
 }
 
 // Host memory for C: 2 MiB-aligned and marked for transparent huge pages,
@@ -1967,10 +1979,9 @@ cas_status cas_create(int device, cas_ctx** out) {
     CAS_CUDA(ctx, cudaHostGetDevicePointer((void**)&ctx->h_counts_dev, ctx->h_counts, 0));
     CAS_CUDA(ctx, cudaHostGetDevicePointer((void**)&ctx->h_misc_dev, ctx->h_misc, 0));
     // keep freed device memory in the stream-ordered pool between calls
-    cudaMemPool_t pool;
-    CAS_CUDA(ctx, cudaDeviceGetDefaultMemPool(&pool, device));
+    CAS_CUDA(ctx, cudaDeviceGetDefaultMemPool(&ctx->def_pool, device));
     uint64_t thresh = UINT64_MAX;
-    CAS_CUDA(ctx, cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thresh));
+    CAS_CUDA(ctx, cudaMemPoolSetAttribute(ctx->def_pool, cudaMemPoolAttrReleaseThreshold, &thresh));
     CAS_TRY(scratch_pool_get(ctx));
     CAS_TRY(setup_kernels(ctx));
     return CAS_OK;
