@@ -1533,8 +1533,9 @@ cas_status compute_dev(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, De
   return CAS_OK;
 }
 
-// compute_dev, once more without the workspace when memory runs out beside it.
-// After an error nothing of the call is left, neither memory nor kernels.
+// compute_dev, once more without the workspace when the device's memory runs out
+// beside it (the host's, which at_cap takes, does not depend on it).  After an
+// error nothing of the call is left, neither memory nor kernels.
 template <typename F>
 cas_status compute(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, DevC& o, F&& at_cap) {
   auto undo = [&] {
@@ -1542,12 +1543,18 @@ cas_status compute(cas_ctx* ctx, cas_accum accum, Call& c, bool validate, DevC& 
     scratch_free(ctx, c);
     free_dev_c(o, ctx->stream);
   };
-  cas_status st = compute_dev(ctx, accum, c, validate, o, at_cap);
-  if (st == CAS_ERR_OOM && ctx->ws.mem) {
+  bool host_failed = false;
+  auto host_part = [&](int64_t cap) {
+    const cas_status s = at_cap(cap);
+    host_failed |= s != CAS_OK;
+    return s;
+  };
+  cas_status st = compute_dev(ctx, accum, c, validate, o, host_part);
+  if (st == CAS_ERR_OOM && !host_failed && ctx->ws.mem) {
     undo();
     ws_drop(ctx);
     ctx->ws.need = 0;
-    st = compute_dev(ctx, accum, c, validate, o, at_cap);
+    st = compute_dev(ctx, accum, c, validate, o, host_part);
   }
   if (st != CAS_OK) undo();
   ws_end(ctx);
