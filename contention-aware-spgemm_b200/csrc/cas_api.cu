@@ -60,7 +60,6 @@ constexpr int kSlotSymbCur = 228;   // [228, 237) symbolic bin cursors
 constexpr int kSlotSmall = 240;     // [240, 242) rows of the kNB_E1K and kNB_H256 bins that a warp takes
 constexpr int kSlotStatus = 256;    // [256, 258) the device status, behind the counters
 constexpr size_t kStageBytes = size_t(64) << 20;  // pinned staging chunk for host copies
-constexpr double kSavedBitmapBytes = 8.0 * (1ull << 30);  // heavy-row bitmaps kept between the phases
 
 }  // namespace
 
@@ -1180,14 +1179,11 @@ cas_status launch_symb_bins(cas_ctx* ctx, Call& c, int64_t* row_nz) {
         int64_t nd = n;
         if (ctx->heavy_split) CAS_TRY(symb_split_heavy(ctx, c, drows, nd, row_nz, s));
         if (nd == 0) break;
-        // bitmaps kept for the numeric kernel: every slice of each row when that fits a quarter
-        // of the free device memory, at most 24 GiB (and at least kSavedBitmapBytes), else
-        // one-slice rows only
-        const double free_b = free_device_bytes(ctx);
-        const double cap = ctx->mem_share * std::max(kSavedBitmapBytes, std::min(24.0 * (1ull << 30), 0.25 * free_b));
         const int64_t max_slices = (c.ncol + kRankCols - 1) / kRankCols;
-        c.saved_slices = (double)nd * max_slices * (kRankCols / 8) <= cap ? (int)max_slices : 1;
-        if ((double)nd * c.saved_slices * (kRankCols / 8) <= cap) {
+        const SavedBitmaps keep =
+            saved_bitmaps(nd, max_slices, kRankCols / 8, ctx->mem_share, [&] { return free_device_bytes(ctx); });
+        c.saved_slices = keep.slices;
+        if (keep.any) {
           CAS_TRY(ws_alloc(ctx, c.spill, (void**)&c.dbits, (size_t)nd * c.saved_slices * (kRankCols / 8)));
           CAS_TRY(ws_alloc(ctx, c.spill, (void**)&c.dslot, sizeof(int32_t) * (c.m + 1)));
           CAS_CUDA(ctx, cudaMemsetAsync(c.dslot, 0xFF, sizeof(int32_t) * (c.m + 1), ctx->stream));

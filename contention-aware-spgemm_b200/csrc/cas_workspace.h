@@ -14,6 +14,7 @@
 #pragma once
 #include <algorithm>
 #include <cstddef>
+#include <cstdint>
 #include <mutex>
 #include <vector>
 
@@ -115,5 +116,24 @@ class WorkspaceBook {
   std::vector<Workspace*> all_;
   size_t held_ = 0;
 };
+
+// Heavy-row bitmaps kept from the symbolic phase for the numeric one: every
+// slice of each row when that fits a quarter of the free device memory, at most
+// 24 GiB and at least 8, else the rows of one slice.  The free memory is asked
+// for only where it decides: cudaMemGetInfo waits for the driver's lock, which
+// other processes hold for 1 to 90 ms now and then (every product with heavy
+// rows asked, one in five to thirty of a 7.6 ms batch's passes took 10 to 90).
+struct SavedBitmaps {
+  int slices;  // of a row, at most
+  bool any;
+};
+template <typename Free>
+SavedBitmaps saved_bitmaps(int64_t rows, int64_t max_slices, size_t slice_bytes, double share, Free&& free_bytes) {
+  const double gib = (double)(size_t(1) << 30), whole = (double)rows * (double)max_slices * (double)slice_bytes;
+  double cap = share * 8.0 * gib;
+  if (whole > cap) cap = share * std::max(8.0 * gib, std::min(24.0 * gib, 0.25 * free_bytes()));
+  const int slices = whole <= cap ? (int)max_slices : 1;
+  return {slices, (double)rows * slices * (double)slice_bytes <= cap};
+}
 
 }  // namespace cas
