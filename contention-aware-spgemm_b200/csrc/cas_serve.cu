@@ -305,8 +305,9 @@ static cas_status serve_device_rows(cas_server* srv, const cas_csr* A, const cas
   int* d_bad = nullptr;
   int bad = 0;
   cas_status rc = CAS_OK;
-  if (cudaMallocAsync((void**)&d_out, sizeof(int64_t) * (size_t)(m > 0 ? m : 1), s) != cudaSuccess ||
-      cudaMallocAsync((void**)&d_bad, sizeof(int), s) != cudaSuccess) {
+  cas_ctx* any = srv->ctxs[0];  // for its device's pools, which give back what they hold idle
+  if (pool_alloc(any, current_pool(any), (void**)&d_out, sizeof(int64_t) * (size_t)m, s) != cudaSuccess ||
+      pool_alloc(any, current_pool(any), (void**)&d_bad, sizeof(int), s) != cudaSuccess) {
     rc = CAS_ERR_OOM;
   } else {
     int sms = 148;
