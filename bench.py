@@ -231,6 +231,12 @@ def total_products(A, B):
 def run_reference_arm(args, rank, world):
     if rank != 0:
         return 0
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle
+    if not oracle.ref_available("hybacc", small=False):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's kernels are not built (oracle/_ref), "
+                                                              "which takes its sources"}), flush=True)
+        return 0
     A, B = make_matrix(args.workload)
     base = cpu_reference(A, B, args.ref_products, args.steps, args.warmup)
     line = {"metric": "SpGEMM GFLOP/s (2 x intermediate products / s), C = A*A^T",
