@@ -228,6 +228,29 @@ def total_products(A, B):
     return _TOTAL_P[key]
 
 
+def host_memory(root="/"):
+    """Bytes of host memory that can still be taken: what the kernel has available, within the control group's limit."""
+    have = 0
+    with open(os.path.join(root, "proc/meminfo")) as fh:
+        for ln in fh:
+            if ln.startswith("MemAvailable:"):
+                have = int(ln.split()[1]) * 1024
+    for limit, used in (("memory.max", "memory.current"),
+                        ("memory/memory.limit_in_bytes", "memory/memory.usage_in_bytes")):
+        try:
+            n = [int(open(os.path.join(root, "sys/fs/cgroup", f)).read()) for f in (limit, used)]
+            have = min(have, n[0] - n[1])
+        except (OSError, ValueError):  # no such file, or "max"
+            pass
+    return max(0, have)
+
+
+def output_in_host_memory(c_bytes, input_bytes, have):
+    """Whether the end-to-end leg's C goes to host memory: where C, the pinned inputs and 8 GB beside them fit.  A
+    process that takes more than there is gets killed, with what it has measured."""
+    return c_bytes + input_bytes + 8e9 <= have
+
+
 def run_reference_arm(args, rank, world):
     if rank != 0:
         return 0
@@ -487,6 +510,9 @@ def main():
                     help="N > 1: assemble C's row shards on rank 0 after the timed steps (reported, not timed)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
+    ap.add_argument("--e2e-output", default="auto", choices=["auto", "host", "device"],
+                    help="the end-to-end leg's C: in host memory, or left on the device with its row pointers read "
+                         "back; auto: in host memory where that holds it")
     args = ap.parse_args()
 
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -704,6 +730,15 @@ def main():
     # end to end through the public C ABI with pinned host buffers: H2D of A and
     # B, the product, D2H of C into host memory, every step
     if not args.no_e2e:
+        csr_bytes = lambda M: 8 * (M.num_row + 1) + 12 * M.nnz  # noqa: E731
+        to_host = args.e2e_output == "host"
+        if args.e2e_output == "auto":
+            ins = [csr_bytes(As), 0 if world == 1 and B is A else csr_bytes(B)]
+            to_host = output_in_host_memory(12 * nnz_total + 8 * (r_end + world), world * sum(ins), host_memory())
+        if dist:  # rank 0's answer for all
+            flag = torch.tensor([int(to_host)], device=dev)
+            dist.broadcast(flag, 0)
+            to_host = bool(flag.item())
         pin = lambda x: torch.from_numpy(np.ascontiguousarray(x)).pin_memory()  # noqa: E731
         hA = [pin(As.row_ptrs), pin(As.cols), pin(As.vals)]
         hB = hA if (world == 1 and B is A) else [pin(B.row_ptrs), pin(B.cols), pin(B.vals)]
@@ -715,7 +750,7 @@ def main():
         walls, h2d, d2h = [], 0.0, 0.0
         for it in range(1 + args.e2e_steps):  # one untimed warm-up call first
             cc = casgemm.CasCsr()
-            cc.on_device, cc.col_bytes = 0, 4
+            cc.on_device, cc.col_bytes = 0 if to_host else 1, 4
             torch.cuda.synchronize()
             if dist:
                 dist.barrier()
@@ -724,12 +759,19 @@ def main():
                                      ctypes.byref(cc), None)
             if stt != 0:
                 raise casgemm.CasError(stt, ctx.lib.cas_last_error(ctx.h).decode())
-            _ = int(np.ctypeslib.as_array(ctypes.cast(cc.row_ptrs, ctypes.POINTER(ctypes.c_int64)), (cc.num_row + 1,))[-1])
+            if to_host:
+                rp = np.ctypeslib.as_array(ctypes.cast(cc.row_ptrs, ctypes.POINTER(ctypes.c_int64)), (cc.num_row + 1,))
+            else:
+                rp = casgemm.device_tensors(cc)[0].cpu()
+            assert int(rp[-1]) == cc.num_nnz
             if it > 0:
                 walls.append(time.perf_counter() - tw)
             s = ctx.stats()
             h2d, d2h, d2h_direct = s["h2d_bytes"], s["d2h_bytes"], s["d2h_direct_bytes"]
             out_blocks = s["out_blocks"]
+            if not to_host:
+                d2h = 8.0 * (cc.num_row + 1)
+            del rp
             ctx.lib.cas_csr_free(ctx.h, ctypes.byref(cc))
         wall = statistics.mean(walls)
         if dist:
@@ -740,10 +782,13 @@ def main():
                        "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                        "steps": args.e2e_steps, "s_per_step": round(wall, 3),
                        "warmup": 1, "d2h_direct_bytes_per_step": d2h_direct, "out_blocks": out_blocks,
-                       "path": "cas_spgemm on pinned host A, B; C returned in host memory (after one untimed "
-                               "call, so C's host blocks are the context's resident ones, registered with "
-                               "CUDA when they came back; d2h_direct bytes went to them by DMA directly), "
-                               "computed in out_blocks row blocks, each copied out while the next is computed"}
+                       "path": "cas_spgemm on pinned host A, B; " + (
+                           "C returned in host memory (after one untimed call, so C's host blocks are the context's "
+                           "resident ones, registered with CUDA when they came back; d2h_direct bytes went to them "
+                           "by DMA directly), computed in out_blocks row blocks, each copied out while the next is "
+                           "computed" if to_host else
+                           "C left on the device and its row pointers read back (host memory does not hold C's "
+                           "%.0f GB)" % (12e-9 * nnz_total))}
         del hA, hB
 
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
