@@ -251,6 +251,38 @@ def output_in_host_memory(c_bytes, input_bytes, have):
     return c_bytes + input_bytes + 8e9 <= have
 
 
+def warp_rows(A, B):
+    """Rows of A that a warp may take: 33 to 512 products, at most 128 entries."""
+    products = np.diff(row_products(A, B))
+    return int(((products > 32) & (products <= 512) & (np.diff(A.row_ptrs) <= 128)).sum())
+
+
+def numc_kernel(bin_name, ncol, form, fused_rows, warp, bin_rows, sms):
+    """The kernels that run a numeric bin, as the library picks them (cas_tuning.esc_form `form`): `warp` of its rows
+    are a warp's by their products and entries, which it takes where there are 8 of them per SM."""
+    ranked = form == 2 and ncol <= 1 << 21
+    by_warps = ranked and min(warp, bin_rows) >= 8 * sms
+    if bin_name == "hash256":
+        return "k_numc_warp + k_numc_hash<256,9>" if by_warps else "k_numc_hash<256,9>"
+    if bin_name in ("tiny", "hash1k", "hash4k", "dense"):
+        return {"tiny": "k_numc_tiny<256>", "hash1k": "k_numc_dense<512>" if ncol <= 1 << 16 else "k_numc_hash<256,11>",
+                "hash4k": "k_numc_dense<512>" if ncol <= 1 << 18 else "k_numc_hash<512,13>",
+                "dense": "k_numc_dense<512>"}[bin_name]
+    if ranked and (bin_name != "fused" or fused_rows >= sms):
+        shape = {"fused": "256,4,5120,fused", "esc1k": "128,12,1024", "esc2k": "256,6,2048", "esc6k": "256,3,6144",
+                 "esc8k": "256,2,8192"}.get(bin_name, "256,4,5120")
+        name = "k_numc_rank<%s>" % shape
+        return "k_numc_warp + " + name if bin_name == "esc1k" and by_warps and ncol <= 1 << 18 else name
+    if bin_name == "fused":
+        return "k_numc_esc_%s<256,5120,11,fused%s>" % ("idx" if form >= 1 else "msd",
+                                                       ",keys in registers" if form == 2 else "")
+    shape = {"esc1k": "1024,9", "esc2k": "2048,9", "esc3k": "3072,10", "esc4k": "4096,10", "esc5k": "4800,11",
+             "esc6k": "6144,11", "esc8k": "8192,11"}[bin_name]
+    big = bin_name in ("esc5k", "esc6k", "esc8k")
+    return "k_numc_esc_%s<256,%s%s>" % ("idx" if form >= 1 and big else "msd", shape,
+                                        ",keys in registers" if form == 2 and bin_name in ("esc5k", "esc6k") else "")
+
+
 def run_reference_arm(args, rank, world):
     if rank != 0:
         return 0
@@ -672,29 +704,10 @@ def main():
     dom_ms = bin_ms[dom]
     dom_bytes = bin_bytes[dom]
     achieved = dom_bytes / (dom_ms * 1e-3) / 1e9 if dom_ms > 0 else 0.0
-    ncol = B.num_col
-    kernel_name = {"tiny": "k_numc_tiny<256>", "hash256": "k_numc_hash<256,9>",
-                   "hash1k": "k_numc_dense<512>" if ncol <= 1 << 16 else "k_numc_hash<256,11>",
-                   "hash4k": "k_numc_dense<512>" if ncol <= 1 << 18 else "k_numc_hash<512,13>",
-                   "dense": "k_numc_dense<512>"}.get(dom)
-    # the index form runs the fused rows and the ESC bins over 4096 products when esc_form is 1;
-    # the ranked bitmap runs them all when it is 2 and C has at most 2^21 columns
     form = ctx.get_tuning().get("esc_form", 1)
-    idx_form = form >= 1
-    rank_shape = {"fused": "256,4,5120,fused", "esc1k": "128,12,1024", "esc2k": "256,6,2048", "esc3k": "256,4,5120",
-                  "esc4k": "256,4,5120", "esc5k": "256,4,5120", "esc6k": "256,3,6144", "esc8k": "256,2,8192"}
-    if form == 2 and ncol <= 1 << 21 and dom in rank_shape:
-        kernel_name = "k_numc_rank<%s>" % rank_shape[dom]
-    elif dom == "fused":
-        kernel_name = "k_numc_esc_%s<256,5120,11,fused%s>" % ("idx" if idx_form else "msd",
-                                                            ",keys in registers" if form == 2 else "")
-    if kernel_name is None and dom.startswith("esc"):
-        shape = {"esc1k": "1024,9", "esc2k": "2048,9", "esc3k": "3072,10", "esc4k": "4096,10",
-                 "esc5k": "4800,11", "esc6k": "6144,11", "esc8k": "8192,11"}[dom]
-        big = dom in ("esc5k", "esc6k", "esc8k")
-        kernel_name = "k_numc_esc_%s<256,%s%s>" % ("idx" if idx_form and big else "msd", shape,
-                                                  ",keys in registers" if form == 2 and dom in ("esc5k", "esc6k")
-                                                  else "")
+    warp = warp_rows(As, B) if dom in ("esc1k", "hash256") else 0
+    kernel_name = numc_kernel(dom, B.num_col, form, stats["fused_rows"], warp, stats["numc_bins"].get(dom, 0),
+                              torch.cuda.get_device_properties(dev).multi_processor_count)
     alg_bytes_total = 12.0 * (A.nnz if world == 1 else As.nnz) + 12.0 * P_local + 12.0 * nnz_local + 16.0 * (As.num_row + 1)
     pipe_frac = alg_bytes_total / (ms_step * 1e-3) / (peak * 1e9)
 

@@ -1063,7 +1063,7 @@ cas_status launch_fused(cas_ctx* ctx, Call& c, const int64_t* known, int32_t* cc
         <<<(unsigned)c.nf, 256, smem_numc_esc_msd<(int)kFusedHi, 11, VIn>(), ctx->stream>>>(
             nullptr, c.A.csr, c.B.csr, c.b_sorted ? 1 : 0, nullptr, ccol, static_cast<AT*>(cval), c.ovf, ovf_count,
             ctx->d_status, fu);
-  CAS_TRY(check_launch(ctx, "k_numc_esc_msd (fused)"));
+  CAS_TRY(check_launch(ctx, "fused rows"));
   if (ctx->profile) CAS_CUDA(ctx, cudaEventRecord(ctx->ev_fused[1], ctx->stream));
   return CAS_OK;
 }

@@ -151,16 +151,20 @@ typedef struct {
 	int32_t esc_max_products;    /* ESC rows have at most this many products, <= 8192 [8192] */
 	int32_t hash_max_nnz;        /* hash rows have at most this many distinct columns, <= 4096 [4096];
 	                                larger rows take the dense kernels */
-	int32_t esc_form;            /* bucketed ESC kernel of the fused rows and of ESC rows over 4096
-	                                products: 1 keeps column, product index and place per product in
-	                                shared memory, 4 rows per SM; 2 [the default] ranks the columns in a
-	                                two-level bitmap instead of sorting them, where B has at most 2^21
-	                                columns (and, for the fused rows, there is at least one per SM),
-	                                else it is form 1 with each thread's columns held in registers
-	                                between its histogram and scatter passes (B's columns read once)
-	                                and, for rows whose B rows average 32 products or more, a warp per
-	                                B row in the value pass (rows of up to 6144 products; larger ones
-	                                take form 1); 0 keeps column and value, 3 rows per SM */
+	int32_t esc_form;            /* kernel of the fused rows and of all ESC rows over 32 products.
+	                                2 [the default], where B has at most 2^21 columns: their columns are
+	                                ranked in a two-level bitmap instead of sorted (fused rows: where
+	                                there is at least one per SM), and rows of at most 512 products and
+	                                128 A entries, where there are 8 per SM, take a warp each (ESC rows
+	                                of at most 2^18 columns of B; hash rows of at most 256 distinct
+	                                columns too).  Else ESC rows of up to 4096 products sort bucketed
+	                                columns and values, and for the fused rows and those over 4096: 0
+	                                does so too, 3 rows per SM; 1 keeps column, product index and place
+	                                per product in shared memory, 4 rows per SM; 2 is form 1 with each
+	                                thread's columns held in registers between its histogram and scatter
+	                                passes (B's columns read once) and, for rows whose B rows average 32
+	                                products or more, a warp per B row in the value pass (rows of up to
+	                                6144 products; larger ones take form 1) */
 	int32_t heavy_split;         /* 1: dense rows of 2^17 products or more are split across thread blocks
 	                                by A-entry ranges, heaviest row first, adding into C by atomics that
 	                                stay in L2 [1]; 0: one block per dense row */
