@@ -263,7 +263,7 @@ def numc_kernel(bin_name, ncol, form, fused_rows, warp, bin_rows, sms):
     ranked = form == 2 and ncol <= 1 << 21
     by_warps = ranked and min(warp, bin_rows) >= 8 * sms
     if bin_name == "hash256":
-        return "k_numc_warp + k_numc_hash<256,9>" if by_warps else "k_numc_hash<256,9>"
+        return "k_numc_warp + k_numc_hash<256,9>" if by_warps and ncol <= 1 << 20 else "k_numc_hash<256,9>"
     if bin_name in ("tiny", "hash1k", "hash4k", "dense"):
         return {"tiny": "k_numc_tiny<256>", "hash1k": "k_numc_dense<512>" if ncol <= 1 << 16 else "k_numc_hash<256,11>",
                 "hash4k": "k_numc_dense<512>" if ncol <= 1 << 18 else "k_numc_hash<512,13>",

@@ -1342,9 +1342,12 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
   // warp's bitmap is much for it to clear and scan, and leaves fewer warps on an
   // SM: 192,500 join rows over 6e5 columns take 1.33 ms by warps and 0.97 by
   // k_numc_rank, 131,000 uniform rows over 1.3e5 0.50 and 0.72.  The hash rows,
-  // whose other kernel sorts, go by warps at any width.
+  // whose other kernel sorts, go by warps up to 2^20 columns (a product with
+  // 677,000 such rows over 1.0e6: 11.3 ms by hash, 4.2 by warps); beyond, a
+  // row's bitmap is 16 KB and an SM holds four warps (1,890,000 rows over 2.0e6:
+  // 33.4 ms by warps, 23.2 by hash; 2^20 + 1 columns, edge factor 3, 11.6 and 8.5).
   auto by_warps = [&](int b, int64_t ws) {
-    return rank && many_rows(ctx, ws) && (b == kNB_H256 || (b == kNB_E1K && c.ncol <= (int64_t(1) << kWarpBits)));
+    return rank && many_rows(ctx, ws) && c.ncol <= (int64_t(1) << (b == kNB_H256 ? kWarpHashBits : kWarpBits));
   };
   auto launch_warp = [&](const int32_t* wrows, int64_t n, cudaStream_t s) -> cas_status {
     const int cell_bits = rank_cell_bits<kWarpProducts>(c.ncol);

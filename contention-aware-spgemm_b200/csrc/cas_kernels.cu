@@ -249,7 +249,8 @@ __global__ void k_fused_scatter(int64_t m, const int64_t* __restrict__ row_flp, 
 // Rows a warp takes (k_symb_warp, k_numc_warp): products, and A entries.
 constexpr int kWarpProducts = 512;
 constexpr int kWarpEntries = 128;
-constexpr int kWarpBits = 18;  // log2 of the matrix's columns, at most, for the ESC rows
+constexpr int kWarpBits = 18;      // log2 of the matrix's columns, at most, for the ESC rows
+constexpr int kWarpHashBits = 20;  // and for the hash rows
 
 // Numeric bin histogram plus, per bin, the sums of products, nnz(C) and
 // nnz(A) of its rows (for the per-kernel algorithmic byte count).

@@ -156,8 +156,8 @@ typedef struct {
 	                                ranked in a two-level bitmap instead of sorted (fused rows: where
 	                                there is at least one per SM), and rows of at most 512 products and
 	                                128 A entries, where there are 8 per SM, take a warp each (ESC rows
-	                                of at most 2^18 columns of B; hash rows of at most 256 distinct
-	                                columns too).  Else ESC rows of up to 4096 products sort bucketed
+	                                where B has at most 2^18 columns, hash rows of at most 256 distinct
+	                                columns where it has at most 2^20).  Else ESC rows of up to 4096 products sort bucketed
 	                                columns and values, and for the fused rows and those over 4096: 0
 	                                does so too, 3 rows per SM; 1 keeps column, product index and place
 	                                per product in shared memory, 4 rows per SM; 2 is form 1 with each

@@ -28,7 +28,8 @@ IDX = "k_numc_esc_idx<256,%s,keys in registers>"
     ("esc5k", 1 << 22, 2, 0, 0, 10, IDX % "4800,11"),
     ("esc8k", 1 << 22, 2, 0, 0, 10, "k_numc_esc_idx<256,8192,11>"),
     ("esc4k", 1 << 22, 2, 0, 0, 10, "k_numc_esc_msd<256,4096,10>"),
-    ("hash256", 1 << 21, 2, 0, 5000, 5000, "k_numc_warp + k_numc_hash<256,9>"),
+    ("hash256", 1 << 20, 2, 0, 5000, 5000, "k_numc_warp + k_numc_hash<256,9>"),
+    ("hash256", (1 << 20) + 1, 2, 0, 5000, 5000, "k_numc_hash<256,9>"),
     ("hash256", 1 << 22, 2, 0, 5000, 5000, "k_numc_hash<256,9>"),
     ("hash256", 1 << 15, 1, 0, 5000, 5000, "k_numc_hash<256,9>"),
     ("hash1k", 1 << 16, 2, 0, 0, 9, "k_numc_dense<512>"), ("hash1k", 1 << 17, 2, 0, 0, 9, "k_numc_hash<256,11>"),
