@@ -3168,14 +3168,25 @@ k_numc_warp(const int32_t* __restrict__ rows, int64_t nrows, Csr A, Csr B, int32
       sts_if((dup >> u) & 1u, &rep[listed + __popc(in & lanemask_lt())], (32u * u + lane) | (half(u) << 16));
       listed += __popc(in);
     }
+    __syncwarp();
+    uint32_t d_next = 0;
+    AT x_next = AT(0);
+    auto fetch = [&](uint32_t i) {  // the lane's next repeat, loaded a turn ahead
+      x_next = AT(0);
+      if (i >= nrep) return;
+      d_next = rep[i];
+      const uint32_t e = d_next >> 25;
+      x_next = Acc<VIn>::mul(sg.av[e], __ldg(bval + (sg.off[e] + (d_next & 0xFFFFu))));
+    };
+    fetch(lane);
     for (uint32_t i0 = 0; i0 < nrep; i0 += 32) {
       __syncwarp();
       const bool in = i0 + lane < nrep;
-      const uint32_t d = in ? rep[i0 + lane] : 0u, e = d >> 25, at = (d >> 16) & 0x1FFu;
+      const uint32_t at = (d_next >> 16) & 0x1FFu;
+      AT x = x_next;
+      fetch(i0 + 32 + lane);
       const unsigned peers = __match_any_sync(kFull, in ? at : (uint32_t)kWarpProducts);
       const bool first = in && lane == __ffs(peers) - 1;
-      AT x = AT(0);
-      if (in) x = Acc<VIn>::mul(sg.av[e], __ldg(bval + (sg.off[e] + (d & 0xFFFFu))));
       if (first && i0 == 0) x += sval[at];
       x = peers_sum(peers, x);
       if (first) {
