@@ -1341,7 +1341,7 @@ cas_status launch_numc_bins(cas_ctx* ctx, Call& c, const int64_t* crp, int32_t* 
   // The warps' rows lead their two bins.  Wider than 2^kWarpBits columns a
   // warp's bitmap is much for it to clear and scan, and leaves fewer warps on an
   // SM: 192,500 join rows over 6e5 columns take 1.33 ms by warps and 0.97 by
-  // k_numc_rank, 131,000 uniform rows over 1.3e5 0.50 and 0.72.  The hash rows,
+  // k_numc_rank, 131,000 uniform rows over 1.3e5 0.48 and 0.72.  The hash rows,
   // whose other kernel sorts, go by warps up to 2^20 columns (a product with
   // 677,000 such rows over 1.0e6: 11.3 ms by hash, 4.2 by warps); beyond, a
   // row's bitmap is 16 KB and an SM holds four warps (1,890,000 rows over 2.0e6:

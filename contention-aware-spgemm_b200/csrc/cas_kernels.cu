@@ -2214,14 +2214,16 @@ k_numc_esc_idx(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted,
 //      and 4 a repeat are at most 8 a product), and each place's are summed by
 //      one warp, pairwise 32 at a time.  Added one by one, the error of a
 //      column of 64 products was 2.8 times a pairwise sum's; it is 0.7 to 1.1
-//      times, for 1.2% of the product of 70,001 ragged rows (839 to 849 us);
+//      times, for 1.3% of the product of 70,001 ragged rows (839 to 850 us), 0.7%
+//      of a join of 600,000 rows and up to 15% where a row has three products a
+//      column (20,000 rows of 1100 products over 300 columns: 500 to 590 us);
 //   5. the values, then the columns (still in registers), are copied to C in
 //      order.
 // The slots are scanned eight to a thread; rank_slot swaps every second pair
 // of 16-byte groups, so that those accesses meet no bank twice.
-// Bound: shared-memory accesses (about 59 wavefronts per 32 products, half of
-// them bank conflicts of the random cell, slot and value accesses; the LSU
-// data pipe is 69% busy) and, at 32 warps per SM, their latency.  A sort of
+// Bound: shared-memory accesses (59 wavefronts per 32 products, 37% of them
+// bank conflicts of the random cell, slot and value accesses; the LSU data
+// pipe is 66% busy, the issue slots 49%) and, at 32 warps per SM, their latency.  A sort of
 // each row (k_numc_esc_idx) issues half as many instructions again.  Uniform
 // rows of about 4115 products (505,000 of them, 5.2e5 columns): 31.3 ms with
 // k_numc_esc_idx, 22.7 ms here; skewed rows over 1.3e5 columns (12,918 of
@@ -2828,11 +2830,11 @@ k_numc_rank(const int32_t* __restrict__ rows, Csr A, Csr B, int32_t b_sorted, in
 // ---- a warp per row ---------------------------------------------------------
 // Rows of at most kWarpProducts products.  A block per row spends most of its
 // time at barriers between steps of a few hundred instructions; a warp needs
-// none, and some 30 rows are in flight on an SM.  Bound: issue slots and the
-// shared-memory pipe, each about 60% busy, and instruction fetches (the loops
-// over a lane's products are unrolled).  63,897 rows of 39 products over 5e5
+// none, and some 30 rows are in flight on an SM.  Bound: issue slots (59%
+// busy), the shared-memory pipe (61%) and instruction fetches (the loops over a
+// lane's products are unrolled).  63,897 rows of 39 products over 5e5
 // columns: symbolic 167 us by blocks, 34 by warps; 130,923 rows of 272 over
-// 1.3e5: symbolic 436 and 240, numeric 725 and 504; 63,897 hash rows of 39 over
+// 1.3e5: symbolic 436 and 240, numeric 725 and 480; 63,897 hash rows of 39 over
 // 5e5 columns took 671 us.
 constexpr int kWarpsPerBlock = 4;
 
@@ -3149,8 +3151,8 @@ k_numc_warp(const int32_t* __restrict__ rows, int64_t nrows, Csr A, Csr B, int32
   // owner's with the first.  Added one by one, the error of the diagonal of
   // A*A^T (one product per A entry) was 1.5 times a pairwise sum's at 16
   // products and 2.3 times at 65, that of a product of uniform rows of 256
-  // products 1.44 times; these are 1.0 now, and the product of 131072 such rows
-  // took 909 us then, 877 now (a 32-lane pass a list instead of one a group).
+  // products 1.44 times.  These are 1.0 times now; the product of 131072 such
+  // rows takes 877 us, 909 when every group of products added its own.
   uint16_t* rest = nullptr;
   if (distinct < n) {
     uint32_t* rep = reinterpret_cast<uint32_t*>(sval + distinct);  // product, entry and place
@@ -3402,8 +3404,8 @@ struct DenseSmem {
 // its place in C with a global atomic add (resolved in L2: a row's values are
 // at most 8 bytes x nnz(row) there).  A range wider than one slice is cut into
 // slices, B rows cut to each by binary search (B rows sorted).
-// Bound: the atomic adds, 125e9 to 180e9 a second with their share of L2
-// misses, so two blocks per SM: with four, the rows open at once overflow L2
+// Bound: the atomic adds, 151e9 a second here and 221e9 in k_dense_acc, half of
+// whose sectors miss L2, so two blocks per SM: with four, the rows open at once overflow L2
 // (dense rows of Graph500 scale 17, 1.13e9 products: 7.6 ms against 7.0).
 // Sums in shared memory, a run of columns at a time, are no faster where one
 // run holds the row (compare-and-swap loops) and slower where it takes several

@@ -119,7 +119,13 @@ typedef struct {
 
 typedef struct cas_ctx cas_ctx;
 
-/* Context on `device`; the stream is a new non-blocking stream. */
+/* Context on `device`; the stream is a new non-blocking stream.  A context
+ * keeps a workspace that its products take their scratch from: all contexts of
+ * a device together at most a sixteenth of its memory.  Before an allocation of
+ * the library fails it takes back those that no product runs in; cas_destroy
+ * gives the context's back.  While a memory pool of the program's own is current
+ * on the device (cudaDeviceSetMemPool), results and scratch come from there and
+ * no workspace is kept. */
 cas_status cas_create(int device, cas_ctx **out);
 void cas_destroy(cas_ctx *ctx);
 /* Use an existing cudaStream_t (passed as void*); NULL restores the context's own. */
